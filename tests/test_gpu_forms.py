@@ -1,0 +1,72 @@
+"""Forms of the tiled projectors that depend on the data or on the launch.
+
+The projectors take a shorter filter form where their data are finite, and
+other forms for angles whose whole tile lies inside or beyond the detector
+edges; the launch shape follows the number of tiles. Every form must give
+what the plain float32 sequence gives, infinities and NaNs included. The
+reference is that sequence in numpy, one rounding per operation: each sample
+reads its two taps in one row, (1 - t) * T0 + t * T1, zero outside. Equality
+is exact (NaN where NaN).
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+f32 = np.float32
+
+
+def _lut(na, step):
+    a = np.arange(na, dtype=f32) * f32(step)
+    return np.sin(a.astype(np.float64)).astype(f32), np.cos(a.astype(np.float64)).astype(f32)
+
+
+def _lerp(rows, c):
+    """rows: [n] values with a zero border; c: float32 coordinates."""
+    n = rows.shape[0]
+    pad = np.zeros(n + 4, f32)
+    pad[2:-2] = rows
+    cm = c - f32(0.5)
+    i0 = np.floor(cm)
+    t = cm - i0
+    k = i0.astype(np.int64)
+    a, b = pad[np.clip(k, -2, n + 1) + 2], pad[np.clip(k + 1, -2, n + 1) + 2]
+    return (f32(1) - t) * a + t * b
+
+
+def _backward(sino, step, axis):
+    """One slice, relaxation 1, volume starting at zero, one sum per direction run."""
+    na, n = sino.shape
+    sn, cs = _lut(na, step)
+    w, ax = f32(n), f32(axis)
+    diff = w - ax * f32(2)
+    half = w - ax if diff < 0 else ax
+    e0, e1 = ax - half + f32(0.5), ax + half - f32(0.5)
+    os_, shift = w / f32(2), w / f32(2) - diff / f32(2)
+    f = np.arange(n, dtype=f32) + f32(0.5) - os_
+    v, total = np.zeros((n, n), f32), np.zeros((n, n), f32)
+    vertical = np.abs(sn.astype(np.float64)) <= np.abs(cs.astype(np.float64))
+    for a in range(na):
+        if a and vertical[a] != vertical[a - 1]:
+            v, total = v + total, np.zeros((n, n), f32)
+        c = (f[None, :] * cs[a] - f[:, None] * sn[a]) + shift
+        total = total + _lerp(sino[a], np.minimum(np.maximum(c, e0), e1))
+    return v + total
+
+
+@pytest.mark.parametrize("special", [False, True])
+@pytest.mark.parametrize("slices,axis", [(1, 64.5), (12, 64.5), (137, 64.5), (304, 64.5), (12, 60.3), (1, 71.0)])
+def test_backprojector_launch_shapes_and_non_finite_data(ufoir_lib, gpu_ctx, slices, axis, special):
+    n, na = 129, 37      # one full chunk of 32 angles and a part; ragged tiles
+    step = f32(np.pi / na)
+    rng = np.random.default_rng(slices)
+    sino = rng.standard_normal((slices, na, n)).astype(f32)
+    if special:
+        sino[0, 3, 40], sino[0, 20, 64], sino[-1, 33, 100] = np.inf, -np.inf, np.nan
+        sino[0, 10, 0], sino[0, 11, n - 1] = np.inf, np.inf
+    p = ufoir_lib.ParallelProjector(gpu_ctx, step=float(step), is_forward=0, axis_position=axis, angles_num=na)
+    got = p.process(sino)
+    p.close()
+    with np.errstate(invalid="ignore"):
+        for s in sorted({0, slices - 1}):
+            np.testing.assert_array_equal(got[s], _backward(sino[s], step, axis))

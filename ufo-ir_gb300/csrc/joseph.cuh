@@ -178,6 +178,23 @@ __device__ __forceinline__ float2 lerp2(float2 t, float2 t0, float2 t1, float2 z
 }
 
 /* a * b + c per lane, fused (one rounding). */
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c);
+
+/*
+ * The same value from nt = -t in three packed operations instead of four:
+ * t is a multiple of 2^-24 in [0, 1] (the fraction of a float coordinate), so
+ * 1 - t is exact and (1 - t) * T0 is T0 - t * T0 rounded once, one fused
+ * multiply-add. It needs finite taps: with T0 = inf the fused form gives
+ * inf - inf = NaN where the four-operation form gives inf, so callers use
+ * lerp2 where the data hold a non-finite value. (A zero result may differ in
+ * sign, which no sum that starts at +0 can show.)
+ */
+__device__ __forceinline__ float2 lerp2n(float2 nt, float2 t0, float2 t1, float2 z)
+{
+    return sub2(fma2(nt, t0, t0), mul2z(nt, t1, z));
+}
+
+/* a * b + c per lane, fused (one rounding). */
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
 {
     unsigned long long r;
@@ -212,6 +229,14 @@ __device__ __forceinline__ float2 floor_half2(float2 c, float2 &t)
 {
     const float2 y = add2_rd(c, splat(kHalfFloorMagic));
     t = sub2(c, sub2(y, splat(kHalfFloorMagic)));
+    return y;
+}
+
+/* The same with the fraction negated (for lerp2n). */
+__device__ __forceinline__ float2 floor_half2n(float2 c, float2 &nt)
+{
+    const float2 y = add2_rd(c, splat(kHalfFloorMagic));
+    nt = sub2(sub2(y, splat(kHalfFloorMagic)), c);
     return y;
 }
 

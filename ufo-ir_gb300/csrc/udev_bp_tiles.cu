@@ -2,19 +2,32 @@
  * udev_bp_tiles.cu - pixel-driven backprojection over many angles, with the
  * sinogram windows of a pixel tile staged in shared memory.
  *
- * One CTA owns a 32 x 128 pixel tile; thread (tx, ty) owns the 16 pixels
- * (x0 + tx, y0 + ty + 8p), p < 16, which share fX * cos(theta) and the
- * per-angle set-up (16 pixels amortise it better than 8: 2.3 % on the C2
- * backprojection; 32 pixels, 32 x 256 tiles, need 139 KB of shared memory
- * and 132 registers, one CTA per SM, and were 23 % slower; a 64-register
- * build with 16-angle chunks, four CTAs per SM, was 6 % slower). Launches
- * with fewer than three waves of such tiles (a single slice of 1448^2: 552
- * tiles for 456 CTA slots) use 32 x 64 tiles, 8 pixels per thread, whose
- * last wave is fuller. For a chunk of
- * 32 angles the CTA copies, per angle, the
- * 160 detector values that the tile can reach (cp.async, double buffered;
- * detectors outside [0, n) read 0), so every sample reads shared memory and
- * a warp's 32 lanes (adjacent x) touch adjacent words.
+ * One CTA owns a tile of pixels; thread (tx, ty) owns COLS columns
+ * (x0 + tx + 32c) of PR rows (y0 + ty + TY p) and walks the angles with one
+ * register sum per pixel. Two columns of a row form a packed pair, so an
+ * angle costs COLS / 2 + PR packed products for COLS * PR pixels, and 32
+ * lanes (adjacent x) touch adjacent words of the staged window (no bank
+ * conflicts). For a chunk of 32 angles the CTA copies, per angle, the
+ * detector values the tile can reach (cp.async, double buffered; detectors
+ * outside [0, n) read 0), so every sample reads shared memory.
+ *
+ * Bound by the FMA pipe (a packed FP32 instruction takes two of its cycles)
+ * and the instructions around it: ncu at 4 slices of 1448^2 x 1200 counts
+ * 23.7 instructions and 13.5 on the FMA pipe per warp and 64 samples with 16
+ * pixels of one column per thread and the row products staged in shared
+ * memory, 19.1 and 11.2 with 4 columns x 8 rows and the products in
+ * registers. What that and the forms below gave, 16 slices of 1448^2 x 1200:
+ * 16.13 -> 13.69 ms; one slice 1.112 -> 1.005; six slices of 1001^2 x 451
+ * off-centre in the fast arithmetic 1.096 -> 0.938; one of 367^2 x 180
+ * 0.0424 -> 0.0300 (launch shapes below):
+ *  - the filter's three-operation form (joseph::lerp2n) where a chunk's
+ *    windows are finite, which every chunk checks as it lands (< 1 %);
+ *  - per chunk, a bit per angle says whether the whole tile lies inside the
+ *    detector edges (no clamp: before, whole tiles clamped, and every tile of
+ *    an off-centre axis) or beyond one edge (every pixel adds one value);
+ *  - the angle loop unrolled four times (16 slices: 14.40 -> 13.70 ms; eight
+ *    times 15.33, past the instruction cache). Prefetching the next angle's
+ *    record gained 4 % at two and nothing at four.
  *
  * Arithmetic is the reference's BP (projector-parallel-joseph.cl:158-218):
  * s = fX * cos - fY * sin + (os - ros), clamped to the active detector
@@ -32,15 +45,28 @@
 namespace {
 
 constexpr int kTX = 32;
-constexpr int kTY = 8;
-constexpr int kPY = 16;              /* pixels per thread (one column); 8 for few-tile launches */
-constexpr int kTileX = kTX;          /* tile is kTileX x (kTY * PY) pixels */
-constexpr int kTileY = kTY * kPY;
-constexpr int kAC = 32;              /* angles per chunk */
-constexpr int kWin = 160;            /* detector window per angle (tile span <= 131, +5 margin, +3 alignment) */
+constexpr int kAC = 32;              /* angles per chunk: one per lane of a warp */
 constexpr int kMaxSub = 16;
 
+/* A launch shape: 32 x TY threads, each with COLS pixel columns (32 apart) of
+ * PR rows (TY apart); W detectors staged per angle. */
+template <int COLS_, int PR_, int TY_, int CTAS_, int UNROLL_>
+struct BpShape {
+    static constexpr int COLS = COLS_, PR = PR_, TY = TY_, CTAS = CTAS_, Unroll = UNROLL_;
+    static constexpr int H = COLS / 2;                 /* packed pairs per row */
+    static constexpr int TileX = kTX * COLS, TileY = TY * PR, Threads = kTX * TY;
+    /* a tile spans at most its diagonal; 2 bins of margin and up to 3 of
+     * alignment before it, 2 for the second tap after it */
+    static constexpr int span(int d) { return d * d >= TileX * TileX + TileY * TileY ? d : span(d + 1); }
+    static constexpr int Win = (span(TileX) + 8 + 3) / 4 * 4;
+};
 
+/* Fewer pixels per thread cost more instructions per sample but leave more,
+ * smaller tiles for launches with few of them (see bp_shape). */
+typedef BpShape<4, 8, 8, 2, 4> ShapeL;      /* 128 x 64 tiles */
+typedef BpShape<4, 4, 8, 3, 4> ShapeM;      /* 128 x 32 */
+typedef BpShape<2, 4, 4, 7, 4> ShapeS;      /* 64 x 16 */
+typedef BpShape<2, 2, 4, 8, 8> ShapeT;      /* 64 x 8 */
 
 struct BpTileArgs {
     const float *sino;
@@ -65,17 +91,25 @@ struct BpTileArgs {
     unsigned int sub_n[kMaxSub];
 };
 
-/* Per angle of a chunk: cos, sin, and the first detector of its window
- * (as int bits); one 16-byte shared load. */
-template <int PY>
-struct __align__(16) BpSmemT {
-    float win[2][kAC][kWin];
-    float4 ang[2][kAC];
-    /* (-fY) * sin for the tile's rows, [angle][ty][pixel p of the thread's
-     * column, 4 per float4]: the same for all 32 lanes of a warp */
-    float4 nys[2][kAC][kTY][PY / 4];
+/* Per angle of a chunk: constants of packed operations twice, the shared
+ * address of the window's detector 0 less the floor bits, the window's first
+ * detector, and the clamped coordinate of a tile outside the detector edges. */
+struct __align__(16) BpAngle {
+    float2 cs, sn;
+    uint32_t base;
+    int w0;
+    float edge;
+    int pad_;
 };
-typedef BpSmemT<kPY> BpSmem;
+
+template <class T>
+struct __align__(16) BpSmem {
+    float win[2][kAC][T::Win];
+    BpAngle ang[2][kAC];
+    /* per chunk: angles whose coordinates over the whole tile lie inside the
+     * detector edges, and angles where all of them lie beyond one edge */
+    unsigned int inside[2], outside[2];
+};
 
 __device__ __forceinline__ void cp_async4(float *dst, const float *src)
 {
@@ -126,163 +160,216 @@ __device__ __forceinline__ float det_coord(float fX, float fY, float cs, float s
  * whose global address is 16-byte aligned, at most 3 before the leftmost
  * reachable tap, so the bulk of it moves in 16-byte cp.async copies; groups
  * that cross the ends of the detector row go element by element, with zeros
- * outside [0, n).
+ * outside [0, n). A warp copies whole windows (lane = group of 4).
+ *
+ * The coordinate is monotone in each pixel index (every rounding step is), so
+ * over the tile it lies between its values at the corners.
  */
-template <bool FM, int PY>
-__device__ void load_chunk(const BpTileArgs &P, BpSmemT<PY> &S, int buf, int chunk, const float *sino, int x0, int y0,
+template <class T>
+__device__ void load_chunk(const BpTileArgs &P, BpSmem<T> &S, int buf, int chunk, const float *sino, int x0, int y0,
                            const joseph::AxisConsts &k, float e0, float e1, float shift)
 {
-    constexpr int kTileH = kTY * PY;
-    const int tid = threadIdx.y * kTX + threadIdx.x;
+    const int lane = (int) threadIdx.x, warp = (int) threadIdx.y;
     const int first = chunk * kAC;
     const int count = min(kAC, P.total_angles - first);
-    if (tid < count) {
-        const int a = angle_of(P, first + tid);
-        const float cs = __ldg(P.cosv + a), sn = __ldg(P.sinv + a);
-        const float fx0 = __fsub_rn(__fadd_rn((float) x0, 0.5f), k.os);
-        const float fx1 = __fsub_rn(__fadd_rn((float) (x0 + kTileX - 1), 0.5f), k.os);
-        const float fy0 = __fsub_rn(__fadd_rn((float) y0, 0.5f), k.os);
-        const float fy1 = __fsub_rn(__fadd_rn((float) (y0 + kTileH - 1), 0.5f), k.os);
-        const float c00 = det_coord(fx0, fy0, cs, sn, shift), c10 = det_coord(fx1, fy0, cs, sn, shift);
-        const float c01 = det_coord(fx0, fy1, cs, sn, shift), c11 = det_coord(fx1, fy1, cs, sn, shift);
-        float lo = fminf(fminf(c00, c10), fminf(c01, c11));
-        lo = fminf(fmaxf(lo, e0), e1);
-        int w0 = (int) floorf(__fsub_rn(lo, 0.5f)) - 2;
-        const int mis = (int) ((reinterpret_cast<uintptr_t>(sino + (size_t) a * P.n) >> 2) & 3);
-        w0 -= (w0 + mis) & 3;
-        S.ang[buf][tid] = make_float4(cs, sn, __int_as_float(w0), 0.0f);
+    if (warp == 0) {
+        bool in = false, out = false;
+        if (lane < count) {
+            const int a = angle_of(P, first + lane);
+            const float cs = __ldg(P.cosv + a), sn = __ldg(P.sinv + a);
+            const float fx0 = __fsub_rn(__fadd_rn((float) x0, 0.5f), k.os);
+            const float fx1 = __fsub_rn(__fadd_rn((float) (x0 + T::TileX - 1), 0.5f), k.os);
+            const float fy0 = __fsub_rn(__fadd_rn((float) y0, 0.5f), k.os);
+            const float fy1 = __fsub_rn(__fadd_rn((float) (y0 + T::TileY - 1), 0.5f), k.os);
+            const float c00 = det_coord(fx0, fy0, cs, sn, shift), c10 = det_coord(fx1, fy0, cs, sn, shift);
+            const float c01 = det_coord(fx0, fy1, cs, sn, shift), c11 = det_coord(fx1, fy1, cs, sn, shift);
+            const float lo = fminf(fminf(c00, c10), fminf(c01, c11));
+            const float hi = fmaxf(fmaxf(c00, c10), fmaxf(c01, c11));
+            in = lo >= e0 && hi <= e1;
+            out = hi <= e0 || lo >= e1;
+            const float clo = fminf(fmaxf(lo, e0), e1);
+            int w0 = (int) floorf(__fsub_rn(clo, 0.5f)) - 2;
+            const int mis = (int) ((reinterpret_cast<uintptr_t>(sino + (size_t) a * P.n) >> 2) & 3);
+            w0 -= (w0 + mis) & 3;
+            BpAngle A;
+            A.cs = joseph::splat(cs);
+            A.sn = joseph::splat(sn);
+            A.base = (uint32_t) __cvta_generic_to_shared(&S.win[buf][lane][0]) -
+                     4u * (uint32_t) (w0 + joseph::kHalfFloorBits);
+            A.w0 = w0;
+            A.edge = hi <= e0 ? e0 : e1;
+            A.pad_ = 0;
+            S.ang[buf][lane] = A;
+        }
+        const unsigned int mi = __ballot_sync(0xffffffffu, in), mo = __ballot_sync(0xffffffffu, out);
+        if (lane == 0) {
+            S.inside[buf] = mi;
+            S.outside[buf] = mo & ~mi;
+        }
     }
     __syncthreads();
-    /* row products of the chunk's angles, rounded as the in-loop product
-     * (fast arithmetic: with the shift already added) */
-    float *nys = reinterpret_cast<float *>(&S.nys[buf][0][0][0]);
-    for (int idx = tid; idx < count * kTileH; idx += kTX * kTY) {
-        const int slot = idx / kTileH, r = idx % kTileH;      /* row r = ty + kTY * p */
-        const float nfy = -__fsub_rn(__fadd_rn((float) (y0 + r), 0.5f), k.os);
-        const float prod = __fmul_rn(nfy, S.ang[buf][slot].y);
-        nys[(slot * kTY + r % kTY) * PY + r / kTY] = FM ? __fadd_rn(prod, shift) : prod;
-    }
-    constexpr int kGroups = kWin / 4;
-    for (int idx = tid; idx < count * kGroups; idx += kTX * kTY) {
-        const int slot = idx / kGroups, g = idx % kGroups;
-        const int a = angle_of(P, first + slot);
-        const int d = __float_as_int(S.ang[buf][slot].z) + 4 * g;
-        float *dst = &S.win[buf][slot][4 * g];
-        const float *src = sino + (size_t) a * P.n + d;
-        if (d >= 0 && d + 4 <= P.n) {
-            cp_async16(dst, src);
-        } else {
+    for (int slot = warp; slot < count; slot += T::TY) {
+        const int w0 = S.ang[buf][slot].w0;
+        const float *src = sino + (size_t) angle_of(P, first + slot) * P.n + w0;
+        float *dst = S.win[buf][slot];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                if (d + e >= 0 && d + e < P.n)
-                    cp_async4(dst + e, src + e);
-                else
-                    dst[e] = 0.0f;
+        for (int g = 0; g < T::Win / 4; g += 32) {
+            const int e = 4 * (g + lane), d = w0 + e;
+            if (e >= T::Win)
+                continue;
+            if (d >= 0 && d + 4 <= P.n) {
+                cp_async16(dst + e, src + e);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (d + q >= 0 && d + q < P.n)
+                        cp_async4(dst + e + q, src + e + q);
+                    else
+                        dst[e + q] = 0.0f;
+                }
             }
         }
     }
 }
 
-/*
- * All angles of one staged chunk for the thread's 16 pixels, two pixels per
- * packed instruction. FAST: every clamped coordinate is >= 0.5, so the
- * three-step floor applies.
- */
-template <bool CLAMP, bool FAST, bool FM, int PY>
-__device__ __forceinline__ void sample_chunk(const BpSmemT<PY> &S, int buf, int count, int first_vi,
-                                             const BpTileArgs &P, float fX, float shift, float e0, float e1,
-                                             float2 sum[PY / 2], float2 v[PY / 2], int &sub, int &sub_end)
+/* Whether the windows of a staged chunk hold a non-finite value, in the
+ * groups this thread staged itself (load_chunk's loop; its own copies have
+ * landed). x * 0 is NaN for infinities and NaNs and 0 for all else. */
+template <class T>
+__device__ __forceinline__ bool chunk_nonfinite(const BpSmem<T> &S, int buf, int count)
 {
-    const uint32_t win0 = (uint32_t) __cvta_generic_to_shared(&S.win[buf][0][0]);
-    const uint32_t bits = FAST ? (uint32_t) joseph::kHalfFloorBits : (uint32_t) joseph::kFloorMagicBits;
+    float acc = 0.0f;
+    for (int slot = (int) threadIdx.y; slot < count; slot += T::TY) {
+#pragma unroll
+        for (int g = 0; g < T::Win / 4; g += 32) {
+            const int e = 4 * (g + (int) threadIdx.x);
+            if (e >= T::Win)
+                continue;
+            const float4 w = *reinterpret_cast<const float4 *>(&S.win[buf][slot][e]);
+            acc = fmaf(w.x, 0.0f, acc);
+            acc = fmaf(w.y, 0.0f, acc);
+            acc = fmaf(w.z, 0.0f, acc);
+            acc = fmaf(w.w, 0.0f, acc);
+        }
+    }
+    return !(acc == 0.0f);
+}
+
+/*
+ * Angles [i0, i1) of one staged chunk for the thread's pixels, two pixels of a
+ * row per packed instruction. CLAMP: coordinates are clamped to the detector
+ * edges. FAST: every (clamped) coordinate is >= 0.5, so the three-step floor
+ * applies. FIN: the windows hold finite values only, so the filter takes its
+ * three-operation form (joseph::lerp2n).
+ */
+template <class T, bool CLAMP, bool FAST, bool FM, bool FIN>
+__device__ __forceinline__ void sample_angles(const BpSmem<T> &S, int buf, int i0, int i1, const float2 (&fX)[T::H],
+                                              const float2 (&nfY)[T::PR], float shift, float e0, float e1, float2 z2,
+                                              float2 (&sum)[T::PR][T::H])
+{
+    constexpr uint32_t bits = FAST ? 0u : 4u * (uint32_t) (joseph::kFloorMagicBits - joseph::kHalfFloorBits);
     const float2 shift2 = joseph::splat(shift);
-    const float2 z2 = joseph::splat(P.neg_zero);
-    for (int i = 0; i < count; ++i) {
-        const int vi = first_vi + i;
-        if (vi == sub_end) {
-            /* end of a subset: v = v + relax * sum (one BP launch of the reference) */
+#pragma unroll T::Unroll
+    for (int i = i0; i < i1; ++i) {
+        const BpAngle A = S.ang[buf][i];
+        float2 px[T::H], py[T::PR];
 #pragma unroll
-            for (int q = 0; q < PY / 2; ++q) {
-                v[q] = joseph::add2(v[q], joseph::mul2z(joseph::splat(P.relax), sum[q], joseph::splat(P.neg_zero)));
-                sum[q] = make_float2(0.0f, 0.0f);
+        for (int h = 0; h < T::H; ++h)
+            px[h] = joseph::mul2z(fX[h], A.cs, z2);
+#pragma unroll
+        for (int p = 0; p < T::PR; ++p) {
+            py[p] = joseph::mul2z(nfY[p], A.sn, z2);
+            if (FM)
+                py[p] = joseph::add2(py[p], shift2);
+        }
+        const uint32_t base = A.base - bits;
+#pragma unroll
+        for (int p = 0; p < T::PR; ++p)
+#pragma unroll
+            for (int h = 0; h < T::H; ++h) {
+                /* fX * cos - fY * sin + shift, as fX*cos + (-fY)*sin + shift
+                 * (fast arithmetic: fX*cos + ((-fY)*sin + shift)) */
+                float2 sc = joseph::add2(px[h], py[p]);
+                if (!FM)
+                    sc = joseph::add2(sc, shift2);
+                if (CLAMP) {
+                    sc.x = fminf(fmaxf(sc.x, e0), e1);
+                    sc.y = fminf(fmaxf(sc.y, e0), e1);
+                }
+                constexpr bool kFused = FIN && FAST && !FM;
+                float2 t;
+                const float2 y = kFused ? joseph::floor_half2n(sc, t)
+                                        : FAST ? joseph::floor_half2(sc, t) : joseph::floor_any2(sc, t);
+                const uint32_t a0 = base + 4u * (uint32_t) __float_as_int(y.x);
+                const uint32_t a1 = base + 4u * (uint32_t) __float_as_int(y.y);
+                const float2 t0 = make_float2(joseph::lds(a0), joseph::lds(a1));
+                const float2 t1 = make_float2(joseph::lds(a0 + 4u), joseph::lds(a1 + 4u));
+                if (FM)
+                    sum[p][h] = joseph::lerp_acc_fast2(sum[p][h], t, t0, t1);
+                else
+                    sum[p][h] = joseph::add2(sum[p][h], kFused ? joseph::lerp2n(t, t0, t1, z2)
+                                                               : joseph::lerp2(t, t0, t1, z2));
             }
-            ++sub;
-            sub_end += (int) P.sub_n[sub];
-        }
-        const float4 ang = S.ang[buf][i];
-        float2 nys[PY / 2];
+    }
+}
+
+/* The same where the whole tile lies beyond one detector edge: every pixel's
+ * coordinate is clamped to that edge, so all of them add one value. */
+template <class T, bool FM>
+__device__ __forceinline__ void edge_angles(const BpSmem<T> &S, int buf, int i0, int i1, float2 z2,
+                                            float2 (&sum)[T::PR][T::H])
+{
+    for (int i = i0; i < i1; ++i) {
+        const BpAngle A = S.ang[buf][i];
+        float2 t;
+        const float2 y = joseph::floor_any2(joseph::splat(A.edge), t);
+        const uint32_t a = A.base + 4u * (uint32_t) (__float_as_int(y.x) -
+                                                     (joseph::kFloorMagicBits - joseph::kHalfFloorBits));
+        const float2 t0 = joseph::splat(joseph::lds(a)), t1 = joseph::splat(joseph::lds(a + 4u));
+        const float2 val = joseph::lerp2(t, t0, t1, z2);
 #pragma unroll
-        for (int f = 0; f < PY / 4; ++f) {
-            const float4 ny = S.nys[buf][i][threadIdx.y][f];
-            nys[2 * f] = make_float2(ny.x, ny.y);
-            nys[2 * f + 1] = make_float2(ny.z, ny.w);
-        }
-        /* shared address of detector 0 of this angle's window, less the floor bits */
-        const uint32_t base = win0 + 4u * (uint32_t) (i * kWin) - 4u * ((uint32_t) __float_as_int(ang.z) + bits);
-        const float2 fxc = joseph::splat(__fmul_rn(fX, ang.x));
+        for (int p = 0; p < T::PR; ++p)
 #pragma unroll
-        for (int q = 0; q < PY / 2; ++q) {
-            /* fX * cos - fY * sin + shift, as fX*cos + (-fY)*sin + shift
-             * (fast arithmetic: fX*cos + ((-fY)*sin + shift)) */
-            float2 sc = FM ? joseph::add2(fxc, nys[q]) : joseph::add2(joseph::add2(fxc, nys[q]), shift2);
-            if (CLAMP) {
-                sc.x = fminf(fmaxf(sc.x, e0), e1);
-                sc.y = fminf(fmaxf(sc.y, e0), e1);
-            }
-            float2 t;
-            const float2 y = FAST ? joseph::floor_half2(sc, t) : joseph::floor_any2(sc, t);
-            const uint32_t a0 = base + 4u * (uint32_t) __float_as_int(y.x);
-            const uint32_t a1 = base + 4u * (uint32_t) __float_as_int(y.y);
-            const float2 t0 = make_float2(joseph::lds(a0), joseph::lds(a1));
-            const float2 t1 = make_float2(joseph::lds(a0 + 4u), joseph::lds(a1 + 4u));
-            sum[q] = FM ? joseph::lerp_acc_fast2(sum[q], t, t0, t1) : joseph::add2(sum[q], joseph::lerp2(t, t0, t1, z2));
-        }
+            for (int h = 0; h < T::H; ++h)
+                sum[p][h] = FM ? joseph::lerp_acc_fast2(sum[p][h], t, t0, t1) : joseph::add2(sum[p][h], val);
     }
 }
 
 /* One CTA's work: pixel tile `tile` of slice `slice`. */
-template <bool FM, int PY>
-__device__ __forceinline__ void bp_tile(const BpTileArgs &P, BpSmemT<PY> &S, int tile, int slice)
+template <class T, bool FM>
+__device__ __forceinline__ void bp_tile(const BpTileArgs &P, BpSmem<T> &S, int tile, int slice)
 {
-    constexpr int kTileH = kTY * PY;
     const int n = P.n;
-    const int tiles_x = (n + kTileX - 1) / kTileX;
-    const int x0 = (tile % tiles_x) * kTileX;
-    const int y0 = (tile / tiles_x) * kTileH;
+    const int tiles_x = (n + T::TileX - 1) / T::TileX;
+    const int x0 = (tile % tiles_x) * T::TileX;
+    const int y0 = (tile / tiles_x) * T::TileY;
     const float *sino = P.sino + (size_t) slice * P.sino_stride;
 
     const joseph::AxisConsts k = joseph::axis_consts(n, P.axis);
     float e0, e1;
     joseph::bp_edges(k, n, P.axis, e0, e1);
     const float shift = __fsub_rn(k.os, k.ros);
+    const float2 z2 = joseph::splat(P.neg_zero);
 
+    /* pixel pairs: columns x + 64h and x + 64h + 32 of one row */
     const int x = x0 + (int) threadIdx.x;
-    const float fX = __fsub_rn(__fadd_rn((float) x, 0.5f), k.os);
-    /* pixel pairs (p, p + 1) of the thread's column */
-    float2 sum[PY / 2], v[PY / 2];
+    float2 fX[T::H], nfY[T::PR], sum[T::PR][T::H], v[T::PR][T::H];
 #pragma unroll
-    for (int q = 0; q < PY / 2; ++q) {
-        float b[2];
+    for (int h = 0; h < T::H; ++h)
+        fX[h] = make_float2(__fsub_rn(__fadd_rn((float) (x + 2 * kTX * h), 0.5f), k.os),
+                            __fsub_rn(__fadd_rn((float) (x + 2 * kTX * h + kTX), 0.5f), k.os));
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int y = y0 + (int) threadIdx.y + kTY * (2 * q + h);
-            const size_t pix = (size_t) slice * P.vol_stride + (size_t) y * n + x;
-            b[h] = (P.base && x < n && y < n) ? P.base[pix] : 0.0f;
+    for (int p = 0; p < T::PR; ++p) {
+        const int y = y0 + (int) threadIdx.y + T::TY * p;
+        nfY[p] = joseph::splat(-__fsub_rn(__fadd_rn((float) y, 0.5f), k.os));
+        const size_t row = (size_t) slice * P.vol_stride + (size_t) y * n;
+#pragma unroll
+        for (int h = 0; h < T::H; ++h) {
+            const int xa = x + 2 * kTX * h, xb = xa + kTX;
+            v[p][h] = make_float2((P.base && xa < n && y < n) ? P.base[row + xa] : 0.0f,
+                                  (P.base && xb < n && y < n) ? P.base[row + xb] : 0.0f);
+            sum[p][h] = make_float2(0.0f, 0.0f);
         }
-        v[q] = make_float2(b[0], b[1]);
-        sum[q] = make_float2(0.0f, 0.0f);
-    }
-
-    /* A tile whose every pixel lies within distance (n/2 - 2) of the centre
-     * never reaches the clamp edges (on-axis geometry), so the clamp can be
-     * skipped without changing any result; its coordinates lie in
-     * [2, n - 2]. */
-    bool clamp = true;
-    if (k.diff == 0.0f) {
-        const float r = 0.5f * (float) n - 2.0f;
-        const float ax = fmaxf(fabsf((float) x0 - k.os), fabsf((float) (x0 + kTileX) - k.os));
-        const float ay = fmaxf(fabsf((float) y0 - k.os), fabsf((float) (y0 + kTileH) - k.os));
-        clamp = ax * ax + ay * ay > r * r;
     }
     /* clamped coordinates are >= min(e0, e1) */
     const bool fast = fminf(e0, e1) >= 0.5f;
@@ -291,56 +378,86 @@ __device__ __forceinline__ void bp_tile(const BpTileArgs &P, BpSmemT<PY> &S, int
     int sub = 0;
     int sub_end = P.n_subsets > 0 ? (int) P.sub_n[0] : 0;
     if (nchunks > 0) {
-        load_chunk<FM, PY>(P, S, 0, 0, sino, x0, y0, k, e0, e1, shift);
+        load_chunk<T>(P, S, 0, 0, sino, x0, y0, k, e0, e1, shift);
         cp_async_commit();
     }
     for (int ch = 0; ch < nchunks; ++ch) {
         const int buf = ch & 1;
         if (ch + 1 < nchunks) {
-            load_chunk<FM, PY>(P, S, buf ^ 1, ch + 1, sino, x0, y0, k, e0, e1, shift);
+            load_chunk<T>(P, S, buf ^ 1, ch + 1, sino, x0, y0, k, e0, e1, shift);
             cp_async_commit();
             cp_async_wait<1>();
         } else {
             cp_async_wait<0>();
         }
-        __syncthreads();
-        const int count = min(kAC, P.total_angles - ch * kAC);
-        if (!clamp)
-            sample_chunk<false, true, FM, PY>(S, buf, count, ch * kAC, P, fX, shift, e0, e1, sum, v, sub, sub_end);
-        else if (fast)
-            sample_chunk<true, true, FM, PY>(S, buf, count, ch * kAC, P, fX, shift, e0, e1, sum, v, sub, sub_end);
+        const int first = ch * kAC, count = min(kAC, P.total_angles - first);
+        bool fin = false;
+        if (FM)
+            __syncthreads();
         else
-            sample_chunk<true, false, FM, PY>(S, buf, count, ch * kAC, P, fX, shift, e0, e1, sum, v, sub, sub_end);
+            fin = !__syncthreads_or(chunk_nonfinite<T>(S, buf, count));
+        const unsigned int in = S.inside[buf], out = S.outside[buf];
+        for (int i = 0; i < count;) {
+            if (first + i == sub_end) {
+                /* end of a subset: v = v + relax * sum (one BP launch of the reference) */
+#pragma unroll
+                for (int p = 0; p < T::PR; ++p)
+#pragma unroll
+                    for (int h = 0; h < T::H; ++h) {
+                        v[p][h] = joseph::add2(v[p][h], joseph::mul2z(joseph::splat(P.relax), sum[p][h], z2));
+                        sum[p][h] = make_float2(0.0f, 0.0f);
+                    }
+                ++sub;
+                sub_end += (int) P.sub_n[sub];
+                continue;
+            }
+            /* the run of angles of one form from here on */
+            const bool is_in = (in >> i) & 1u, is_out = (out >> i) & 1u;
+            const unsigned int same = (is_in ? in : is_out ? out : ~(in | out)) >> i;
+            const int run = same == 0xffffffffu ? 32 : __ffs((int) ~same) - 1;
+            const int end = min(min(count, sub_end - first), i + run);
+            if (!fast)
+                sample_angles<T, true, false, FM, false>(S, buf, i, end, fX, nfY, shift, e0, e1, z2, sum);
+            else if (is_in && (FM || fin))
+                sample_angles<T, false, true, FM, true>(S, buf, i, end, fX, nfY, shift, e0, e1, z2, sum);
+            else if (is_out)
+                edge_angles<T, FM>(S, buf, i, end, z2, sum);
+            else
+                sample_angles<T, true, true, FM, false>(S, buf, i, end, fX, nfY, shift, e0, e1, z2, sum);
+            i = end;
+        }
         __syncthreads();
     }
-    if (P.n_subsets > 0) {
 #pragma unroll
-        for (int q = 0; q < PY / 2; ++q)
-            v[q] = joseph::add2(v[q], joseph::mul2z(joseph::splat(P.relax), sum[q], joseph::splat(P.neg_zero)));
-    }
-    if (x >= n)
-        return;
+    for (int p = 0; p < T::PR; ++p) {
+        const int y = y0 + (int) threadIdx.y + T::TY * p;
 #pragma unroll
-    for (int p = 0; p < PY; ++p) {
-        const int y = y0 + (int) threadIdx.y + kTY * p;
-        if (y >= n)
-            continue;
-        float r = (p & 1) ? v[p >> 1].y : v[p >> 1].x;
-        if (P.cw)
-            r = __fmul_rn(r, P.cw[(size_t) slice * P.cw_stride + (size_t) y * n + x]);
-        const size_t pix = (size_t) slice * P.vol_stride + (size_t) y * n + x;
-        if (P.add)
-            r = __fadd_rn(r, P.add[pix]);
-        P.dst[pix] = r;
+        for (int c = 0; c < T::COLS; ++c) {
+            const int xc = x + kTX * c;
+            float2 vv = v[p][c >> 1];
+            if (P.n_subsets > 0)
+                vv = joseph::add2(vv, joseph::mul2z(joseph::splat(P.relax), sum[p][c >> 1], z2));
+            if (xc >= n || y >= n)
+                continue;
+            float r = (c & 1) ? vv.y : vv.x;
+            if (P.cw)
+                r = __fmul_rn(r, P.cw[(size_t) slice * P.cw_stride + (size_t) y * n + xc]);
+            const size_t pix = (size_t) slice * P.vol_stride + (size_t) y * n + xc;
+            if (P.add)
+                r = __fadd_rn(r, P.add[pix]);
+            P.dst[pix] = r;
+        }
     }
 }
 
-template <bool FM, int PY>
-__global__ void __launch_bounds__(kTX * kTY) bp_tiles_kernel(const __grid_constant__ BpTileArgs P)
+template <class T, bool FM>
+__global__ void __launch_bounds__(T::Threads, T::CTAS) bp_tiles_kernel(const __grid_constant__ BpTileArgs P)
 {
-    __shared__ BpSmemT<PY> S;
-    bp_tile<FM, PY>(P, S, (int) blockIdx.x, (int) blockIdx.y);
+    __shared__ BpSmem<T> S;
+    bp_tile<T, FM>(P, S, (int) blockIdx.x, (int) blockIdx.y);
 }
+
+typedef ShapeM BatchShape;
 
 /*
  * Mixed batch: the pixel tiles of many one-slice jobs (any size and angle
@@ -349,12 +466,11 @@ __global__ void __launch_bounds__(kTX * kTY) bp_tiles_kernel(const __grid_consta
  * memory. Jobs whose active flag is 0 are skipped.
  */
 template <bool FM>
-__global__ void __launch_bounds__(kTX * kTY, 3) bp_tiles_batch_kernel(const BpTileArgs *__restrict__ recs,
-                                                                   const int *__restrict__ item_start, int n_jobs,
-                                                                   const int *__restrict__ job_index,
-                                                                   const int *__restrict__ active)
+__global__ void __launch_bounds__(BatchShape::Threads, BatchShape::CTAS)
+    bp_tiles_batch_kernel(const BpTileArgs *__restrict__ recs, const int *__restrict__ item_start, int n_jobs,
+                          const int *__restrict__ job_index, const int *__restrict__ active)
 {
-    __shared__ BpSmem S;
+    __shared__ BpSmem<BatchShape> S;
     __shared__ BpTileArgs rec;
     __shared__ int job_s;
     const int b = (int) blockIdx.x;
@@ -377,11 +493,11 @@ __global__ void __launch_bounds__(kTX * kTY, 3) bp_tiles_batch_kernel(const BpTi
     {
         const int *src = reinterpret_cast<const int *>(recs + j);
         int *dst = reinterpret_cast<int *>(&rec);
-        for (int e = tid; e < (int) (sizeof(BpTileArgs) / sizeof(int)); e += kTX * kTY)
+        for (int e = tid; e < (int) (sizeof(BpTileArgs) / sizeof(int)); e += BatchShape::Threads)
             dst[e] = __ldg(src + e);
     }
     __syncthreads();
-    bp_tile<FM, kPY>(rec, S, b - __ldg(item_start + j), 0);
+    bp_tile<BatchShape, FM>(rec, S, b - __ldg(item_start + j), 0);
 }
 
 static_assert(sizeof(BpTileArgs) % sizeof(int) == 0, "records are copied as ints");
@@ -433,6 +549,40 @@ static int fill_args(udev *d, const udev_geom *g, const ufoir_subset *subsets, i
     return UFOIR_OK;
 }
 
+template <class T>
+static int launch_bp(udev *d, const BpTileArgs &B, int fast_arith, int n_slices)
+{
+    const unsigned int tiles = udev_div_up(B.n, T::TileX) * udev_div_up(B.n, T::TileY);
+    const dim3 grid(tiles, (unsigned int) n_slices), block(kTX, T::TY);
+    if (fast_arith)
+        bp_tiles_kernel<T, true><<<grid, block, 0, d->stream>>>(B);
+    else
+        bp_tiles_kernel<T, false><<<grid, block, 0, d->stream>>>(B);
+    return udev_after_launch(d, "bp_tiles_kernel");
+}
+
+/*
+ * The launch shape by how many waves of tiles a launch has (ms, GB300, at
+ * L / M / S / T):
+ *   16 x 1448^2 x 1200 (14.5 waves of L)  13.69 / 14.06 / 14.74 / -
+ *    2 x 2900^2 x 360  (7.0)               2.04 /  2.05 /  2.24 / -
+ *    6 x 1001^2 x 451  (2.5; 3.4 of M)     1.08 /  1.03 /  1.06 / 1.26
+ *    3 x 1448^2 x 1200 (2.7; 3.6 of M)     2.86 /  2.77 /  2.85 / 3.62
+ *    2 x 1448^2 x 1200 (2.4 of M)          1.99 /  1.96 /  1.93 / 2.43
+ *    1 x 1448^2 x 1200 (1.2 of M)          1.05 /  1.05 /  1.01 / 1.26
+ *    4 x 367^2 x 180   (3.6 S tiles per SM) 0.112 / 0.067 / 0.062 / 0.067
+ *    1 x 512^2 x 400   (1.7)               0.220 / 0.117 / 0.080 / 0.078
+ *    1 x 367^2 x 180   (0.9)               0.112 / 0.067 / 0.037 / 0.030
+ */
+static int bp_shape(udev *d, int n, int n_slices)
+{
+    const long long sms = udev_sm_count(d);
+    const long long l = (long long) udev_div_up(n, ShapeL::TileX) * udev_div_up(n, ShapeL::TileY) * n_slices;
+    const long long m = (long long) udev_div_up(n, ShapeM::TileX) * udev_div_up(n, ShapeM::TileY) * n_slices;
+    const long long s = (long long) udev_div_up(n, ShapeS::TileX) * udev_div_up(n, ShapeS::TileY) * n_slices;
+    return l >= 6 * ShapeL::CTAS * sms ? 0 : m >= 3 * ShapeM::CTAS * sms ? 1 : s >= 2 * sms ? 2 : 3;
+}
+
 }  // namespace
 
 extern "C" size_t udev_bp_record_bytes(void)
@@ -449,8 +599,8 @@ extern "C" int udev_bp_record(udev *d, const udev_geom *g, const ufoir_subset *s
     if (rc)
         return rc;
     memcpy(record, &A, sizeof(A));
-    const int tiles_x = (g->n_dets + kTileX - 1) / kTileX;
-    const int tiles_y = (g->n_dets + kTileY - 1) / kTileY;
+    const int tiles_x = (g->n_dets + BatchShape::TileX - 1) / BatchShape::TileX;
+    const int tiles_y = (g->n_dets + BatchShape::TileY - 1) / BatchShape::TileY;
     *items = tiles_x * tiles_y;
     return UFOIR_OK;
 }
@@ -462,10 +612,10 @@ extern "C" int udev_bp_batch(udev *d, int fast_arith, const void *d_records, con
         return UFOIR_OK;
     UDEV_BIND(d);
     if (fast_arith)
-        bp_tiles_batch_kernel<true><<<(unsigned int) n_items, dim3(kTX, kTY), 0, d->stream>>>(
+        bp_tiles_batch_kernel<true><<<(unsigned int) n_items, dim3(kTX, BatchShape::TY), 0, d->stream>>>(
             static_cast<const BpTileArgs *>(d_records), d_item_start, n_jobs, d_job_index, d_active);
     else
-        bp_tiles_batch_kernel<false><<<(unsigned int) n_items, dim3(kTX, kTY), 0, d->stream>>>(
+        bp_tiles_batch_kernel<false><<<(unsigned int) n_items, dim3(kTX, BatchShape::TY), 0, d->stream>>>(
             static_cast<const BpTileArgs *>(d_records), d_item_start, n_jobs, d_job_index, d_active);
     return udev_after_launch(d, "bp_tiles_batch_kernel");
 }
@@ -481,16 +631,7 @@ extern "C" int udev_bp_tiles(udev *d, const udev_geom *g, const ufoir_subset *su
     if (rc0)
         return rc0;
     UDEV_BIND(d);
-    /* Tiles of 16 pixels per thread (32 x 128) unless the launch has fewer than
-     * three waves of them (three CTAs per SM): then 8 per thread (32 x 64), whose
-     * last wave is fuller. At 1448^2 x 1200 one slice's BP took 1.131 instead of
-     * 1.194 ms, two slices' 2.155 instead of 2.266; three slices (3.6 waves)
-     * keep the tall tiles (3.130 against 3.197 ms). */
-    const int tiles_x = (g->n_dets + kTileX - 1) / kTileX;
-    const long long tiles16 = (long long) tiles_x * ((g->n_dets + kTileY - 1) / kTileY);
-    const bool short_tiles = tiles16 * n_slices < 3LL * 3 * udev_sm_count(d);
-    const int tile_h = short_tiles ? kTY * 8 : kTileY;
-    const unsigned int n_tiles = (unsigned int) (tiles_x * ((g->n_dets + tile_h - 1) / tile_h));
+    const int shape = bp_shape(d, g->n_dets, n_slices);
     for (int done = 0; done < n_slices;) {
         const int chunk = n_slices - done > 65535 ? 65535 : n_slices - done;
         BpTileArgs B = A;
@@ -502,16 +643,10 @@ extern "C" int udev_bp_tiles(udev *d, const udev_geom *g, const ufoir_subset *su
         if (B.add)
             B.add += (size_t) done * A.vol_stride;
         B.dst += (size_t) done * A.vol_stride;
-        const dim3 grid(n_tiles, (unsigned int) chunk), block(kTX, kTY);
-        if (g->fast_arith && short_tiles)
-            bp_tiles_kernel<true, 8><<<grid, block, 0, d->stream>>>(B);
-        else if (g->fast_arith)
-            bp_tiles_kernel<true, kPY><<<grid, block, 0, d->stream>>>(B);
-        else if (short_tiles)
-            bp_tiles_kernel<false, 8><<<grid, block, 0, d->stream>>>(B);
-        else
-            bp_tiles_kernel<false, kPY><<<grid, block, 0, d->stream>>>(B);
-        int rc = udev_after_launch(d, "bp_tiles_kernel");
+        const int rc = shape == 0   ? launch_bp<ShapeL>(d, B, g->fast_arith, chunk)
+                       : shape == 1 ? launch_bp<ShapeM>(d, B, g->fast_arith, chunk)
+                       : shape == 2 ? launch_bp<ShapeS>(d, B, g->fast_arith, chunk)
+                                    : launch_bp<ShapeT>(d, B, g->fast_arith, chunk);
         if (rc)
             return rc;
         done += chunk;

@@ -8,11 +8,11 @@
  *    does not change with occupancy (24 to 64 warps per SM give the same);
  *    it is bound by the FMA pipe, where a packed FP32 instruction takes two
  *    cycles.
- *  - backward: bp_tiles_kernel's inner loop for an unclamped tile: per angle
- *    the angle record and the row products from shared memory, per pixel pair
- *    the coordinate, the three-step floor, two taps per pixel from the
- *    angle's window, the filter and the per-pixel sum; 16 pixels per thread
- *    and three 256-thread CTAs per SM, as the kernel runs.
+ *  - backward: bp_tiles_kernel's inner loop for a tile inside the detector
+ *    edges: per angle its record from shared memory and the row and column
+ *    products, per pixel pair the coordinate, the three-step floor, two taps
+ *    per pixel from the angle's window, the filter and the per-pixel sum; 32
+ *    pixels per thread and two 256-thread CTAs per SM, as the kernel runs.
  */
 #include <cuda_runtime.h>
 
@@ -79,59 +79,66 @@ constexpr int kBpAngles = 4096;      /* angles walked per launch */
 constexpr int kBpChunk = 32;         /* distinct angles staged, as one chunk of the kernel */
 constexpr int kBpWin = 320;          /* window per angle */
 
-__global__ void __launch_bounds__(256) sample_ceiling_bp_kernel(float neg_zero, float *out)
+struct __align__(16) CeilAngle {
+    float2 cs, sn;
+    uint32_t base;
+    int pad_[3];
+};
+
+__global__ void __launch_bounds__(256, 2) sample_ceiling_bp_kernel(float neg_zero, float *out)
 {
     __shared__ float win[kBpChunk][kBpWin];
-    __shared__ float4 ang[kBpChunk];
-    __shared__ float4 nys[kBpChunk][8][4];
+    __shared__ CeilAngle ang[kBpChunk];
     const int tid = (int) (threadIdx.y * 32 + threadIdx.x);
     for (int i = tid; i < kBpChunk * kBpWin; i += 256)
         (&win[0][0])[i] = (float) ((i * 37) & 255) * 0.0078125f;
-    if (tid < kBpChunk)
-        ang[tid] = make_float4(0.96875f - 0.0078125f * (float) tid, 0.5f, __int_as_float(0), 0.0f);
-    /* row products of rows ty + 8p, spread so that the coordinates stay in
-     * [150, 300] */
-    for (int i = tid; i < kBpChunk * 8 * 16; i += 256)
-        reinterpret_cast<float *>(&nys[0][0][0])[i] = (float) ((i * 7) % 97) + 30.0f;
+    if (tid < kBpChunk) {
+        /* columns up to 127.5 and rows up to 63.5 keep every coordinate in
+         * [150, 315] */
+        ang[tid].cs = joseph::splat(0.96875f - 0.0078125f * (float) tid);
+        ang[tid].sn = joseph::splat(0.5f);
+        ang[tid].base = (uint32_t) __cvta_generic_to_shared(&win[tid][0]) - 4u * (uint32_t) joseph::kHalfFloorBits;
+    }
     __syncthreads();
     const float2 z2 = joseph::splat(neg_zero);
-    const float2 shift2 = joseph::splat(120.25f);
-    const float fX = (float) threadIdx.x + 0.5f;
-    const uint32_t win0 = (uint32_t) __cvta_generic_to_shared(&win[0][0]);
-    float2 sum[8];
+    const float2 shift2 = joseph::splat(150.25f);
+    float2 fX[2], fY[8], sum[8][2];
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-        sum[q] = make_float2(0.0f, 0.0f);
-#pragma unroll 1
+    for (int h = 0; h < 2; ++h)
+        fX[h] = make_float2((float) (threadIdx.x + 64 * h) + 0.5f, (float) (threadIdx.x + 64 * h + 32) + 0.5f);
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+        fY[p] = joseph::splat((float) (threadIdx.y + 8 * p) + 0.5f);
+        sum[p][0] = sum[p][1] = make_float2(0.0f, 0.0f);
+    }
+#pragma unroll 4
     for (int a = 0; a < kBpAngles; ++a) {
-        const int i = a & (kBpChunk - 1);
-        const float4 an = ang[i];
-        float2 ny[8];
+        const CeilAngle A = ang[a & (kBpChunk - 1)];
+        float2 px[2], py[8];
 #pragma unroll
-        for (int f = 0; f < 4; ++f) {
-            const float4 v = nys[i][threadIdx.y][f];
-            ny[2 * f] = make_float2(v.x, v.y);
-            ny[2 * f + 1] = make_float2(v.z, v.w);
-        }
-        const uint32_t base = win0 + 4u * (uint32_t) (i * kBpWin) -
-                              4u * ((uint32_t) __float_as_int(an.z) + (uint32_t) joseph::kHalfFloorBits);
-        const float2 fxc = joseph::splat(__fmul_rn(fX, an.x));
+        for (int h = 0; h < 2; ++h)
+            px[h] = joseph::mul2z(fX[h], A.cs, z2);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const float2 sc = joseph::add2(joseph::add2(fxc, ny[q]), shift2);
-            float2 t;
-            const float2 y = joseph::floor_half2(sc, t);
-            const uint32_t a0 = base + 4u * (uint32_t) __float_as_int(y.x);
-            const uint32_t a1 = base + 4u * (uint32_t) __float_as_int(y.y);
-            const float2 t0 = make_float2(joseph::lds(a0), joseph::lds(a1));
-            const float2 t1 = make_float2(joseph::lds(a0 + 4u), joseph::lds(a1 + 4u));
-            sum[q] = joseph::add2(sum[q], joseph::lerp2(t, t0, t1, z2));
-        }
+        for (int p = 0; p < 8; ++p)
+            py[p] = joseph::mul2z(fY[p], A.sn, z2);
+#pragma unroll
+        for (int p = 0; p < 8; ++p)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float2 sc = joseph::add2(joseph::add2(px[h], py[p]), shift2);
+                float2 t;
+                const float2 y = joseph::floor_half2n(sc, t);
+                const uint32_t a0 = A.base + 4u * (uint32_t) __float_as_int(y.x);
+                const uint32_t a1 = A.base + 4u * (uint32_t) __float_as_int(y.y);
+                const float2 t0 = make_float2(joseph::lds(a0), joseph::lds(a1));
+                const float2 t1 = make_float2(joseph::lds(a0 + 4u), joseph::lds(a1 + 4u));
+                sum[p][h] = joseph::add2(sum[p][h], joseph::lerp2n(t, t0, t1, z2));
+            }
     }
     float acc = 0.0f;
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-        acc += sum[q].x + sum[q].y;
+    for (int p = 0; p < 8; ++p)
+        acc += sum[p][0].x + sum[p][0].y + sum[p][1].x + sum[p][1].y;
     out[blockIdx.x * 256 + tid] = acc;
 }
 
@@ -140,7 +147,7 @@ __global__ void __launch_bounds__(256) sample_ceiling_bp_kernel(float neg_zero, 
 extern "C" int udev_sample_ceiling_bp(udev *d, double *samples_per_s)
 {
     UDEV_BIND(d);
-    const int blocks = 3 * d->sm_count;
+    const int blocks = 2 * d->sm_count;
     float *out = nullptr;
     int rc = udev_malloc(d, (void **) &out, sizeof(float) * (size_t) blocks * 256);
     if (rc)
@@ -159,7 +166,7 @@ extern "C" int udev_sample_ceiling_bp(udev *d, double *samples_per_s)
     udev_free(d, out);
     if (rc)
         return rc;
-    const double samples = (double) blocks * 256 * 16 * kBpAngles;
+    const double samples = (double) blocks * 256 * 32 * kBpAngles;
     *samples_per_s = ms > 0.0f ? samples / (ms * 1e-3) : 0.0;
     return UFOIR_OK;
 }
