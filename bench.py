@@ -421,13 +421,11 @@ def run_ufoir(args, dist):
 # FP32 operations per pair of samples on the FMA pipe (packed f32x2: one
 # lane-op per sample each), the dominant forms: the BP's coordinate (2),
 # floor (3), interpolation (3: one fused for (1 - t) T0, the other product,
-# their sum) and sum (1);
-# the FP's inside form: floor (3), interpolation (4: 1 - t, two products, their
-# sum), block sum (1) and the
+# their sum) and sum (1); the FP's inside form: floor (3), interpolation (3), block sum (1) and the
 # coordinate recurrence (1). Fast arithmetic: the BP's shift is folded (1)
 # and interpolation + sum take 3 (T1 - T0, acc + T0, one fma); the FP's
 # interpolation + sum take 3.
-FMA_OPS_PER_SAMPLE = {("bp", False): 9, ("fp", False): 9, ("bp", True): 7, ("fp", True): 7}
+FMA_OPS_PER_SAMPLE = {("bp", False): 9, ("fp", False): 8, ("bp", True): 7, ("fp", True): 7}
 
 
 def fma_pipe_bound(kernel, rate, sm_count, clock_info, fast):

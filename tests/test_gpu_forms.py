@@ -70,3 +70,44 @@ def test_backprojector_launch_shapes_and_non_finite_data(ufoir_lib, gpu_ctx, sli
     with np.errstate(invalid="ignore"):
         for s in sorted({0, slices - 1}):
             np.testing.assert_array_equal(got[s], _backward(sino[s], step, axis))
+
+
+def _forward(vol, na, step, axis):
+    """One slice, scale 1, sinogram starting at zero: 64-sample blocks of a float coordinate recurrence."""
+    n = vol.shape[0]
+    sn, cs = _lut(na, step)
+    diff = f32(n) - f32(axis) * f32(2)
+    ros, os_, half_n = diff / f32(2), f32(n) / f32(2), f32(0.5) * f32(n)
+    k = np.arange(n)
+    off = (diff < 0) & (k < abs(diff)) | (diff > 0) & (k > f32(axis) * f32(2))
+    out = np.zeros((na, n), f32)
+    for a in range(na):
+        vert = abs(float(sn[a])) <= abs(float(cs[a]))
+        det = f32(1) / cs[a] if vert else f32(-1) / sn[a]
+        st = sn[a] / cs[a] if vert else cs[a] / sn[a]
+        c = ((0.5 + float(ros) + k - float(half_n)) * float(det) + float(-os_ * st) + float(half_n)).astype(f32)
+        img = vol if vert else vol.T
+        total, block = np.zeros(n, f32), np.zeros(n, f32)
+        for r in range(n):
+            block = block + _lerp(img[r], c)
+            c = c + st
+            if r % 64 == 63:
+                total, block = total + block, np.zeros(n, f32)
+        out[a] = np.where(off, f32(0), total + block)
+    return out
+
+
+@pytest.mark.parametrize("special", [False, True])
+@pytest.mark.parametrize("n,slices,axis", [(129, 1, 64.5), (129, 40, 64.5), (800, 1, 400.0), (800, 40, 396.2), (61, 2, 34.0)])
+def test_forward_projector_row_forms_and_non_finite_data(ufoir_lib, gpu_ctx, n, slices, axis, special):
+    na = 37
+    step = f32(np.pi / na)
+    vol = np.random.default_rng(n).standard_normal((slices, n, n)).astype(f32)
+    if special:
+        vol[0, 5, 7], vol[0, n // 2, 3], vol[-1, n - 1, n - 1] = np.inf, -np.inf, np.nan
+    p = ufoir_lib.ParallelProjector(gpu_ctx, step=float(step), is_forward=1, axis_position=axis, angles_num=na)
+    got = p.process(vol)
+    p.close()
+    with np.errstate(invalid="ignore"):
+        for s in sorted({0, slices - 1}):
+            np.testing.assert_array_equal(got[s], _forward(vol[s], na, step, axis))

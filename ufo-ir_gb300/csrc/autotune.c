@@ -79,7 +79,7 @@ static int time_shape(ufoir_projector *p, const udev_fp_cfg *c, const float *P, 
     for (int r = 0; r < 3; r++) {
         float t = 0.0f;
         if ((rc = udev_timer_begin(d)) ||
-            (rc = udev_fp_tiles_cfg(d, &g, c, tiles, n_tiles, P, TP, sino, NULL, 0, sino, -1.0f, slices)) ||
+            (rc = udev_fp_tiles_cfg(d, &g, c, tiles, n_tiles, P, TP, NULL, sino, NULL, 0, sino, -1.0f, slices)) ||
             (rc = udev_timer_end(d, &t)))
             return rc;
         if (r > 0 && t < best)
@@ -162,6 +162,7 @@ int ufoir__fp_tune(ufoir_projector *p, int n_slices, ufoir_fp_tuning *out)
     static const int As[3] = {8, 4, 2};
     static const int Js[4] = {1, 2, 4, 8};
     static const int Ks[3] = {32, 16, 8};
+    static const int Ds[5] = {1, 2, 3, 4, 8};
     const int sm = udev_sm_count(d);
     for (int ia = 0; ia < 3; ia++) {
         const int A = As[ia];
@@ -172,8 +173,10 @@ int ufoir__fp_tune(ufoir_projector *p, int n_slices, ufoir_fp_tuning *out)
         for (int ij = 0; ij < 4; ij++)
             for (int win = 0; win <= 1; win++)
                 for (int ik = 0; ik < 3; ik++)
-                    for (int ds = 1; ds <= 8; ds *= 2) {
-                        if ((ds > 1 || win) && !underfilled)
+                    for (int id = 0; id < 5; id++) {
+                        const int ds = Ds[id];
+                        /* windows and many parts pay where tiles are few */
+                        if ((ds > 4 || win) && !underfilled)
                             continue;
                         udev_fp_cfg c;
                         memset(&c, 0, sizeof(c));
@@ -255,7 +258,7 @@ int ufoir__fp_tune_wanted(ufoir_projector *p, int n_slices)
     int n_tiles = 0;
     const int rc = ufoir__fp_shape(p, n_slices, &c, &tiles, &n_tiles);
     p->fp_cfg_valid = valid;
-    return rc == UFOIR_OK && c.dsplit > 1;
+    return rc == UFOIR_OK && c.dsplit > 1 && (long long) n_tiles * n_slices < udev_sm_count(p->ctx->dev);
 }
 
 int ufoir_projector_autotune(ufoir_projector *proj, size_t n_slices, ufoir_fp_tuning *out)

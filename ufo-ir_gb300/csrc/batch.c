@@ -383,7 +383,7 @@ int ufoir__batch_build(ufoir_ctx *ctx, const ufoir__bmember *mem, int n, ufoir_b
         const int nt = (int) m->cost;
         int slices = mem[i].shape_slices;
         if (total >= 2LL * sm && nt > 0) {
-            const int fill = (2 * sm + nt - 1) / nt;
+            const int fill = (16 * sm + nt - 1) / nt;
             slices = slices > fill ? slices : fill;
         }
         m->p = mem[i].p;
@@ -425,8 +425,8 @@ int ufoir__batch_launch(ufoir_batch *b, unsigned int iterations)
 
 /* The launch-shape slice count of each geometry. When the batch's tiles fill
  * the GPU twice over, a member's shape is chosen as for a GPU full of work
- * (as many slices as fill it with this geometry's tiles): no detector
- * splits, whose extra CTAs only pay when a projection has too few tiles.
+ * (as many slices as fill it many times with this geometry's tiles, so that
+ * members of one size get one shape whatever their angle counts).
  * Otherwise as for the members sharing the geometry alone. */
 static int shape_slices(ufoir_ctx *ctx, ufoir_projector **projs, const int *count, int n_projs, int *eff)
 {
@@ -446,7 +446,7 @@ static int shape_slices(ufoir_ctx *ctx, ufoir_projector **projs, const int *coun
     for (int g = 0; g < n_projs && !rc; g++) {
         eff[g] = count[g];
         if (total >= 2LL * sm && tiles[g] > 0) {
-            const int fill = (2 * sm + tiles[g] - 1) / tiles[g];
+            const int fill = (16 * sm + tiles[g] - 1) / tiles[g];
             eff[g] = eff[g] > fill ? eff[g] : fill;
         }
     }
@@ -596,10 +596,9 @@ int ufoir_batch_create(ufoir_ctx *ctx, const ufoir_batch_job *jobs, size_t n_job
         m->lambda = j->relaxation_factor;
         m->cost = 2.0 * (double) nn * (double) nn * (double) j->n_angles;
         UFOIR_TRY(ufoir__alloc(ctx, &m->resid, ns));
-        UFOIR_TRY(ufoir__alloc(ctx, &m->P, nn * pitch));
+        UFOIR_TRY(ufoir__alloc(ctx, &m->P, nn * pitch + 1));     /* and the non-finite flag */
         UFOIR_TRY(ufoir__alloc(ctx, &m->TP, nn * pitch));
-        UFOIR_TRY(udev_memset(d, m->P, 0, nn * pitch * sizeof(float)));
-        UFOIR_TRY(udev_memset(d, m->TP, 0, nn * pitch * sizeof(float)));
+        UFOIR_TRY(udev_memset(d, m->P + nn * pitch, 0, sizeof(int)));
         if (!j->keep_vol)
             UFOIR_TRY(udev_fill(d, m->x, nn * nn, 0.0f));
     }

@@ -49,9 +49,11 @@ struct ufoir_projector {
 };
 
 /* Scratch of the tiled forward projector: the padded copy and the padded
- * transpose of n_slices volumes (pad columns zero). */
+ * transpose of n_slices volumes, and the flag after P that says whether any
+ * of them was not finite (sticky: it only selects the filter's form). */
 typedef struct {
     float *P, *TP;
+    int *nonfinite;
     size_t slices;
 } ufoir_fp_scratch;
 

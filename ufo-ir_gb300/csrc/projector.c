@@ -400,15 +400,16 @@ int ufoir__fp_scratch_alloc(ufoir_projector *p, ufoir_fp_scratch *s, size_t slic
 {
     const size_t n = p->n_dets, pitch = (size_t) udev_fp_pitch((int) n);
     s->P = s->TP = NULL;
+    s->nonfinite = NULL;
     s->slices = slices;
     const size_t count = n * pitch * slices;
-    int rc = ufoir__alloc(p->ctx, &s->P, count);
+    int rc = ufoir__alloc(p->ctx, &s->P, count + 1);
     if (!rc)
         rc = ufoir__alloc(p->ctx, &s->TP, count);
-    if (!rc)
-        rc = udev_memset(p->ctx->dev, s->P, 0, count * sizeof(float));
-    if (!rc)
-        rc = udev_memset(p->ctx->dev, s->TP, 0, count * sizeof(float));
+    if (!rc) {
+        s->nonfinite = (int *) (s->P + count);
+        rc = udev_memset(p->ctx->dev, s->nonfinite, 0, sizeof(int));
+    }
     if (rc)
         ufoir__fp_scratch_free(p, s);
     return rc;
@@ -419,12 +420,13 @@ void ufoir__fp_scratch_free(ufoir_projector *p, ufoir_fp_scratch *s)
     ufoir__free(p->ctx, s->P);
     ufoir__free(p->ctx, s->TP);
     s->P = s->TP = NULL;
+    s->nonfinite = NULL;
 }
 
 int ufoir__fp_prepare(ufoir_projector *p, ufoir_fp_scratch *s, const float *vol, int n_slices)
 {
     if (udev_fp_tile_angles(p->ctx->dev, (int) p->n_dets) > 0)
-        return udev_pad_transpose(p->ctx->dev, vol, s->P, s->TP, (int) p->n_dets, n_slices);
+        return udev_pad_transpose(p->ctx->dev, vol, s->P, s->TP, s->nonfinite, (int) p->n_dets, n_slices);
     /* the tiled kernel cannot serve this size: plain transpose for the row kernel */
     return udev_transpose(p->ctx->dev, vol, s->TP, (int) p->n_dets, n_slices);
 }
@@ -439,8 +441,8 @@ int ufoir__fp_project(ufoir_projector *p, ufoir_fp_scratch *s, const float *vol,
     int n_tiles = 0;
     const int rc = ufoir__fp_shape(p, n_slices, &c, &tiles, &n_tiles);
     if (rc == UFOIR_OK)
-        return udev_fp_tiles_cfg(p->ctx->dev, &g, &c, tiles, n_tiles, s->P, s->TP, src, w, w_shared, out, scale,
-                                 n_slices);
+        return udev_fp_tiles_cfg(p->ctx->dev, &g, &c, tiles, n_tiles, s->P, s->TP, s->nonfinite, src, w, w_shared,
+                                 out, scale, n_slices);
     if (rc != UFOIR_ERR_UNSUPPORTED)
         return rc;
     return udev_fp(p->ctx->dev, &g, 0, (int) p->n_angles, -1, vol, s->TP, src, w, w_shared, out, scale, n_slices);
@@ -469,7 +471,7 @@ static int siddon_fp(ufoir_projector *p, ufoir_fp_scratch *s, int a0, int na, co
 {
     udev_geom g;
     ufoir__projector_geom(p, &g);
-    int rc = udev_pad_transpose(p->ctx->dev, dvol, s->P, s->TP, (int) p->n_dets, n_slices);
+    int rc = udev_pad_transpose(p->ctx->dev, dvol, s->P, s->TP, s->nonfinite, (int) p->n_dets, n_slices);
     if (!rc)
         rc = udev_siddon_fp(p->ctx->dev, &g, a0, na, s->P, s->TP, dsino, NULL, 0, dsino, p->prm.correction_scale,
                             n_slices);

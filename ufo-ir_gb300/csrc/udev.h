@@ -129,16 +129,9 @@ int udev_fp_pitch(int n);
 /* Angles per CTA tile for n detectors; 0 if the tiled kernel cannot serve n. */
 int udev_fp_tile_angles(udev *d, int n);
 /* Writes the padded copy and the padded transpose of n_slices n x n images
- * into buffers of n * pitch floats per slice whose pad columns are zero. */
-int udev_pad_transpose(udev *d, const float *vol, float *volP, float *volTP, int n, int n_slices);
-/* Same contract as udev_fp over all angles, reading the padded images.
- * d_tiles: device array of int4 {first angle, count, direction, 0};
- * tile_spread: an upper bound, in columns, of how far the rays of one
- * detector at one row lie apart over the angles of a tile (computed by the
- * projector with its tiles), used to size the column windows of split tiles. */
-int udev_fp_tiles(udev *d, const udev_geom *g, const void *d_tiles, int n_tiles, float tile_spread,
-                  const float *volP, const float *volTP, const float *src, const float *w, int w_shared,
-                  float *out, float scale, int n_slices);
+ * into buffers of n * pitch floats per slice, pad columns included; sets
+ * *nonfinite (device int) where an image holds an infinity or a NaN. */
+int udev_pad_transpose(udev *d, const float *vol, float *volP, float *volTP, int *nonfinite, int n, int n_slices);
 /* Launch shape of the tiled forward projector. J detector pairs per thread
  * and angle slot, A angles per tile (the tile list must have been built with
  * A), win: detector-split CTAs stage column windows, K rows per chunk
@@ -151,23 +144,28 @@ typedef struct {
     int fm;                        /* fast arithmetic (from the geometry) */
     size_t smem;
 } udev_fp_cfg;
-/* The fixed rules (what udev_fp_tiles uses) for n_tiles tiles of the
- * default angle count and n_slices slices. */
+/* The fixed rules for n_tiles tiles of the default angle count and n_slices
+ * slices. tile_spread: an upper bound, in columns, of how far the rays of one
+ * detector at one row lie apart over the angles of a tile (computed by the
+ * projector with its tiles), used to size the column windows of split tiles. */
 int udev_fp_default_cfg(udev *d, const udev_geom *g, int n_tiles, int n_slices, float tile_spread, udev_fp_cfg *c);
 /* Fills the derived fields of a shape given J, A, win, K, dsplit;
  * UFOIR_ERR_UNSUPPORTED if no kernel or not enough shared memory serves it. */
 int udev_fp_cfg_finish(udev *d, const udev_geom *g, float tile_spread, udev_fp_cfg *c);
-/* udev_fp_tiles with an explicit shape. */
+/* Same contract as udev_fp over all angles, reading the padded images.
+ * d_tiles: device array of int4 {first angle, count, direction, 0};
+ * nonfinite: what udev_pad_transpose set (NULL: the images are finite). */
 int udev_fp_tiles_cfg(udev *d, const udev_geom *g, const udev_fp_cfg *c, const void *d_tiles, int n_tiles,
-                      const float *volP, const float *volTP, const float *src, const float *w, int w_shared,
-                      float *out, float scale, int n_slices);
+                      const float *volP, const float *volTP, const int *nonfinite, const float *src, const float *w,
+                      int w_shared, float *out, float scale, int n_slices);
 
 /* ---- Mixed batches: one launch per kernel over many one-slice jobs ----
  * Each job contributes an opaque record (built on the host by *_record,
  * copied to device memory by the caller) and `items` CTAs; item_start is
  * the exclusive prefix sum of the items (n_jobs entries, device memory),
  * job_index maps a record to its entry of the active array (device ints;
- * 0 = skip the job). */
+ * 0 = skip the job). A member's padded copy (volP) is followed by its
+ * non-finite flag: n * pitch floats, then an int. */
 size_t udev_fp_record_bytes(void);
 /* 1 if a shape's shared memory leaves room for the batch kernel's record. */
 int udev_fp_batch_fits(const udev *d, const udev_fp_cfg *c);

@@ -21,6 +21,14 @@
  * row), one 1-D copy per row, with two zero slots after the window for taps
  * outside it (they lie outside the image). 2900^2 x 90 angles: 925 -> 818 us.
  *
+ * Bound by the FMA pipe and, at one CTA per SM, by the barrier at each chunk.
+ * 16 slices of 1448^2 x 1200: 13.03 -> 11.72 ms, two of 2900^2 x 360 3.53 ->
+ * 2.58, six of 1001^2 x 451 1.21 -> 0.92, one of 724^2 x 360 0.151 -> 0.104,
+ * from three changes: the filter's three-operation form on finite data (3 %
+ * at 16 slices; the padding pass says whether they are), row ranges per warp
+ * in place of a comparison of every ray at every chunk (3 to 14 %), and two
+ * or more CTAs per tile with whole rows (fp_split_cost).
+ *
  * Arithmetic is the reference's: per ray, the float coordinate recurrence,
  * one linear-filter sample per row with (1 - t) * T0 + t * T1, samples
  * summed in blocks of 64, then sino = src + scale * sum
@@ -41,6 +49,7 @@ namespace {
 
 constexpr int kPadL = 2;
 constexpr int kHeader = 256;   /* shared bytes before the stages: barriers, window starts, extreme rays */
+constexpr int kStages = 2;     /* row chunks in shared memory (double buffered) */
 /* bits of floor(c - 0.5) + 1.5 * 2^23, less the padded column of index 0 */
 constexpr int kColBits = joseph::kFloorMagicBits - kPadL;
 
@@ -67,6 +76,8 @@ struct FpTileArgs {
     int wcols;             /* columns staged per row: pitch (whole rows), or a window of the CTA's rays */
     int wstride;           /* shared floats per staged row (wcols + 4 for windows: 2 zero slots) */
     int margin;            /* window margin in columns (the recurrence's drift and the filter's taps) */
+    float drift;           /* bound of the coordinate recurrence's error over n rows, in columns */
+    const int *nonfinite;  /* non-zero where the volume holds infinities or NaNs (null: it does not) */
     int skip_chunk;        /* testing: row chunk whose barrier never completes (-1 = none) */
     int *err;
 };
@@ -76,6 +87,38 @@ static_assert(sizeof(FpTileArgs) % sizeof(int) == 0, "records are copied as ints
 constexpr size_t kBatchStatic = (sizeof(FpTileArgs) + 16 + 127) / 128 * 128;
 
 constexpr int kMaxWinThreads = 448;   /* detector-split CTAs hold at most half the slots */
+
+/* Rows of a ray with coordinate c + r st (r in [0, n)) inside [lo, hi): an
+ * inner bound [a, b) where `inner`, else an outer one. An empty set gives
+ * a = n, b = 0. */
+__device__ __forceinline__ void ray_rows(float c, float st, float lo, float hi, int n, bool inner, int &a, int &b)
+{
+    a = n;
+    b = 0;
+    if (!(fabsf(c) < 1e9f) || !(fabsf(st) < 1e9f)) {   /* no geometry: never inside, never outside */
+        if (!inner) {
+            a = 0;
+            b = n;
+        }
+        return;
+    }
+    if (fabsf(st) < 1e-6f) {       /* moves less than 0.01 column over the image */
+        if (c >= lo && c < hi) {
+            a = 0;
+            b = n;
+        }
+        return;
+    }
+    const float inv = __fdividef(1.0f, st), fn = (float) n;
+    const float x = (lo - c) * inv, y = (hi - c) * inv;
+    const float x0 = fminf(fmaxf(fminf(x, y), -4.0f), fn + 4.0f), x1 = fminf(fmaxf(fmaxf(x, y), -4.0f), fn + 4.0f);
+    if (x1 < -2.0f || x0 > fn + 2.0f)
+        return;
+    const int ia = inner ? (int) ceilf(x0) + 1 : (int) floorf(x0) - 1;
+    const int ib = inner ? (int) floorf(x1) : (int) ceilf(x1) + 2;
+    a = min(max(ia, 0), n);
+    b = min(max(ib, 0), n);
+}
 
 /* Windowed CTAs of the J = 1 variants made for large n (A <= 4) hold few
  * rays per thread: two of them per SM. (The A = 8 variant, the default at
@@ -88,6 +131,7 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
 {
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem_raw);
     int *w0s = reinterpret_cast<int *>(smem_raw + 16);     /* window start of each stage */
+    int *wok = reinterpret_cast<int *>(smem_raw + 24);     /* the window holds every tap inside the image */
     float *ext = reinterpret_cast<float *>(smem_raw + 32);   /* [3][A]: extreme rays' starts, steps */
     float *stage0 = reinterpret_cast<float *>(smem_raw + kHeader);
     const int K = P.rows_per_chunk;
@@ -113,14 +157,15 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
      * adjacent detectors of one angle (spread 1/|cos| apart) are not.
      * A thread owns A/2 angles x 2J detectors d0 + 16 i, so a warp's rays
      * are 32J adjacent detectors of A adjacent angles, which cross the
-     * image together (see the chunk modes below); detectors (2m, 2m + 1) of
+     * image together (see the row ranges below); detectors (2m, 2m + 1) of
      * one angle travel as a pair through packed FP32. Slots past the tile's
      * angles or the CTA's detectors repeat its last angle or detector (their
      * sums are not written), so every slot holds a ray of the image. */
+    const bool nonfinite = !FM && P.nonfinite && __ldg(P.nonfinite) != 0;
     constexpr int A2 = A / 2;
-    const int lane = (int) (threadIdx.x & 31);
+    const int lane = (int) (threadIdx.x & 31), warp = (int) (threadIdx.x >> 5);
     const int g = lane >> 4;
-    const int d0 = dstart + (int) (threadIdx.x >> 5) * 32 * J + (lane & 15);
+    const int d0 = dstart + warp * 32 * J + (lane & 15);
     float2 c[A2][J], inner[A2][J], sum[A2][J], stp[A2];
 #pragma unroll
     for (int k = 0; k < A2; ++k) {
@@ -154,7 +199,7 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
         ext[2 * A + a] = st;
     }
     /* window start (a multiple of 4 columns) of the chunk at row r0 */
-    auto window = [&](int r0, int rows) -> int {
+    auto window = [&](int r0, int rows, int st_) -> int {
         /* in FP32: the rounding (< 1e-3 column here) is covered by the margin */
         float lo = 1e30f, hi = -1e30f;
         const float ya = (float) r0, yb = (float) (r0 + rows - 1);
@@ -169,6 +214,7 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
         w0 = max(0, min(w0, pitch - wcols));
         if (min(chi, kPadL + n - 1) >= w0 + wcols)
             atomicOr(P.err, tma::kErrWindow);      /* the host's width bound was too small */
+        wok[st_] = min(chi, pitch - 1) < w0 + wcols && max(clo, 0) >= w0;
         return w0;
     };
     if (threadIdx.x == 0) {
@@ -196,7 +242,7 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
             tma::mbar_arrive_expect_tx(&bars[ch & 1], bytes + extra);
             tma::bulk_g2s(dst, img + (size_t) r0 * pitch, bytes, &bars[ch & 1]);
         } else {
-            const int w0 = window(r0, rows);
+            const int w0 = window(r0, rows, ch & 1);
             w0s[ch & 1] = w0;
             tma::mbar_arrive_expect_tx(&bars[ch & 1], (uint32_t) (rows * wcols) * 4u + extra);
             for (int r = 0; r < rows; ++r)
@@ -209,22 +255,43 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
         for (; issued < 2 && issued < nchunks; ++issued)
             issue(issued);
 
+    /* Row ranges of the warp, from its rays' linear coordinates and the
+     * recurrence's error bound (once per tile, while the first copies are in
+     * flight; lane = angle and end of the warp's detectors, between which a
+     * ray's coordinate at a row is monotone; comparing every ray's
+     * coordinates at every chunk cost 9 % of the kernel's instructions):
+     *  - [rin0, rin1): every ray's coordinate lies in [0.5, n + 1.5), so
+     *    floor(c - 0.5) takes the three-operation form (floor_half2) and the
+     *    tap address is one multiply-add on its bits, with no clamp;
+     *  - before rout0 and from rout1 on: every coordinate is below -0.5 or at
+     *    least n + 0.5, where both taps are border zeros. Only the recurrence
+     *    advances: adding +-0 leaves a block sum unchanged (it starts at +0
+     *    and a sum of finite floats in round-to-nearest is never -0);
+     *  - the rows between take the general form. */
+    int rin0, rin1, rout0, rout1;
+    {
+        const int angle = tile.x + min(lane % A, tile.y - 1);
+        const int s = min(dstart + warp * 32 * J + (lane / A & 1) * (32 * J - 1), dend - 1);
+        /* in FP32 and fast division: the error (< 0.01 column) is part of P.drift */
+        const float sn = __ldg(P.sinv + angle), cs = __ldg(P.cosv + angle);
+        const float inv = __fdividef(1.0f, dir == 0 ? sn : cs), st = (dir == 0 ? cs : sn) * inv;
+        const float cc = fmaf(0.5f + kc.ros + (float) s - 0.5f * (float) n, dir == 0 ? -inv : inv,
+                              fmaf(-kc.os, st, 0.5f * (float) n));
+        ray_rows(cc, st, 0.5f + P.drift, (float) n + 1.5f - P.drift, n, true, rin0, rin1);
+        ray_rows(cc, st, -0.5f - P.drift, (float) n + 0.5f + P.drift, n, false, rout0, rout1);
+        rin0 = __reduce_max_sync(0xffffffffu, rin0);
+        rin1 = __reduce_min_sync(0xffffffffu, rin1);
+        rout0 = __reduce_min_sync(0xffffffffu, rout0);
+        rout1 = __reduce_max_sync(0xffffffffu, rout1);
+        /* the inside form's filter (joseph::lerp2n) needs finite data */
+        if (rin0 >= rin1 || nonfinite)
+            rin0 = rin1 = n + 64;
+    }
+
     /* A tap pair starts at padded column floor(c - 0.5) + kPadL; pairs that
-     * start outside [0, n + 2] lie wholly in the zero border, so the start
-     * is clamped (as unsigned) to n + 2, whose taps are two pad zeros.
-     * Each warp picks one of three forms per chunk, from its rays'
-     * coordinates at the chunk's first and last rows (monotone along a ray;
-     * the float recurrence drifts < 0.03 columns over a chunk, and the
-     * bounds keep 0.25):
-     *  - inside: every coordinate lies in [0.5, n + 1.5) and in the staged
-     *    columns, so floor(c - 0.5) takes the three-operation form
-     *    (floor_half2) and the tap address is one multiply-add on its bits,
-     *    with no clamp;
-     *  - outside: every coordinate is below -0.5 or at least n + 0.5, where
-     *    both taps are border zeros. Only the recurrence advances: adding
-     *    +-0 leaves a block sum unchanged (it starts at +0 and a sum of
-     *    finite floats in round-to-nearest is never -0);
-     *  - otherwise the general form above. */
+     * start outside [0, n + 2] lie wholly in the zero border, so the general
+     * form clamps the start (as unsigned) to n + 2, whose taps are two pad
+     * zeros. Each warp picks the form of a chunk from its row ranges. */
     const uint32_t col_lim = (uint32_t) n + 2u;
     const float2 z2 = joseph::splat(P.neg_zero);
     const uint32_t stage_s = (uint32_t) __cvta_generic_to_shared(stage0);
@@ -246,41 +313,26 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
             const int colbits = kColBits + w0;
             const uint32_t lim = WIN ? (uint32_t) wcols : col_lim;
             /* the chunk's form */
-            const float span = (float) (rows - 1);
-            const float in_lo = fmaxf(0.5f, (float) (w0 - kPadL) + 0.5f) + 0.25f;
-            const float in_hi = (float) ((int) lim - kPadL + w0) + 1.25f;
-            const float out_hi = (float) n + 0.75f;
-            bool inside = true, outside = true;
-#pragma unroll
-            for (int k = 0; k < A2; ++k)
-#pragma unroll
-                for (int m = 0; m < J; ++m) {
-                    const float ex = fmaf(span, stp[k].x, c[k][m].x), ey = fmaf(span, stp[k].y, c[k][m].y);
-                    const float lo = fminf(fminf(c[k][m].x, ex), fminf(c[k][m].y, ey));
-                    const float hi = fmaxf(fmaxf(c[k][m].x, ex), fmaxf(c[k][m].y, ey));
-                    inside = inside && lo >= in_lo && hi < in_hi;
-                    const bool xo = fmaxf(c[k][m].x, ex) < -0.75f || fminf(c[k][m].x, ex) >= out_hi;
-                    const bool yo = fmaxf(c[k][m].y, ey) < -0.75f || fminf(c[k][m].y, ey) >= out_hi;
-                    outside = outside && xo && yo;
-                }
-            inside = __all_sync(0xffffffffu, inside);
-            outside = !inside && __all_sync(0xffffffffu, outside);
+            const bool inside = r0 >= rin0 && r0 + rows <= rin1 && (!WIN || wok[st]);
+            const bool outside = r0 + rows <= rout0 || r0 >= rout1;
             if (inside) {
                 /* address = row + 4 (floor(c - 0.5) + kPadL - w0) = base + 4 bits(y) */
                 uint32_t base = row_s0 + 4u * (uint32_t) (kPadL - w0) - 4u * (uint32_t) joseph::kHalfFloorBits;
+/* more rows at once outgrow the instruction cache at small n */
+#pragma unroll (J == 1 ? 2 : 4)
                 for (int r = 0; r < rows; ++r, base += 4u * (uint32_t) wstride) {
 #pragma unroll
                     for (int k = 0; k < A2; ++k) {
 #pragma unroll
                         for (int m = 0; m < J; ++m) {
                             float2 t;
-                            const float2 y = joseph::floor_half2(c[k][m], t);
+                            const float2 y = FM ? joseph::floor_half2(c[k][m], t) : joseph::floor_half2n(c[k][m], t);
                             const uint32_t a0 = base + 4u * (uint32_t) __float_as_int(y.x);
                             const uint32_t a1 = base + 4u * (uint32_t) __float_as_int(y.y);
                             const float2 t0 = make_float2(joseph::lds(a0), joseph::lds(a1));
                             const float2 t1 = make_float2(joseph::lds(a0 + 4u), joseph::lds(a1 + 4u));
                             inner[k][m] = FM ? joseph::lerp_acc_fast2(inner[k][m], t, t0, t1)
-                                             : joseph::add2(inner[k][m], joseph::lerp2(t, t0, t1, z2));
+                                             : joseph::add2(inner[k][m], joseph::lerp2n(t, t0, t1, z2));
                             c[k][m] = joseph::add2(c[k][m], stp[k]);
                         }
                     }
@@ -295,6 +347,7 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
                 }
             } else {
                 uint32_t row_s = row_s0;
+#pragma unroll 1
                 for (int r = 0; r < rows; ++r, row_s += 4u * (uint32_t) wstride) {
 #pragma unroll
                     for (int k = 0; k < A2; ++k) {
@@ -423,31 +476,48 @@ __global__ void __launch_bounds__(WIN ? kMaxWinThreads : 768, (WIN && J == 1 && 
     fp_tile<J, A, WIN, FM>(rec, local / rec.dsplit, local % rec.dsplit, 0, smem_raw);
 }
 
-/* Writes the padded copy and the padded transpose of n x n slices; the pad
- * columns are left as they are (zeroed once when the buffers are made). */
-__global__ void __launch_bounds__(256) pad_transpose_kernel(const float *__restrict__ in, float *__restrict__ outP,
-                                                            float *__restrict__ outTP, int n, int pitch,
-                                                            long long in_stride, long long out_stride)
+/* One 32 x 32 block (bx, by) of an image's padded copy and padded transpose,
+ * with the zero pad columns beside it where it lies at a row's end; sets
+ * *nonfinite where it meets an infinity or a NaN. 32 x 8 threads. */
+__device__ __forceinline__ void pad_block(const float *__restrict__ src, float *__restrict__ dp, float *__restrict__ dt,
+                                          int n, int pitch, int bx, int by, int *nonfinite, float (&tile)[32][33])
 {
-    __shared__ float tile[32][33];
-    const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
-    const float *src = in + (size_t) blockIdx.z * in_stride;
-    float *dp = outP + (size_t) blockIdx.z * out_stride;
-    float *dt = outTP + (size_t) blockIdx.z * out_stride;
+    const int tx = (int) threadIdx.x;
     for (int j = threadIdx.y; j < 32; j += 8) {
-        const int x = bx + threadIdx.x, y = by + j;
+        const int x = bx + tx, y = by + j;
         if (x < n && y < n) {
             const float v = src[(size_t) y * n + x];
-            tile[j][threadIdx.x] = v;
+            tile[j][tx] = v;
             dp[(size_t) y * pitch + kPadL + x] = v;
+            if (!(fabsf(v) <= 3.402823466e38f))
+                atomicOr(nonfinite, 1);
         }
+        if (bx == 0 && tx < kPadL && y < n)
+            dp[(size_t) y * pitch + tx] = 0.0f;
+        if (bx + 32 >= n && kPadL + n + tx < pitch && y < n)
+            dp[(size_t) y * pitch + kPadL + n + tx] = 0.0f;
     }
     __syncthreads();
     for (int j = threadIdx.y; j < 32; j += 8) {
-        const int x = by + threadIdx.x, y = bx + j;
+        const int x = by + tx, y = bx + j;
         if (x < n && y < n)
-            dt[(size_t) y * pitch + kPadL + x] = tile[threadIdx.x][j];
+            dt[(size_t) y * pitch + kPadL + x] = tile[tx][j];
+        if (by == 0 && tx < kPadL && y < n)
+            dt[(size_t) y * pitch + tx] = 0.0f;
+        if (by + 32 >= n && kPadL + n + tx < pitch && y < n)
+            dt[(size_t) y * pitch + kPadL + n + tx] = 0.0f;
     }
+}
+
+/* Writes the padded copy and the padded transpose of n x n slices. */
+__global__ void __launch_bounds__(256) pad_transpose_kernel(const float *__restrict__ in, float *__restrict__ outP,
+                                                            float *__restrict__ outTP, int *nonfinite, int n, int pitch,
+                                                            long long in_stride, long long out_stride)
+{
+    __shared__ float tile[32][33];
+    pad_block(in + (size_t) blockIdx.z * in_stride, outP + (size_t) blockIdx.z * out_stride,
+              outTP + (size_t) blockIdx.z * out_stride, n, pitch, (int) blockIdx.x * 32, (int) blockIdx.y * 32,
+              nonfinite, tile);
 }
 
 struct TileCfg {
@@ -467,9 +537,9 @@ TileCfg tile_cfg(int n, int smem_optin)
     c.threads = (slots + 15) / 16 * 32;
     const int pitch = udev_fp_pitch(n);
     c.K = 32;
-    while (c.K > 4 && kHeader + 2 * (size_t) c.K * pitch * 4 > (size_t) smem_optin)
+    while (c.K > 4 && kHeader + kStages * (size_t) c.K * pitch * 4 > (size_t) smem_optin)
         c.K /= 2;
-    c.smem = kHeader + 2 * (size_t) c.K * pitch * 4;
+    c.smem = kHeader + kStages * (size_t) c.K * pitch * 4;
     return c;
 }
 
@@ -500,6 +570,36 @@ int launch_tiles(udev *d, const FpTileArgs &args, int n_tiles, int n_slices, int
 extern "C" int udev_fp_pitch(int n)
 {
     return (n + kPadL + 2 + 3) / 4 * 4;
+}
+
+/* Threads of a CTA with 1 / dsplit of n detectors, J pairs per thread and angle slot. */
+static int fp_threads(int n, int dsplit, int J)
+{
+    const int dper = (n + dsplit - 1) / dsplit, slots = (dper + 2 * J - 1) / (2 * J);
+    return (slots + 15) / 16 * 32;
+}
+
+/*
+ * Relative time of a launch of `ctas` tiles with their detectors in ds parts
+ * of whole rows each. A part costs its warps; an SM that gets more parts than
+ * the mean sets the end of a short launch. Two parts per tile beat one also
+ * where tiles abound (4.6 % at 16 slices of 1448^2 x 1200: 12.23 -> 11.69 ms;
+ * two CTAs of 384 threads wait at their own barriers where one of 736 stops
+ * the SM); more parts stage every row more often (11.89 and 12.12 ms at 3 and
+ * 4). Measured ms at 1 / 2 / 3 / 4 parts against the rule's choice (*):
+ *   6 x 1001^2 x 451  1.165 / 0.929* / 1.038 / 0.969
+ *   4 x 724^2 x 360   0.447 / 0.344 / 0.334* / 0.367
+ *   2 x 724^2 x 360   0.244 / 0.238 / 0.191* / 0.221
+ *   2 x 2900^2 x 360  3.025 / 2.540*   (more parts do not fit two to an SM)
+ *   1 x 1001^2 x 451  0.403 / 0.282* / 0.340 / 0.309
+ *   1 x 512^2 x 400   0.129 / 0.088* / 0.100 / 0.092
+ */
+static double fp_split_cost(long long ctas, int sms, int threads, int ds)
+{
+    static const double pen[5] = {0.0, 1.046, 1.0, 1.02, 1.08};
+    const double mean = (double) (ctas * ds) / sms;
+    const double most = mean >= 8.0 ? mean : (double) ((ctas * ds + sms - 1) / sms);
+    return pen[ds] * (threads / 32) * (0.7 * most + 0.3 * mean);
 }
 
 static bool tiles_supported(const TileCfg &cfg, int smem_optin)
@@ -551,7 +651,8 @@ int udev_kernels_init(udev *d)
     return rc ? rc : udev_sart_init(d);
 }
 
-extern "C" int udev_pad_transpose(udev *d, const float *vol, float *volP, float *volTP, int n, int n_slices)
+extern "C" int udev_pad_transpose(udev *d, const float *vol, float *volP, float *volTP, int *nonfinite, int n,
+                                  int n_slices)
 {
     if (n_slices <= 0)
         return UFOIR_OK;
@@ -561,8 +662,8 @@ extern "C" int udev_pad_transpose(udev *d, const float *vol, float *volP, float 
         const int chunk = n_slices - done > 65535 ? 65535 : n_slices - done;
         dim3 grid(udev_div_up(n, 32), udev_div_up(n, 32), (unsigned int) chunk);
         pad_transpose_kernel<<<grid, dim3(32, 8), 0, d->stream>>>(
-            vol + (size_t) done * n * n, volP + (size_t) done * n * pitch, volTP + (size_t) done * n * pitch, n, pitch,
-            (long long) n * n, (long long) n * pitch);
+            vol + (size_t) done * n * n, volP + (size_t) done * n * pitch, volTP + (size_t) done * n * pitch, nonfinite, n,
+            pitch, (long long) n * n, (long long) n * pitch);
         int rc = udev_after_launch(d, "pad_transpose_kernel");
         if (rc)
             return rc;
@@ -608,7 +709,7 @@ extern "C" int udev_fp_cfg_finish(udev *d, const udev_geom *g, float tile_spread
         c->wcols = wc;
         c->wstride = wc + 4;
     }
-    c->smem = kHeader + 2 * (size_t) c->K * c->wstride * 4;
+    c->smem = kHeader + kStages * (size_t) c->K * c->wstride * 4;
     if (c->smem > (size_t) d->smem_optin)
         return UFOIR_ERR_UNSUPPORTED;
     return UFOIR_OK;
@@ -635,29 +736,58 @@ extern "C" int udev_fp_default_cfg(udev *d, const udev_geom *g, int n_tiles, int
     c->wcols = c->wstride = pitch;
     c->margin = 4 + n / 512;
     c->smem = cfg.smem;
-    /* Too few tiles to fill the GPU (one slice, few angles): split each
-     * angle tile's detectors over up to 8 CTAs, with chunks small enough
-     * for two CTAs per SM. Every CTA walks all rows; it stages only the
-     * window of columns its rays can reach (the detector range times
-     * max |det_step| = sqrt 2, the chunk's rows times max |step| = 1, the
-     * spread of the tile's angles, and a margin), unless that is the whole
-     * row. */
+    /* A tile's detectors may be spread over several CTAs, each walking all
+     * rows for its range (fp_split_cost says when that pays). */
     const long long ctas = (long long) n_tiles * n_slices;
-    if (ctas < d->sm_count) {
+    const int sms = d->sm_count;
+    if (4 * ctas >= sms) {
+        double best = fp_split_cost(ctas, sms, cfg.threads, 1);
+        for (int ds = 2; ds <= 4; ++ds) {
+            udev_fp_cfg w = *c;
+            w.dsplit = ds;
+            if ((n + ds - 1) / ds < 64)
+                break;
+            /* rows per chunk: as many as leave room for the CTAs that the
+             * registers allow and the launch has */
+            long long occ = 65536 / (80 * fp_threads(n, ds, cfg.J));
+            const long long per_sm = (ctas * ds + sms - 1) / sms;
+            occ = occ < 1 ? 1 : occ > per_sm ? per_sm : occ;
+            for (w.K = cfg.K > 16 ? 16 : cfg.K; w.K >= 4; w.K /= 2)
+                if (udev_fp_cfg_finish(d, g, tile_spread, &w) == UFOIR_OK &&
+                    (size_t) occ * (w.smem + 1024) <= (size_t) d->smem_optin + 1024)
+                    break;
+            if (w.K < 4)
+                continue;
+            const double cost = fp_split_cost(ctas, sms, w.threads, ds);
+            if (cost < best) {
+                best = cost;
+                *c = w;
+            }
+        }
+        return UFOIR_OK;
+    }
+    /* Fewer tiles than a quarter of the SMs (one slice, few angles): up to 8
+     * CTAs per tile, with chunks small enough for two CTAs per SM, and each
+     * CTA stages only the window of columns its rays can reach (the detector
+     * range times max |det_step| = sqrt 2, the chunk's rows times max |step|
+     * = 1, the spread of the tile's angles, and a margin), unless that is the
+     * whole row. One slice of 2900^2 x 90: 0.639 ms, against 1.30 in two whole-row
+     * parts per tile. */
+    {
         int split = (int) ((2LL * d->sm_count + ctas - 1) / ctas);
         split = split > 8 ? 8 : split;
         while (split > 1 && (n + split - 1) / split < 64)
             split--;
         int k2 = cfg.K;
-        while (k2 > 4 && 2 * (kHeader + 2 * (size_t) k2 * pitch * 4) > (size_t) d->smem_optin)
+        while (k2 > 4 && 2 * (kHeader + kStages * (size_t) k2 * pitch * 4) > (size_t) d->smem_optin)
             k2 /= 2;
-        if (split > 1 && 2 * (kHeader + 2 * (size_t) k2 * pitch * 4) <= (size_t) d->smem_optin) {
+        if (split > 1 && 2 * (kHeader + kStages * (size_t) k2 * pitch * 4) <= (size_t) d->smem_optin) {
             c->dsplit = split;
             c->dper = (n + split - 1) / split;
             const int slots = (c->dper + 2 * cfg.J - 1) / (2 * cfg.J);
             c->threads = (slots + 15) / 16 * 32;
             c->K = k2;
-            c->smem = kHeader + 2 * (size_t) k2 * pitch * 4;
+            c->smem = kHeader + kStages * (size_t) k2 * pitch * 4;
             /* Windowed CTAs take one detector pair per angle slot (J = 1)
              * where that fits: a split CTA holds few rays, and at J = 4
              * (n = 2900) it would run 3 warps of 16 rays per thread, too few
@@ -687,9 +817,18 @@ extern "C" int udev_fp_default_cfg(udev *d, const udev_geom *g, int n_tiles, int
 template <bool FM>
 static int dispatch_tiles(udev *d, const FpTileArgs &A, const udev_fp_cfg *c, int n_tiles, int n_slices);
 
+/* A bound, in columns, of the coordinate recurrence's error over n rows: each
+ * of n additions rounds by at most half an ulp of 2 n (n 2^-23), half a column
+ * of slack beside it. */
+static float recurrence_drift(int n)
+{
+    return 0.5f + (float) n * (float) n * 1.1920929e-7f;
+}
+
 extern "C" int udev_fp_tiles_cfg(udev *d, const udev_geom *g, const udev_fp_cfg *c, const void *d_tiles,
-                                 int n_tiles, const float *volP, const float *volTP, const float *src,
-                                 const float *w, int w_shared, float *out, float scale, int n_slices)
+                                 int n_tiles, const float *volP, const float *volTP, const int *nonfinite,
+                                 const float *src, const float *w, int w_shared, float *out, float scale,
+                                 int n_slices)
 {
     if (n_slices <= 0 || n_tiles <= 0)
         return UFOIR_OK;
@@ -714,6 +853,8 @@ extern "C" int udev_fp_tiles_cfg(udev *d, const udev_geom *g, const udev_fp_cfg 
     A.w_stride = w_shared ? 0 : A.sino_stride;
     A.neg_zero = -0.0f;
     A.err = d->d_err;
+    A.drift = recurrence_drift(n);
+    A.nonfinite = nonfinite;
     A.skip_chunk = d->inject_skip_chunk;   /* one-shot test injection */
     d->inject_skip_chunk = -1;
     A.dsplit = c->dsplit;
@@ -748,19 +889,6 @@ static int dispatch_tiles(udev *d, const FpTileArgs &A, const udev_fp_cfg *c, in
     }
     udev_set_error(d, "fp_tiles: no kernel for J=%d A=%d win=%d", c->J, c->A, c->win);
     return UFOIR_ERR_UNSUPPORTED;
-}
-
-extern "C" int udev_fp_tiles(udev *d, const udev_geom *g, const void *d_tiles, int n_tiles, float tile_spread,
-                             const float *volP, const float *volTP, const float *src, const float *w, int w_shared,
-                             float *out, float scale, int n_slices)
-{
-    if (n_slices <= 0 || n_tiles <= 0)
-        return UFOIR_OK;
-    udev_fp_cfg c;
-    const int rc = udev_fp_default_cfg(d, g, n_tiles, n_slices, tile_spread, &c);
-    if (rc)
-        return rc;
-    return udev_fp_tiles_cfg(d, g, &c, d_tiles, n_tiles, volP, volTP, src, w, w_shared, out, scale, n_slices);
 }
 
 /* ---- mixed batches ---- */
@@ -802,6 +930,8 @@ extern "C" int udev_fp_record(udev *d, const udev_geom *g, const udev_fp_cfg *c,
     A.w_stride = 0;
     A.neg_zero = -0.0f;
     A.err = d->d_err;
+    A.drift = recurrence_drift(n);
+    A.nonfinite = reinterpret_cast<const int *>(volP + (size_t) n * A.pitch);
     A.skip_chunk = -1;
     A.dsplit = c->dsplit;
     A.dper = c->dper;
@@ -895,21 +1025,8 @@ __global__ void __launch_bounds__(256) pad_batch_kernel(const PadRec *__restrict
         return;
     const PadRec r = recs[j];
     const int local = b - __ldg(item_start + j);
-    const int bx = (local % r.tiles_x) * 32, by = (local / r.tiles_x) * 32;
-    for (int k = threadIdx.y; k < 32; k += 8) {
-        const int x = bx + threadIdx.x, y = by + k;
-        if (x < r.n && y < r.n) {
-            const float v = r.vol[(size_t) y * r.n + x];
-            tile[k][threadIdx.x] = v;
-            r.P[(size_t) y * r.pitch + kPadL + x] = v;
-        }
-    }
-    __syncthreads();
-    for (int k = threadIdx.y; k < 32; k += 8) {
-        const int x = by + threadIdx.x, y = bx + k;
-        if (x < r.n && y < r.n)
-            r.TP[(size_t) y * r.pitch + kPadL + x] = tile[threadIdx.x][k];
-    }
+    pad_block(r.vol, r.P, r.TP, r.n, r.pitch, (local % r.tiles_x) * 32, (local / r.tiles_x) * 32,
+              reinterpret_cast<int *>(r.P + (size_t) r.n * r.pitch), tile);
 }
 
 extern "C" size_t udev_pad_record_bytes(void)
