@@ -1,0 +1,56 @@
+"""The reference's float reductions, which are sums in a fixed order, computed
+in parallel: equality is exact. The L1 norm's reference is numpy's running
+float32 sum (one addition after another), the dot product's the oracle.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+KINDS = ("normal", "ones", "ties", "growing", "stagnating", "subnormal", "sparse", "overflow", "inf", "nan")
+
+
+def _values(kind, count):
+    rng = np.random.default_rng(count)
+    x = rng.standard_normal(count).astype(np.float32)
+    if kind == "ones":
+        x[:] = 1.0
+    elif kind == "ties":        # half units of the running sum again and again
+        x = (rng.integers(0, 8, count) * np.float32(0.5)).astype(np.float32)
+        x[0] = 2.0 ** 23 - 1
+    elif kind == "growing":     # a new binade every few elements
+        x = np.exp2(np.linspace(-126, 100, count)).astype(np.float32) * np.sign(x)
+    elif kind == "stagnating":
+        x[: count // 7] *= np.float32(1e7)
+        x[count // 7:] *= np.float32(1e-3)
+    elif kind == "subnormal":
+        x *= np.float32(1e-41)
+    elif kind == "sparse":
+        x[rng.random(count) < 0.98] = -0.0
+    elif kind == "overflow":
+        x *= np.float32(3e37)
+    elif kind in ("inf", "nan"):
+        x[count // 3] = np.inf
+        if kind == "nan":
+            x[count // 2] = np.nan
+    return x
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("h,w", [(1, 1), (1, 5), (7, 73), (16, 32), (63, 65), (301, 433), (1200, 731)])
+def test_compat_l1_norm_is_the_sequential_sum(ufoir_lib, gpu_ctx, h, w, kind):
+    x = _values(kind, h * w).reshape(h, w)
+    with np.errstate(over="ignore", invalid="ignore"):
+        want = np.cumsum(np.abs(x).reshape(-1), dtype=np.float32)[-1]
+    np.testing.assert_array_equal(np.float32(gpu_ctx.l1_norm(x, ufoir_lib.NORM_COMPAT)), want)
+
+
+@pytest.mark.parametrize("h,w", [(1, 1), (3, 17), (33, 31), (65, 300), (367, 367)])
+def test_dot_products(ufoir_lib, gpu_ctx, oracle, h, w):
+    rng = np.random.default_rng(h)
+    a, b = (rng.standard_normal((h, w)).astype(np.float32) for _ in range(2))
+    assert np.float32(gpu_ctx.dot_product(a, b, ufoir_lib.NORM_COMPAT)) == np.float32(oracle.dot_product(a, b))
+    want = oracle.dot_product(a, b, fp64=True)
+    terms = float(np.abs(a.astype(np.float64)).max() * np.abs(b.astype(np.float64)).max()) * h * w
+    # one rounding of the result to float, and FP64 rounding of every sum
+    assert abs(gpu_ctx.dot_product(a, b) - want) <= 2.0 ** -24 * abs(want) + 2.0 ** -50 * terms

@@ -104,9 +104,7 @@ int ufoir__ray_weights(ufoir_projector *p, float *R, float *ones)
         return rc;
     rc = udev_fill(ctx->dev, ones, nv, 1.0f);
     if (!rc)
-        rc = udev_fill(ctx->dev, R, ns, 0.0f);
-    if (!rc)
-        rc = ufoir__fp_full(p, &fs, ones, R, NULL, 0, R, 1.0f, 1);
+        rc = ufoir__fp_full(p, &fs, ones, NULL, NULL, 0, R, 1.0f, 1);
     if (!rc)
         rc = udev_unary(ctx->dev, UDEV_INV, R, 0, 0, R, ns);
     ufoir__fp_scratch_free(p, &fs);
@@ -933,7 +931,7 @@ done:
  * discarded), so each slice sees the same operations in the same order as
  * when it runs alone.
  */
-#define SBTV_MAX_BATCH 16
+#define SBTV_MAX_BATCH UDEV_SBTV_SLICES
 
 typedef struct {
     ufoir_projector *p;
@@ -943,7 +941,7 @@ typedef struct {
     int S;
     float lambda, mu;
     int mode;
-    float *tmpA, *tmpAt, *tmpD, *tmpDxt;
+    float *tmpA, *tmpAt;
     ufoir_fp_scratch fs;
 } sbtv_ctx;
 
@@ -952,57 +950,34 @@ static int sbtv_processA(sbtv_ctx *c, const float *in, float *out)
 {
     udev *d = c->d;
     const int n = (int) c->n, S = c->S;
-    const size_t nvS = c->nv * (size_t) S;
-    int rc = udev_fill(d, c->tmpA, c->ns * (size_t) S, 0.0f);
-    if (!rc)
-        rc = ufoir__fp_full(c->p, &c->fs, in, c->tmpA, NULL, 0, c->tmpA, c->p->prm.correction_scale, S);
+    int rc = ufoir__fp_full(c->p, &c->fs, in, NULL, NULL, 0, c->tmpA, c->p->prm.correction_scale, S);
     if (!rc)
         rc = udev_bp(d, &c->g, c->p->subsets, (int) c->p->n_subsets, c->tmpA, NULL, NULL, 0, NULL, c->tmpAt,
                      c->p->prm.relaxation, S);
     if (!rc)
-        rc = udev_unary(d, UDEV_SCALE, c->tmpAt, c->mu, 0, c->tmpAt, nvS);
-    if (!rc)
-        rc = udev_diff(d, UDEV_DY, in, c->tmpD, n, n, S);
-    if (!rc)
-        rc = udev_diff(d, UDEV_DYT, c->tmpD, out, n, n, S);
-    if (!rc)
-        rc = udev_diff(d, UDEV_DX, in, c->tmpD, n, n, S);
-    if (!rc)
-        rc = udev_diff(d, UDEV_DXT, c->tmpD, c->tmpDxt, n, n, S);
-    if (!rc)
-        rc = udev_binary(d, UDEV_ADD, out, c->tmpDxt, 0, out, nvS);
-    if (!rc)
-        rc = udev_unary(d, UDEV_SCALE, out, c->lambda, 0, out, nvS);
-    if (!rc)
-        rc = udev_binary(d, UDEV_ADD, out, c->tmpAt, 0, out, nvS);
+        rc = udev_laplace(d, in, c->tmpAt, out, n, c->lambda, c->mu, S);
     return rc;
 }
 
-/* the reference's inner product of every slice (one launch, one read-back) */
+/* the reference's inner product of every slice (one read-back) */
 static int sbtv_dots(sbtv_ctx *c, const float *a, const float *b, float *out)
 {
-    return udev_dot(c->d, a, b, c->n, c->n, c->S, c->mode, out);
+    return udev_dots(c->d, 1, &a, &b, c->n, c->n, c->S, c->mode, out);
 }
 
 /* l2_norm (basic-ops-processor.c:239-247): sqrt in double of the float dot. */
+static void sbtv_roots(float *v, int count)
+{
+    for (int s = 0; s < count; s++)
+        v[s] = (float) sqrt((double) v[s]);
+}
+
 static int sbtv_l2s(sbtv_ctx *c, const float *a, float *out)
 {
     int rc = sbtv_dots(c, a, a, out);
-    for (int s = 0; s < c->S && !rc; s++)
-        out[s] = (float) sqrt((double) out[s]);
+    if (!rc)
+        sbtv_roots(out, c->S);
     return rc;
-}
-
-#define SL(ptr, s) ((ptr) + (size_t) (s) * c->nv)
-
-static int copy_s(sbtv_ctx *c, float *dst, const float *src, int s)
-{
-    return udev_memcpy_async(c->d, SL(dst, s), SL(src, s), c->nv * sizeof(float));
-}
-
-static int op_s(sbtv_ctx *c, int op, const float *a, const float *b, float m, float *out, int s)
-{
-    return udev_binary(c->d, op, SL(a, s), SL(b, s), m, SL(out, s), c->nv);
 }
 
 /* per-slice CGS state */
@@ -1013,19 +988,20 @@ typedef struct {
     int finished;    /* left before the loop ("initial guess is good enough") */
 } cgs_slice;
 
-/* cgs (sbtv-task.c:404-585) on S slices. */
+/* cgs (sbtv-task.c:404-585) on S slices. The vector updates run on all slices
+ * of a mask in one launch, each slice with its own scalar. */
 static int sbtv_cgs(sbtv_ctx *c, const float *b, float *x, const float *x0, unsigned int max_iter, float **w)
 {
     udev *d = c->d;
     const int S = c->S;
-    const size_t nvS = c->nv * (size_t) S;
-    float *xmin = w[0], *r = w[1], *rt = w[2], *u = w[3], *tmpa = w[4], *pp = w[5], *ph = w[6], *q = w[7];
-    float *vh = w[8], *tempSum = w[9], *uh = w[10], *qh = w[11];
+    const size_t nv = c->nv, nvS = nv * (size_t) S;
+    float *xmin = w[0], *r = w[1], *rt = w[2], *u = w[3], *tmpa = w[4], *pp = w[5], *q = w[6];
+    float *vh = w[7], *uh = w[8], *qh = w[9];
     int rc;
     const float tol = 1E-06f;
     const unsigned int maxmsteps = 5, maxstagsteps = 3;
     cgs_slice st[SBTV_MAX_BATCH];
-    float v[SBTV_MAX_BATCH], v2[SBTV_MAX_BATCH];
+    float v[2 * SBTV_MAX_BATCH], m[SBTV_MAX_BATCH];
     memset(st, 0, sizeof(st));
     if ((rc = sbtv_l2s(c, b, v)))
         return rc;
@@ -1041,6 +1017,7 @@ static int sbtv_cgs(sbtv_ctx *c, const float *b, float *x, const float *x0, unsi
         (rc = sbtv_l2s(c, r, v)))
         return rc;
     int n_active = 0;
+    unsigned int mask = 0;
     for (int s = 0; s < S; s++) {
         st[s].normr = st[s].normr_act = v[s];
         if (st[s].normr <= st[s].tolb) {
@@ -1051,22 +1028,20 @@ static int sbtv_cgs(sbtv_ctx *c, const float *b, float *x, const float *x0, unsi
         st[s].normmin = st[s].normr;
         st[s].rho = 1.0f;
         n_active++;
-        if ((rc = copy_s(c, rt, r, s)))
-            return rc;
+        mask |= 1u << s;
     }
-    if ((rc = udev_fill(d, u, nvS, 0.0f)) || (rc = udev_fill(d, tmpa, nvS, 0.0f)) ||
-        (rc = udev_fill(d, pp, nvS, 0.0f)) || (rc = udev_fill(d, q, nvS, 0.0f)) ||
-        (rc = udev_fill(d, tempSum, nvS, 0.0f)))
+    if ((rc = udev_masked(d, UDEV_COPY, r, NULL, NULL, mask, rt, nv, S)) || (rc = udev_fill(d, u, nvS, 0.0f)) ||
+        (rc = udev_fill(d, pp, nvS, 0.0f)) || (rc = udev_fill(d, q, nvS, 0.0f)))
         return rc;
 
     for (unsigned int iter = 0; iter < max_iter && n_active > 0; ++iter) {
-        float rho1[SBTV_MAX_BATCH];
         if ((rc = sbtv_dots(c, rt, r, v)))
             return rc;
+        mask = 0;
         for (int s = 0; s < S; s++) {
             if (!st[s].active)
                 continue;
-            rho1[s] = st[s].rho;
+            const float rho1 = st[s].rho;
             st[s].rho = v[s];
             const float rho = st[s].rho;
             if (rho == 0 || isinf(rho) || isnan(rho)) {
@@ -1074,26 +1049,21 @@ static int sbtv_cgs(sbtv_ctx *c, const float *b, float *x, const float *x0, unsi
                 st[s].active = 0;
                 continue;
             }
-            if (iter == 0) {
-                if ((rc = copy_s(c, u, r, s)) || (rc = copy_s(c, pp, u, s)))
-                    return rc;
-            } else {
-                const float beta = rho / rho1[s];
+            if (iter > 0) {
+                const float beta = rho / rho1;
                 if (beta == 0 || isinf(beta) || isnan(beta)) {
                     st[s].flag = 4;
                     st[s].active = 0;
                     continue;
                 }
-                if ((rc = op_s(c, UDEV_ADD_SCALED, r, q, beta, u, s)) ||
-                    (rc = op_s(c, UDEV_ADD_SCALED, q, pp, beta, tempSum, s)) ||
-                    (rc = op_s(c, UDEV_ADD_SCALED, u, tempSum, beta, pp, s)))
-                    return rc;
+                m[s] = beta;
             }
-            if ((rc = copy_s(c, ph, pp, s)))
-                return rc;
+            mask |= 1u << s;
         }
-        if ((rc = sbtv_processA(c, ph, vh)) || (rc = sbtv_dots(c, rt, vh, v)))
+        if ((rc = udev_cgs_dir(d, iter ? m : NULL, mask, iter == 0, r, q, u, pp, nv, S)) ||
+            (rc = sbtv_processA(c, pp, vh)) || (rc = sbtv_dots(c, rt, vh, v)))
             return rc;
+        mask = 0;
         for (int s = 0; s < S; s++) {
             if (!st[s].active)
                 continue;
@@ -1108,55 +1078,48 @@ static int sbtv_cgs(sbtv_ctx *c, const float *b, float *x, const float *x0, unsi
                 st[s].active = 0;
                 continue;
             }
-            if ((rc = op_s(c, UDEV_ADD_SCALED, u, vh, -st[s].alpha, q, s)) || (rc = op_s(c, UDEV_ADD, u, q, 0, uh, s)))
-                return rc;
+            m[s] = -st[s].alpha;
+            mask |= 1u << s;
         }
-        if ((rc = sbtv_l2s(c, uh, v)) || (rc = sbtv_l2s(c, x, v2)))
+        if ((rc = udev_cgs_step(d, m, mask, u, vh, q, uh, nv, S)))
             return rc;
+        {
+            const float *xs[2] = {uh, x};
+            if ((rc = udev_dots(d, 2, xs, xs, c->n, c->n, S, c->mode, v)))
+                return rc;
+            sbtv_roots(v, 2 * S);
+        }
         for (int s = 0; s < S; s++) {
             if (!st[s].active)
                 continue;
             /* fabs() promotes to double; EPS is the double literal 2.2204E-16 (:35, :498) */
-            if (fabs((double) st[s].alpha) * (double) v[s] < 2.2204E-16 * (double) v2[s])
+            if (fabs((double) st[s].alpha) * (double) v[s] < 2.2204E-16 * (double) v[S + s])
                 st[s].stag += 1;
             else
                 st[s].stag = 0;
-            if ((rc = op_s(c, UDEV_ADD_SCALED, x, uh, st[s].alpha, x, s)))
-                return rc;
+            m[s] = st[s].alpha;
         }
-        if ((rc = sbtv_processA(c, uh, qh)))
+        if ((rc = udev_masked(d, UDEV_ADD_SCALED, x, uh, m, mask, x, nv, S)) || (rc = sbtv_processA(c, uh, qh)))
             return rc;
         for (int s = 0; s < S; s++)
-            if (st[s].active && (rc = op_s(c, UDEV_ADD_SCALED, r, qh, -st[s].alpha, r, s)))
-                return rc;
-        if ((rc = sbtv_l2s(c, r, v)))
+            m[s] = -st[s].alpha;
+        if ((rc = udev_masked(d, UDEV_ADD_SCALED, r, qh, m, mask, r, nv, S)) || (rc = sbtv_l2s(c, r, v)))
             return rc;
-        int check = 0;
+        unsigned int check = 0;
         for (int s = 0; s < S; s++) {
             if (!st[s].active)
                 continue;
             st[s].normr = st[s].normr_act = v[s];
             if (st[s].normr <= st[s].tolb || st[s].stag >= maxstagsteps || st[s].moresteps)
-                check = 1;
+                check |= 1u << s;
         }
         if (check) {
             /* the reference applies A to r here (:535) */
-            if ((rc = sbtv_processA(c, r, tmpa)))
-                return rc;
-            int any = 0;
-            for (int s = 0; s < S; s++) {
-                if (!st[s].active ||
-                    !(st[s].normr <= st[s].tolb || st[s].stag >= maxstagsteps || st[s].moresteps))
-                    continue;
-                if ((rc = op_s(c, UDEV_SUB, b, tmpa, 0, r, s)))
-                    return rc;
-                any = 1;
-            }
-            if (any && (rc = sbtv_l2s(c, r, v)))
+            if ((rc = sbtv_processA(c, r, tmpa)) || (rc = udev_masked(d, UDEV_SUB, b, tmpa, NULL, check, r, nv, S)) ||
+                (rc = sbtv_l2s(c, r, v)))
                 return rc;
             for (int s = 0; s < S; s++) {
-                if (!st[s].active ||
-                    !(st[s].normr <= st[s].tolb || st[s].stag >= maxstagsteps || st[s].moresteps))
+                if (!((check >> s) & 1u))
                     continue;
                 st[s].normr_act = v[s];
                 if (st[s].normr_act <= st[s].tolb) {
@@ -1174,13 +1137,13 @@ static int sbtv_cgs(sbtv_ctx *c, const float *b, float *x, const float *x0, unsi
             }
         }
         n_active = 0;
+        mask = 0;
         for (int s = 0; s < S; s++) {
             if (!st[s].active)
                 continue;
             if (st[s].normr_act < st[s].normmin) {
                 st[s].normmin = st[s].normr_act;
-                if ((rc = copy_s(c, xmin, x, s)))
-                    return rc;
+                mask |= 1u << s;
             }
             if (st[s].stag >= maxstagsteps) {
                 st[s].flag = 3;
@@ -1189,39 +1152,40 @@ static int sbtv_cgs(sbtv_ctx *c, const float *b, float *x, const float *x0, unsi
             }
             n_active++;
         }
+        if ((rc = udev_masked(d, UDEV_COPY, x, NULL, NULL, mask, xmin, nv, S)))
+            return rc;
     }
-    int any_flag = 0;
+    mask = 0;
     for (int s = 0; s < S; s++)
-        any_flag |= !st[s].finished && st[s].flag != 0;
-    if (any_flag) {
-        if ((rc = sbtv_processA(c, xmin, tmpa)))
+        if (!st[s].finished && st[s].flag != 0)
+            mask |= 1u << s;
+    if (mask) {
+        if ((rc = sbtv_processA(c, xmin, tmpa)) || (rc = udev_masked(d, UDEV_SUB, b, tmpa, NULL, mask, r, nv, S)) ||
+            (rc = sbtv_l2s(c, r, v)))
             return rc;
+        unsigned int back = 0;
         for (int s = 0; s < S; s++)
-            if (!st[s].finished && st[s].flag != 0 && (rc = op_s(c, UDEV_SUB, b, tmpa, 0, r, s)))
-                return rc;
-        if ((rc = sbtv_l2s(c, r, v)))
+            if (((mask >> s) & 1u) && v[s] <= st[s].normr_act)
+                back |= 1u << s;
+        if ((rc = udev_masked(d, UDEV_COPY, xmin, NULL, NULL, back, x, nv, S)))
             return rc;
-        for (int s = 0; s < S; s++)
-            if (!st[s].finished && st[s].flag != 0 && v[s] <= st[s].normr_act && (rc = copy_s(c, x, xmin, s)))
-                return rc;
     }
     return UFOIR_OK;
 }
 
-#undef SL
-
-/* normalization (basic-ops-processor.c:342-367), in place on the device. */
-static int sbtv_normalize(udev *d, float *v, size_t count)
+/* normalization (basic-ops-processor.c:342-367) of S slices, in place on the device. */
+static int sbtv_normalize(udev *d, float *v, size_t count, int S)
 {
-    float lo, hi;
-    int rc = udev_minmax(d, v, count, 1, &lo, &hi);
-    if (rc)
-        return rc;
-    const float delta = 1 / (hi - lo);
-    return udev_unary(d, UDEV_NORMALIZE, v, delta, lo, v, count);
+    float lo[SBTV_MAX_BATCH], hi[SBTV_MAX_BATCH];
+    int rc = udev_minmax(d, v, count, S, lo, hi);
+    for (int s = 0; s < S && !rc; s++) {
+        const float delta = 1 / (hi[s] - lo[s]);
+        rc = udev_unary(d, UDEV_NORMALIZE, v + (size_t) s * count, delta, lo[s], v + (size_t) s * count, count);
+    }
+    return rc;
 }
 
-#define SBTV_NBUF 26
+#define SBTV_NBUF 21
 
 int ufoir_sbtv_process(ufoir_projector *proj, const ufoir_sbtv_params *prm, const float *sino,
                        const size_t dims[2], float *vol, size_t n_slices)
@@ -1261,12 +1225,10 @@ int ufoir_sbtv_process(ufoir_projector *proj, const ufoir_sbtv_params *prm, cons
     UFOIR_TRY(ufoir__alloc(ctx, &c.tmpA, ns * (size_t) S_max));
     for (int i = 0; i < SBTV_NBUF; i++)
         UFOIR_TRY(ufoir__alloc(ctx, &buf[i], nv * (size_t) S_max));
-    c.tmpAt = buf[12];
-    c.tmpD = buf[13];
-    c.tmpDxt = buf[14];
+    c.tmpAt = buf[10];
     UFOIR_TRY(ufoir__fp_scratch_alloc(proj, &c.fs, (size_t) S_max));
-    float *fbp = buf[16], *up = buf[17], *bvec = buf[18], *bx = buf[19], *by = buf[20], *dx = buf[21];
-    float *dy = buf[22], *tmpx = buf[23], *tmpy = buf[24], *tmp = buf[25];
+    float *fbp = buf[11], *up = buf[12], *bvec = buf[13], *bx = buf[14], *by = buf[15], *dx = buf[16];
+    float *dy = buf[17], *tmpx = buf[18], *tmpy = buf[19], *tmp = buf[20];
 
     for (size_t s0 = 0; s0 < n_slices; s0 += (size_t) S_max) {
         const int S = n_slices - s0 < (size_t) S_max ? (int) (n_slices - s0) : S_max;
@@ -1276,10 +1238,8 @@ int ufoir_sbtv_process(ufoir_projector *proj, const ufoir_sbtv_params *prm, cons
         /* normalise the input (a copy; the reference does it in place, :239),
          * copy it to f and normalise f again (:246-248), per slice */
         UFOIR_TRY(udev_memcpy_async(d, f, bb.dev + s0 * ns, ns * (size_t) S * sizeof(float)));
-        for (int s = 0; s < S; s++) {
-            UFOIR_TRY(sbtv_normalize(d, f + (size_t) s * ns, ns));
-            UFOIR_TRY(sbtv_normalize(d, f + (size_t) s * ns, ns));
-        }
+        UFOIR_TRY(sbtv_normalize(d, f, ns, S));
+        UFOIR_TRY(sbtv_normalize(d, f, ns, S));
         /* fbp = A^T f (:251-253), u = 0, bx = by = dx = dy = 0, fbp *= mu (:279) */
         UFOIR_TRY(udev_bp(d, &c.g, proj->subsets, (int) proj->n_subsets, f, NULL, NULL, 0, NULL, fbp,
                           proj->prm.relaxation, S));
@@ -1363,7 +1323,8 @@ int ufoir_dot_product(ufoir_ctx *ctx, const float *a, const float *b, size_t w, 
     int rc;
     UFOIR_TRY(ufoir__buf_in(ctx, &ba, a, w * h, 1));
     UFOIR_TRY(ufoir__buf_in(ctx, &bb, b, w * h, 1));
-    UFOIR_TRY(udev_dot(ctx->dev, ba.dev, bb.dev, w, h, 1, norm_mode, out));
+    const float *pa = ba.dev, *pb = bb.dev;
+    UFOIR_TRY(udev_dots(ctx->dev, 1, &pa, &pb, w, h, 1, norm_mode, out));
 done:
     ufoir__buf_release(ctx, &ba);
     ufoir__buf_release(ctx, &bb);

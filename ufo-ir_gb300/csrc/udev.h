@@ -74,7 +74,7 @@ typedef struct {
  * dir_override < 0 uses the per-angle direction, else forces it.
  * vol is [n][n] per slice; volT its transpose, read by horizontal rays (if
  * NULL they read vol column-wise instead). src/out/w are full sinograms
- * [n_angles][n] per slice; src may equal out; w may be NULL; w_shared != 0
+ * [n_angles][n] per slice; src may equal out, NULL reads zeros; w may be NULL; w_shared != 0
  * means one w for all slices. */
 int udev_fp(udev *d, const udev_geom *g, int a0, int na, int dir_override,
             const float *vol, const float *volT, const float *src, const float *w,
@@ -253,8 +253,8 @@ int udev_diff(udev *d, int which, const float *in, float *out, int w, int h, int
 int udev_l1_norm(udev *d, const float *v, size_t w, size_t h, int n_slices, int mode,
                  float *host_out);
 /* The same L1 norm into device memory (n_slices floats), with caller-owned
- * FP64 partials (udev_l1_partials(n_slices) doubles; unused in COMPAT
- * mode): no host synchronisation, capturable. */
+ * scratch (udev_l1_partials(n_slices) doubles): no host
+ * synchronisation, capturable. */
 size_t udev_l1_partials(int n_slices);
 int udev_l1_norm_to(udev *d, const float *v, size_t w, size_t h, int n_slices, int mode, double *partials,
                     float *d_out);
@@ -273,11 +273,29 @@ int udev_asd_tv_step(udev *d, float *x, const float *grad, const udev_asd_scalar
                      int n_slices);
 int udev_asd_end(udev *d, const udev_asd_scalars *S, float beta_red, float r_max, float alpha_red, int n_slices);
 
-/* buggy-index dot product of ufo_ir_basic_ops_processor_dot_product. */
-int udev_dot(udev *d, const float *a, const float *b, size_t w, size_t h, int n_slices,
-             int mode, float *host_out);
+/* buggy-index dot product of ufo_ir_basic_ops_processor_dot_product: `pairs`
+ * products a[k] . b[k] of every slice with one read-back,
+ * host_out[k * n_slices + slice]. */
+int udev_dots(udev *d, int pairs, const float *const *a, const float *const *b, size_t w, size_t h, int n_slices,
+              int mode, float *host_out);
 /* min and max of each slice (exact; order independent). */
 int udev_minmax(udev *d, const float *v, size_t n, int n_slices, float *host_min, float *host_max);
+
+/* ---- Split-Bregman TV's vector updates (udev_sbtv.cu): slices whose bit of
+ * mask is set, each with its own scalar. ---- */
+#define UDEV_SBTV_SLICES 16
+/* u = r + beta q;  p = u + beta (q + beta p); with first, u = p = r. */
+int udev_cgs_dir(udev *d, const float *beta, unsigned int mask, int first, const float *r, const float *q, float *u,
+                 float *p, size_t per_slice, int n_slices);
+/* q = u + m v;  uh = u + q. */
+int udev_cgs_step(udev *d, const float *m, unsigned int mask, const float *u, const float *v, float *q, float *uh,
+                  size_t per_slice, int n_slices);
+/* UDEV_ADD_SCALED: out = a + m b; UDEV_SUB: out = a - b; UDEV_COPY: out = a. */
+#define UDEV_COPY (-1)
+int udev_masked(udev *d, int op, const float *a, const float *b, const float *m, unsigned int mask, float *out,
+                size_t per_slice, int n_slices);
+/* out = lambda (Dyt Dy in + Dxt Dx in) + mu at, n x n slices. */
+int udev_laplace(udev *d, const float *in, const float *at, float *out, int n, float lambda, float mu, int n_slices);
 
 /* ---- Streams and events for concurrent jobs ---- */
 int udev_stream_create(udev *d, void **s);

@@ -415,7 +415,7 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
             if (s >= dend)
                 continue;
             const size_t oidx = (size_t) slice * P.sino_stride + (size_t) angle * n + s;
-            float result = P.src[oidx];
+            float result = P.src ? P.src[oidx] : 0.0f;
             const float ray = (i & 1) ? sum[k][i >> 1].y : sum[k][i >> 1].x;
             if (!joseph::detector_inactive(kc, s))
                 result = __fadd_rn(result, __fmul_rn(ray, P.scale));
@@ -551,7 +551,8 @@ int launch_tiles(udev *d, const FpTileArgs &args, int n_tiles, int n_slices, int
         FpTileArgs B = args;
         B.volP += (size_t) done * args.volp_stride;
         B.volTP += (size_t) done * args.volp_stride;
-        B.src += (size_t) done * args.sino_stride;
+        if (B.src)
+            B.src += (size_t) done * args.sino_stride;
         B.out += (size_t) done * args.sino_stride;
         if (B.w)
             B.w += (size_t) done * args.w_stride;

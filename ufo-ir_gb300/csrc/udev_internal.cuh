@@ -67,6 +67,10 @@ int udev_after_launch(udev *d, const char *what);
 /* Ensures the reduction scratch holds `partials` doubles and `outs` results. */
 int udev_reduction_scratch(udev *d, size_t partials, size_t outs);
 
+/* The COMPAT L1 norm of n_slices x count values (udev_norm.cu); scratch:
+ * udev_l1_partials(n_slices) doubles. */
+int udev_l1_compat(udev *d, const float *v, size_t count, int n_slices, double *scratch, float *d_out);
+
 static inline unsigned int udev_div_up(size_t a, size_t b)
 {
     return (unsigned int) ((a + b - 1) / b);

@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(128) fp_rows_kernel(FpArgs A)
         return;
 
     const size_t oidx = (size_t) slice * A.sino_stride + (size_t) a * n + s;
-    const float srcv = A.src[oidx];
+    const float srcv = A.src ? A.src[oidx] : 0.0f;
     const joseph::AxisConsts k = joseph::axis_consts(n, A.axis);
 
     float result;
@@ -224,7 +224,8 @@ extern "C" int udev_fp(udev *d, const udev_geom *g, int a0, int na, int dir_over
         FpArgs B = A;
         B.vol += (size_t) done * A.vol_stride;
         B.volT += (size_t) done * A.vol_stride;
-        B.src += (size_t) done * A.sino_stride;
+        if (B.src)
+            B.src += (size_t) done * A.sino_stride;
         if (B.w)
             B.w += (size_t) done * A.w_stride;
         B.out += (size_t) done * A.sino_stride;
