@@ -466,40 +466,42 @@ static int is_siddon(const ufoir_projector *p)
  * sino = sino + scale * A vol. */
 /* Siddon forward projection of angles [a0, a0 + na): the padded copies
  * first (scratch s), then the ray walk. */
-static int siddon_fp(ufoir_projector *p, ufoir_fp_scratch *s, int a0, int na, const float *dvol, float *dsino,
-                     int n_slices)
+static int siddon_fp(ufoir_projector *p, ufoir_fp_scratch *s, int a0, int na, const float *dvol, const float *src,
+                     float *dsino, int n_slices)
 {
     udev_geom g;
     ufoir__projector_geom(p, &g);
     int rc = udev_pad_transpose(p->ctx->dev, dvol, s->P, s->TP, s->nonfinite, (int) p->n_dets, n_slices);
     if (!rc)
-        rc = udev_siddon_fp(p->ctx->dev, &g, a0, na, s->P, s->TP, dsino, NULL, 0, dsino, p->prm.correction_scale,
+        rc = udev_siddon_fp(p->ctx->dev, &g, a0, na, s->P, s->TP, src, NULL, 0, dsino, p->prm.correction_scale,
                             n_slices);
     return rc;
 }
 
-static int fp_all(ufoir_projector *p, const float *dvol, float *dsino, size_t n_slices)
+/* dsino = src + scale * A dvol (src NULL: zeros). */
+static int fp_all(ufoir_projector *p, const float *dvol, const float *src, float *dsino, size_t n_slices)
 {
     ufoir_fp_scratch s;
     int rc = ufoir__fp_scratch_alloc(p, &s, n_slices);
     if (rc)
         return rc;
     if (is_siddon(p))
-        rc = siddon_fp(p, &s, 0, (int) p->n_angles, dvol, dsino, (int) n_slices);
+        rc = siddon_fp(p, &s, 0, (int) p->n_angles, dvol, src, dsino, (int) n_slices);
     else
-        rc = ufoir__fp_full(p, &s, dvol, dsino, NULL, 0, dsino, p->prm.correction_scale, (int) n_slices);
+        rc = ufoir__fp_full(p, &s, dvol, src, NULL, 0, dsino, p->prm.correction_scale, (int) n_slices);
     ufoir__fp_scratch_free(p, &s);
     return rc;
 }
 
-static int bp_all(ufoir_projector *p, float *dvol, const float *dsino, size_t n_slices)
+/* dvol = base + relaxation * A^T dsino (base NULL: zeros). */
+static int bp_all(ufoir_projector *p, const float *base, float *dvol, const float *dsino, size_t n_slices)
 {
     udev_geom g;
     ufoir__projector_geom(p, &g);
     if (is_siddon(p))
-        return udev_siddon_bp(p->ctx->dev, &g, p->subsets, (int) p->n_subsets, dsino, dvol, dvol,
+        return udev_siddon_bp(p->ctx->dev, &g, p->subsets, (int) p->n_subsets, dsino, base, dvol,
                               p->prm.relaxation, (int) n_slices);
-    return udev_bp(p->ctx->dev, &g, p->subsets, (int) p->n_subsets, dsino, dvol, NULL, 0, NULL, dvol,
+    return udev_bp(p->ctx->dev, &g, p->subsets, (int) p->n_subsets, dsino, base, NULL, 0, NULL, dvol,
                    p->prm.relaxation, (int) n_slices);
 }
 
@@ -516,7 +518,7 @@ int ufoir_projector_forward(ufoir_projector *proj, const float *vol, float *sino
     const size_t nv = n_dets * n_dets, ns = n_dets * n_angles;
     UFOIR_TRY(ufoir__buf_in(ctx, &bv, vol, nv * n_slices, 1));
     UFOIR_TRY(ufoir__buf_in(ctx, &bs, sino, ns * n_slices, 1));
-    UFOIR_TRY(fp_all(proj, bv.dev, bs.dev, n_slices));
+    UFOIR_TRY(fp_all(proj, bv.dev, bs.dev, bs.dev, n_slices));
     UFOIR_TRY(ufoir__buf_out(ctx, &bs, 1));
     UFOIR_TRY(udev_sync(ctx->dev));
 done:
@@ -538,7 +540,7 @@ int ufoir_projector_backward(ufoir_projector *proj, float *vol, const float *sin
     const size_t nv = n_dets * n_dets, ns = n_dets * n_angles;
     UFOIR_TRY(ufoir__buf_in(ctx, &bv, vol, nv * n_slices, 1));
     UFOIR_TRY(ufoir__buf_in(ctx, &bs, sino, ns * n_slices, 1));
-    UFOIR_TRY(bp_all(proj, bv.dev, bs.dev, n_slices));
+    UFOIR_TRY(bp_all(proj, bv.dev, bv.dev, bs.dev, n_slices));
     UFOIR_TRY(ufoir__buf_out(ctx, &bv, 1));
     UFOIR_TRY(udev_sync(ctx->dev));
 done:
@@ -566,16 +568,14 @@ int ufoir_projector_process(ufoir_projector *proj, const float *in, const size_t
             return ufoir__fail(ctx, UFOIR_ERR_INVALID, "forward input must be %zu x %zu", n, n);
         UFOIR_TRY(ufoir__buf_in(ctx, &bi, in, nv * n_slices, 1));
         UFOIR_TRY(ufoir__buf_in(ctx, &bo, out, ns * n_slices, 0));
-        UFOIR_TRY(udev_fill(ctx->dev, bo.dev, ns * n_slices, 0.0f));
-        UFOIR_TRY(fp_all(proj, bi.dev, bo.dev, n_slices));
+        UFOIR_TRY(fp_all(proj, bi.dev, NULL, bo.dev, n_slices));
     } else {
         if (in_dims[1] != proj->n_angles)
             return ufoir__fail(ctx, UFOIR_ERR_INVALID, "angles_num %u does not match the sinogram's %zu rows",
                                proj->n_angles, in_dims[1]);
         UFOIR_TRY(ufoir__buf_in(ctx, &bi, in, ns * n_slices, 1));
         UFOIR_TRY(ufoir__buf_in(ctx, &bo, out, nv * n_slices, 0));
-        UFOIR_TRY(udev_fill(ctx->dev, bo.dev, nv * n_slices, 0.0f));
-        UFOIR_TRY(bp_all(proj, bo.dev, bi.dev, n_slices));
+        UFOIR_TRY(bp_all(proj, NULL, bo.dev, bi.dev, n_slices));
     }
     UFOIR_TRY(ufoir__buf_out(ctx, &bo, 1));
     UFOIR_TRY(udev_sync(ctx->dev));
@@ -605,7 +605,7 @@ int ufoir_projector_subset_fp(ufoir_projector *proj, const float *vol, float *si
     if (is_siddon(proj)) {
         ufoir_fp_scratch fs;
         UFOIR_TRY(ufoir__fp_scratch_alloc(proj, &fs, 1));
-        rc = siddon_fp(proj, &fs, (int) s->offset, (int) s->n, bv.dev, bs.dev, 1);
+        rc = siddon_fp(proj, &fs, (int) s->offset, (int) s->n, bv.dev, bs.dev, bs.dev, 1);
         ufoir__fp_scratch_free(proj, &fs);
         if (rc)
             goto done;
