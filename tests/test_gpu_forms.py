@@ -111,3 +111,26 @@ def test_forward_projector_row_forms_and_non_finite_data(ufoir_lib, gpu_ctx, n, 
     with np.errstate(invalid="ignore"):
         for s in sorted({0, slices - 1}):
             np.testing.assert_array_equal(got[s], _forward(vol[s], na, step, axis))
+
+
+@pytest.mark.parametrize("n,na,axis", [(7, 6, 3.5), (64, 20, 32.0), (65, 12, 30.2), (200, 180, 104.0), (1100, 8, 550.0)])
+def test_subset_projections(ufoir_lib, gpu_ctx, oracle, n, na, axis):
+    """Subsets of one angle, several, and all of one direction, each as vertical
+    and as horizontal rays (whichever the angles are), against the oracle's kernel."""
+    import ctypes
+    fp = ctypes.POINTER(ctypes.c_float)
+    step = f32(np.pi / na)
+    rng = np.random.default_rng(n)
+    vol = rng.random((n, n), dtype=f32)
+    p = ufoir_lib.ParallelProjector(gpu_ctx, step=float(step), angles_num=na, axis_position=axis, correction_scale=-1.0)
+    p.get_requisition((n, n))
+    s, c = oracle.lut(na, step)
+    k, dims = oracle.kernels().contents, oracle.Dims(n, n, n, na)
+    for off, cnt in [(1, 1), (na // 2, 1), (0, 3), (na // 4, na // 3)]:
+        for direction in (0, 1):
+            sino = rng.random((na, n), dtype=f32)
+            want = sino.copy()
+            k.fp(oracle.image(vol), oracle.image(want), s.ctypes.data_as(fp), c.ctypes.data_as(fp), dims, f32(axis),
+                 oracle.Subset(off, cnt, direction), f32(-1.0))
+            np.testing.assert_array_equal(p.subset_fp(vol, sino.copy(), off, cnt, direction), want)
+    p.close()

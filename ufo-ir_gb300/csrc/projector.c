@@ -596,6 +596,7 @@ int ufoir_projector_subset_fp(ufoir_projector *proj, const float *vol, float *si
         return ufoir__fail(ctx, UFOIR_ERR_INVALID, "subset outside the %u angles", proj->n_angles);
     const size_t n = proj->n_dets, nv = n * n, ns = n * proj->n_angles;
     ufoir_buf bv = {0}, bs = {0};
+    float *volT = NULL;
     udev_geom g;
     ufoir__projector_geom(proj, &g);
     int rc;
@@ -609,12 +610,18 @@ int ufoir_projector_subset_fp(ufoir_projector *proj, const float *vol, float *si
         ufoir__fp_scratch_free(proj, &fs);
         if (rc)
             goto done;
-    } else
-        UFOIR_TRY(udev_fp(ctx->dev, &g, (int) s->offset, (int) s->n, s->direction ? 1 : 0, bv.dev, NULL, bs.dev,
+    } else {
+        /* horizontal rays walk the rows of the transpose, or the columns
+         * where there is no memory for it */
+        if (!s->direction && s->n > 0 && ufoir__alloc(ctx, &volT, nv) == UFOIR_OK)
+            UFOIR_TRY(udev_transpose(ctx->dev, bv.dev, volT, (int) n, 1));
+        UFOIR_TRY(udev_fp(ctx->dev, &g, (int) s->offset, (int) s->n, s->direction ? 1 : 0, bv.dev, volT, bs.dev,
                           NULL, 0, bs.dev, proj->prm.correction_scale, 1));
+    }
     UFOIR_TRY(ufoir__buf_out(ctx, &bs, 1));
     UFOIR_TRY(udev_sync(ctx->dev));
 done:
+    ufoir__free(ctx, volT);
     ufoir__buf_release(ctx, &bv);
     ufoir__buf_release(ctx, &bs);
     return rc;

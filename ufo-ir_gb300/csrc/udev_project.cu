@@ -2,14 +2,16 @@
  * udev_project.cu - Joseph forward projector, pixel-driven backprojector and
  * the volume transpose used by the forward projector.
  *
- * Forward projection (replaces FP_hor / FP_vert, projector-parallel-joseph.cl:36-156):
- * one thread per ray walks the rows of a row-major image. Vertical rays
- * (|sin| <= |cos|) walk the rows of the volume and interpolate along x;
- * horizontal rays walk the rows of the transposed volume, so both kinds
- * read along rows and a warp's 32 neighbouring detectors touch a few
- * consecutive cache lines per step. Samples are summed per ray in blocks of
- * 64 in the reference's order, with the float coordinate recurrence, so the
- * sum is the reference's to the last bit.
+ * Forward projection (replaces FP_hor / FP_vert, projector-parallel-joseph.cl:36-156)
+ * of single subsets. Vertical rays (|sin| <= |cos|) walk the rows of the
+ * volume and interpolate along x; horizontal rays walk the rows of the
+ * transposed volume, so both kinds read along rows and a warp's 32
+ * neighbouring detectors touch a few consecutive cache lines per step.
+ * Samples are summed per ray in blocks of 64 in the reference's order, with
+ * the float coordinate recurrence, so the sum is the reference's to the last
+ * bit. The blocks of a ray are spread over the warps of a CTA
+ * (fp_blocks_kernel); beyond 8192 detectors one thread walks a whole ray
+ * (fp_rows_kernel).
  *
  * Backprojection (replaces BP, projector-parallel-joseph.cl:158-218): one
  * thread per pixel gathers every angle of every subset in order; no atomics,
@@ -95,6 +97,87 @@ __global__ void __launch_bounds__(128) fp_rows_kernel(FpArgs A)
             detected = __fadd_rn(detected, inner);
         }
         result = __fadd_rn(srcv, __fmul_rn(detected, A.scale));
+    }
+    if (A.w)
+        result = __fmul_rn(result, A.w[(size_t) slice * A.w_stride + (size_t) a * n + s]);
+    A.out[oidx] = result;
+}
+
+constexpr int kSplitBlocks = 128;   /* 64-sample blocks per ray at most (n <= 8192) */
+constexpr int kSplitWarps = 16;
+constexpr int kBatch = 16;          /* samples whose loads are in flight together */
+
+/*
+ * The same for 32 adjacent rays per CTA, lane = ray, with the rays' 64-sample
+ * blocks dealt to the warps (block b to warp b mod W): a warp replays the
+ * coordinate recurrence up to each of its blocks (n additions of 4 cycles in
+ * all, 3 us at n = 1448), issues 16 samples' loads together and keeps the
+ * blocks' sums in shared memory, which warp 0 adds in block order. Bound by
+ * latency: an angle is n rays, so one thread per ray left 6 CTAs of work at n =
+ * 724 that waited for each row's loads (104 us an angle, columns read one
+ * sector per lane; 11 us here, and 3 us for the transpose that horizontal
+ * angles now read). More rays than the GPU has warps for take fewer warps per
+ * CTA, as each of them replays the recurrence.
+ * Grid (ceil(n / 32), angles, slices), 32 W threads.
+ */
+__global__ void __launch_bounds__(32 * kSplitWarps) fp_blocks_kernel(FpArgs A)
+{
+    __shared__ float bsum[kSplitBlocks][32];
+    const int lane = (int) (threadIdx.x & 31), warp = (int) (threadIdx.x >> 5), W = (int) (blockDim.x >> 5);
+    const int n = A.n;
+    const int s = (int) blockIdx.x * 32 + lane, sc = min(s, n - 1);
+    const int a = A.a0 + (int) blockIdx.y;
+    const int slice = (int) blockIdx.z;
+    const joseph::AxisConsts k = joseph::axis_consts(n, A.axis);
+    const int dir = A.dir_override >= 0 ? A.dir_override : (int) A.dir[a];
+    float det_step, step;
+    joseph::ray_steps(dir, A.sinv[a], A.cosv[a], det_step, step);
+    /* without a transpose horizontal rays read vol column by column */
+    const float *img = (dir == 0 && A.have_volT ? A.volT : A.vol) + (size_t) slice * A.vol_stride;
+    const size_t row_step = dir == 0 && !A.have_volT ? 1 : (size_t) n;
+    const size_t col_step = dir == 0 && !A.have_volT ? (size_t) n : 1;
+    float c = joseph::ray_start(k, sc, n, det_step, step);
+    const int nb = (n + 63) / 64;
+    int row = 0;
+    for (int b = warp; b < nb; b += W) {
+#pragma unroll 8
+        for (; row < 64 * b; ++row)
+            c = __fadd_rn(c, step);
+        float inner = 0.0f;
+#pragma unroll 1
+        for (; row < 64 * (b + 1); row += kBatch) {
+            float t[kBatch], va[kBatch], vb[kBatch];
+            bool ina[kBatch], inb[kBatch];
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q) {
+                int i0;
+                joseph::lerp_coord(c, i0, t[q]);
+                c = __fadd_rn(c, step);
+                /* rows past the image (the padding of the last block) read the zero border */
+                const bool in = row + q < n;
+                const float *r = img + (size_t) min(row + q, n - 1) * row_step;
+                ina[q] = in && (unsigned int) i0 < (unsigned int) n;
+                inb[q] = in && (unsigned int) i0 + 1u < (unsigned int) n;
+                va[q] = ina[q] ? __ldg(r + (size_t) i0 * col_step) : 0.0f;
+                vb[q] = inb[q] ? __ldg(r + (size_t) ((unsigned int) i0 + 1u) * col_step) : 0.0f;
+            }
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q)
+                if (row + q < n)
+                    inner = __fadd_rn(inner, joseph::lerp(t[q], va[q], vb[q]));
+        }
+        bsum[b][lane] = inner;
+    }
+    __syncthreads();
+    if (warp != 0 || s >= n)
+        return;
+    const size_t oidx = (size_t) slice * A.sino_stride + (size_t) a * n + s;
+    float result = A.src ? A.src[oidx] : 0.0f;
+    if (!joseph::detector_inactive(k, s)) {
+        float detected = 0.0f;
+        for (int b = 0; b < nb; ++b)
+            detected = __fadd_rn(detected, bsum[b][lane]);
+        result = __fadd_rn(result, __fmul_rn(detected, A.scale));
     }
     if (A.w)
         result = __fmul_rn(result, A.w[(size_t) slice * A.w_stride + (size_t) a * n + s]);
@@ -229,9 +312,22 @@ extern "C" int udev_fp(udev *d, const udev_geom *g, int a0, int na, int dir_over
         if (B.w)
             B.w += (size_t) done * A.w_stride;
         B.out += (size_t) done * A.sino_stride;
-        dim3 grid(udev_div_up(g->n_dets, 128), (unsigned int) na, (unsigned int) chunk);
-        fp_rows_kernel<<<grid, 128, 0, d->stream>>>(B);
-        int rc = udev_after_launch(d, "fp_rows_kernel");
+        int rc;
+        const int nb = (g->n_dets + 63) / 64;
+        if (nb <= kSplitBlocks) {
+            /* as many warps per ray group as fill the GPU with 16 per SM */
+            const long long groups = (long long) udev_div_up(g->n_dets, 32) * na * chunk;
+            long long W = (16LL * d->sm_count + groups - 1) / groups;
+            W = W > kSplitWarps ? kSplitWarps : W;
+            W = W > nb ? nb : W;
+            dim3 grid(udev_div_up(g->n_dets, 32), (unsigned int) na, (unsigned int) chunk);
+            fp_blocks_kernel<<<grid, 32 * (unsigned int) W, 0, d->stream>>>(B);
+            rc = udev_after_launch(d, "fp_blocks_kernel");
+        } else {
+            dim3 grid(udev_div_up(g->n_dets, 128), (unsigned int) na, (unsigned int) chunk);
+            fp_rows_kernel<<<grid, 128, 0, d->stream>>>(B);
+            rc = udev_after_launch(d, "fp_rows_kernel");
+        }
         if (rc)
             return rc;
         done += chunk;
