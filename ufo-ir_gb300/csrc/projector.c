@@ -402,12 +402,12 @@ int ufoir__fp_scratch_alloc(ufoir_projector *p, ufoir_fp_scratch *s, size_t slic
     s->P = s->TP = NULL;
     s->nonfinite = NULL;
     s->slices = slices;
+    /* one allocation: P, the flag (padded to 16 bytes), TP */
     const size_t count = n * pitch * slices;
-    int rc = ufoir__alloc(p->ctx, &s->P, count + 1);
-    if (!rc)
-        rc = ufoir__alloc(p->ctx, &s->TP, count);
+    int rc = ufoir__alloc(p->ctx, &s->P, 2 * count + 4);
     if (!rc) {
         s->nonfinite = (int *) (s->P + count);
+        s->TP = s->P + count + 4;
         rc = udev_memset(p->ctx->dev, s->nonfinite, 0, sizeof(int));
     }
     if (rc)
@@ -418,7 +418,6 @@ int ufoir__fp_scratch_alloc(ufoir_projector *p, ufoir_fp_scratch *s, size_t slic
 void ufoir__fp_scratch_free(ufoir_projector *p, ufoir_fp_scratch *s)
 {
     ufoir__free(p->ctx, s->P);
-    ufoir__free(p->ctx, s->TP);
     s->P = s->TP = NULL;
     s->nonfinite = NULL;
 }
@@ -520,7 +519,6 @@ int ufoir_projector_forward(ufoir_projector *proj, const float *vol, float *sino
     UFOIR_TRY(ufoir__buf_in(ctx, &bs, sino, ns * n_slices, 1));
     UFOIR_TRY(fp_all(proj, bv.dev, bs.dev, bs.dev, n_slices));
     UFOIR_TRY(ufoir__buf_out(ctx, &bs, 1));
-    UFOIR_TRY(udev_sync(ctx->dev));
 done:
     ufoir__buf_release(ctx, &bv);
     ufoir__buf_release(ctx, &bs);
@@ -542,7 +540,6 @@ int ufoir_projector_backward(ufoir_projector *proj, float *vol, const float *sin
     UFOIR_TRY(ufoir__buf_in(ctx, &bs, sino, ns * n_slices, 1));
     UFOIR_TRY(bp_all(proj, bv.dev, bv.dev, bs.dev, n_slices));
     UFOIR_TRY(ufoir__buf_out(ctx, &bv, 1));
-    UFOIR_TRY(udev_sync(ctx->dev));
 done:
     ufoir__buf_release(ctx, &bv);
     ufoir__buf_release(ctx, &bs);
@@ -578,7 +575,6 @@ int ufoir_projector_process(ufoir_projector *proj, const float *in, const size_t
         UFOIR_TRY(bp_all(proj, NULL, bo.dev, bi.dev, n_slices));
     }
     UFOIR_TRY(ufoir__buf_out(ctx, &bo, 1));
-    UFOIR_TRY(udev_sync(ctx->dev));
 done:
     ufoir__buf_release(ctx, &bi);
     ufoir__buf_release(ctx, &bo);
@@ -619,7 +615,6 @@ int ufoir_projector_subset_fp(ufoir_projector *proj, const float *vol, float *si
                           NULL, 0, bs.dev, proj->prm.correction_scale, 1));
     }
     UFOIR_TRY(ufoir__buf_out(ctx, &bs, 1));
-    UFOIR_TRY(udev_sync(ctx->dev));
 done:
     ufoir__free(ctx, volT);
     ufoir__buf_release(ctx, &bv);
@@ -648,7 +643,6 @@ int ufoir_projector_subset_bp(ufoir_projector *proj, float *vol, const float *si
     else
         UFOIR_TRY(udev_bp(ctx->dev, &g, s, 1, bs.dev, bv.dev, NULL, 0, NULL, bv.dev, proj->prm.relaxation, 1));
     UFOIR_TRY(ufoir__buf_out(ctx, &bv, 1));
-    UFOIR_TRY(udev_sync(ctx->dev));
 done:
     ufoir__buf_release(ctx, &bv);
     ufoir__buf_release(ctx, &bs);

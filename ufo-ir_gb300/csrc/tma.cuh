@@ -9,12 +9,22 @@
 #ifndef UFOIR_TMA_CUH
 #define UFOIR_TMA_CUH
 
+#include <cuda_runtime.h>
+
 #include <cstdint>
 
 namespace tma {
 
 /* Error codes written to the kernel error word. */
 enum : int { kErrWaitTimeout = 1, kErrDrainTimeout = 2, kErrWindow = 8 };
+
+/* Records `code` in the error word, which lies in host memory: the host reads
+ * it after a stream synchronisation, with no copy. */
+__device__ __forceinline__ void report(int *err, int code)
+{
+    *reinterpret_cast<volatile int *>(err) = code;
+    __threadfence_system();
+}
 
 constexpr unsigned long long kWaitLimitNs = 250000000ull;   /* 250 ms */
 
@@ -86,7 +96,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *e
     while (!mbar_try_wait(bar, parity)) {
         if (global_ns() - t0 > kWaitLimitNs) {
             if (err)
-                atomicExch(err, code);
+                report(err, code);
             return false;
         }
     }

@@ -213,7 +213,7 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
         int w0 = (clo >= 0 ? clo : clo - 3) / 4 * 4;
         w0 = max(0, min(w0, pitch - wcols));
         if (min(chi, kPadL + n - 1) >= w0 + wcols)
-            atomicOr(P.err, tma::kErrWindow);      /* the host's width bound was too small */
+            tma::report(P.err, tma::kErrWindow);      /* the host's width bound was too small */
         wok[st_] = min(chi, pitch - 1) < w0 + wcols && max(clo, 0) >= w0;
         return w0;
     };

@@ -26,8 +26,8 @@ struct udev {
     size_t red_out_cap = 0;
     cudaEvent_t ev_start = nullptr;
     cudaEvent_t ev_stop = nullptr;
-    int *d_err = nullptr;           /* kernel error word (bounded-wait timeouts) */
-    int *h_err = nullptr;
+    int *h_err = nullptr;           /* kernel error word (bounded-wait timeouts), mapped host memory */
+    int *d_err = nullptr;           /* the same as kernels address it */
     int inject_skip_chunk = -1;     /* testing: see udev_inject_copy_skip */
     int sart_wide_clusters = 0;     /* 16-CTA clusters of the segment-form SART FP that fit at once */
     cudaStream_t side = nullptr;    /* side copies (udev_copy_after), created on first use */

@@ -82,8 +82,14 @@ int udev_create(int device, udev **out, char *err, size_t errlen)
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &threshold);
     }
     cudaGetLastError();
-    if (cudaMalloc(&d->d_err, sizeof(int)) != cudaSuccess || cudaMemset(d->d_err, 0, sizeof(int)) != cudaSuccess ||
-        cudaMallocHost(&d->h_err, sizeof(int)) != cudaSuccess || udev_kernels_init(d) != UFOIR_OK) {
+    if (cudaHostAlloc(&d->h_err, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer((void **) &d->d_err, d->h_err, 0) != cudaSuccess) {
+        snprintf(err, errlen, "context setup failed: %s", cudaGetErrorString(cudaGetLastError()));
+        udev_destroy(d);
+        return UFOIR_ERR_CUDA;
+    }
+    *d->h_err = 0;
+    if (udev_kernels_init(d) != UFOIR_OK) {
         snprintf(err, errlen, "context setup failed: %s", d->err[0] ? d->err : cudaGetErrorString(cudaGetLastError()));
         udev_destroy(d);
         return UFOIR_ERR_CUDA;
@@ -108,8 +114,6 @@ void udev_destroy(udev *d)
         cudaEventDestroy(d->ev_start);
     if (d->ev_stop)
         cudaEventDestroy(d->ev_stop);
-    if (d->d_err)
-        cudaFree(d->d_err);
     if (d->h_err)
         cudaFreeHost(d->h_err);
     if (d->side) {
@@ -379,13 +383,11 @@ int udev_memset(udev *d, void *p, int value, size_t bytes)
 int udev_take_kernel_error(udev *d)
 {
     UDEV_BIND(d);
-    UDEV_CHECK(d, cudaMemcpyAsync(d->h_err, d->d_err, sizeof(int), cudaMemcpyDeviceToHost, d->stream));
     UDEV_CHECK(d, cudaStreamSynchronize(d->stream));
-    const int code = *d->h_err;
+    const int code = *static_cast<volatile int *>(d->h_err);
     if (code == 0)
         return UFOIR_OK;
-    UDEV_CHECK(d, cudaMemsetAsync(d->d_err, 0, sizeof(int), d->stream));
-    UDEV_CHECK(d, cudaStreamSynchronize(d->stream));
+    *static_cast<volatile int *>(d->h_err) = 0;
     if (code & 3) {
         udev_set_error(d, "a kernel gave up waiting for a shared-memory copy (code %d); results of that call are invalid",
                        code);

@@ -29,6 +29,7 @@
 #include <cuda_runtime.h>
 
 #include "joseph.cuh"
+#include "tma.cuh"
 #include "udev_internal.cuh"
 
 namespace {
@@ -694,7 +695,7 @@ __global__ void __launch_bounds__(256) sart_bp_kernel(SartBpArgs P)
     const int tid = (int) (threadIdx.y * 32 + threadIdx.x);
     if (span > kBpSpan) {      /* cannot happen for |sin|, |cos| <= 1; uniform per CTA */
         if (tid == 0)
-            atomicOr(P.err, kErrSpan);
+            tma::report(P.err, kErrSpan);
         return;
     }
     /* the residual row and the volume were written by earlier kernels */
