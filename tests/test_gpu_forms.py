@@ -134,3 +134,41 @@ def test_subset_projections(ufoir_lib, gpu_ctx, oracle, n, na, axis):
                  oracle.Subset(off, cnt, direction), f32(-1.0))
             np.testing.assert_array_equal(p.subset_fp(vol, sino.copy(), off, cnt, direction), want)
     p.close()
+
+
+@pytest.mark.parametrize("n,na,slices,axis", [(5, 3, 1, 2.5), (129, 37, 1, 64.5), (129, 33, 14, 60.1), (130, 17, 150, 71.3),
+                                              (200, 40, 130, 100.0), (301, 70, 1, 150.5)])
+def test_siddon_launch_shapes(ufoir_lib, gpu_ctx, oracle, n, na, slices, axis):
+    """Each launch shape of the siddon model's tiles, ragged edges and off-centre
+    axes among them, against the double oracle at the model's tolerance (bins
+    that lie on pixel boundaries of an axis-aligned angle have no one answer:
+    see the next test)."""
+    step = f32(np.pi / na)
+    rng = np.random.default_rng(n + slices)
+    vols = rng.random((slices, n, n), dtype=f32)
+    sinos = rng.random((slices, na, n), dtype=f32)
+    fwd = ufoir_lib.ParallelProjector(gpu_ctx, step=float(step), is_forward=1, axis_position=axis, angles_num=na, model="siddon")
+    bwd = ufoir_lib.ParallelProjector(gpu_ctx, step=float(step), is_forward=0, axis_position=axis, angles_num=na, model="siddon")
+    got, back = fwd.process(vols), bwd.process(sinos)
+    for i in sorted({0, slices - 1}):
+        want, wantb = oracle.siddon_forward(n, na, step, vols[i], axis), oracle.siddon_backward(n, na, step, sinos[i], axis)
+        assert np.linalg.norm(got[i] - want) <= 1e-5 * np.linalg.norm(want)
+        assert np.linalg.norm(back[i] - wantb) <= 1e-5 * np.linalg.norm(wantb)
+    fwd.close()
+    bwd.close()
+
+
+@pytest.mark.parametrize("n,na,axis", [(130, 16, 70.5), (129, 8, 60.0)])
+def test_siddon_tiles_and_ray_walk_agree_on_pixel_boundaries(ufoir_lib, gpu_ctx, n, na, axis):
+    """An axis half a bin off the centre puts every ray of the axis-aligned
+    angles on a pixel boundary; whole sets (tiles) and subsets (the ray walk)
+    must put them on the same side. Tolerance: two orders of n float roundings."""
+    step = f32(np.pi / na)
+    vol = np.random.default_rng(n).random((n, n), dtype=f32)
+    p = ufoir_lib.ParallelProjector(gpu_ctx, step=float(step), is_forward=1, axis_position=axis, angles_num=na, model="siddon")
+    whole = p.process(vol)
+    part = np.zeros((na, n), f32)
+    for off, cnt, direction in p.subsets():
+        p.subset_fp(vol, part, off, cnt, direction)
+    p.close()
+    np.testing.assert_allclose(whole, part, rtol=0, atol=2 * n * 2.0 ** -24 * float(np.abs(part).max()))

@@ -249,6 +249,30 @@ __device__ __forceinline__ float2 floor_any2(float2 c, float2 &t)
     return y;
 }
 
+/* a * b per lane; may be fused into an addition that follows. */
+__device__ __forceinline__ float2 mul2(float2 a, float2 b)
+{
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a)), "l"(pack2(b)));
+    return unpack2(r);
+}
+
+/* a * b + c clamped to [0, 1] (NaN gives 0). */
+__device__ __forceinline__ float fma_sat(float a, float b, float c)
+{
+    float r;
+    asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+/* floor(c) and c - floor(c) for |c| < 2^22 (bits kFloorMagicBits + floor(c)). */
+__device__ __forceinline__ float2 floor2(float2 c, float2 &t)
+{
+    const float2 y = add2_rd(c, splat(kFloorMagic));
+    t = sub2(c, sub2(y, splat(kFloorMagic)));
+    return y;
+}
+
 /* Bounds-checked texel of a row with a zero border. */
 __device__ __forceinline__ float texel(const float *__restrict__ row, int i, int n)
 {

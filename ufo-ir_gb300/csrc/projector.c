@@ -477,6 +477,28 @@ static int siddon_fp(ufoir_projector *p, ufoir_fp_scratch *s, int a0, int na, co
     return rc;
 }
 
+/* All angles through the tiled kernel, or the ray walk where it cannot serve
+ * the size. */
+static int siddon_fp_all(ufoir_projector *p, ufoir_fp_scratch *s, const float *dvol, const float *src, float *dsino,
+                         int n_slices)
+{
+    udev_geom g;
+    ufoir__projector_geom(p, &g);
+    udev_fp_cfg c;
+    const void *tiles = NULL;
+    int n_tiles = 0;
+    int rc = ufoir__fp_shape(p, n_slices, &c, &tiles, &n_tiles);
+    if (rc == UFOIR_ERR_UNSUPPORTED)
+        return siddon_fp(p, s, 0, (int) p->n_angles, dvol, src, dsino, n_slices);
+    if (!rc)
+        rc = udev_pad_transpose(p->ctx->dev, dvol, s->P, s->TP, s->nonfinite, (int) p->n_dets, n_slices);
+    c.fm = 2;
+    if (!rc)
+        rc = udev_fp_tiles_cfg(p->ctx->dev, &g, &c, tiles, n_tiles, s->P, s->TP, s->nonfinite, src, NULL, 0, dsino,
+                               p->prm.correction_scale, n_slices);
+    return rc;
+}
+
 /* dsino = src + scale * A dvol (src NULL: zeros). */
 static int fp_all(ufoir_projector *p, const float *dvol, const float *src, float *dsino, size_t n_slices)
 {
@@ -485,7 +507,7 @@ static int fp_all(ufoir_projector *p, const float *dvol, const float *src, float
     if (rc)
         return rc;
     if (is_siddon(p))
-        rc = siddon_fp(p, &s, 0, (int) p->n_angles, dvol, src, dsino, (int) n_slices);
+        rc = siddon_fp_all(p, &s, dvol, src, dsino, (int) n_slices);
     else
         rc = ufoir__fp_full(p, &s, dvol, src, NULL, 0, dsino, p->prm.correction_scale, (int) n_slices);
     ufoir__fp_scratch_free(p, &s);

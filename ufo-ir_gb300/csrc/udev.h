@@ -141,7 +141,7 @@ int udev_pad_transpose(udev *d, const float *vol, float *volP, float *volTP, int
 typedef struct {
     int J, A, win, K, dsplit;
     int threads, dper, wcols, wstride, margin;
-    int fm;                        /* fast arithmetic (from the geometry) */
+    int fm;                        /* 1: fast arithmetic (from the geometry); 2: the siddon model */
     size_t smem;
 } udev_fp_cfg;
 /* The fixed rules for n_tiles tiles of the default angle count and n_slices

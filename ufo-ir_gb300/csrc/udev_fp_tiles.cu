@@ -125,7 +125,41 @@ __device__ __forceinline__ void ray_rows(float c, float st, float lo, float hi, 
  * n <= 768, measured 4 % slower held to that register budget.) */
 /* One CTA's work: angle tile `tile_idx` of P.tiles, detector part `dpart`
  * of P.dsplit, slice `slice`; smem_raw is the dynamic shared memory. */
-template <int J, int A, bool WIN, bool FM>
+/* The tiled kernels' arithmetic: the reference's, the fast interpolation, or
+ * the siddon model (exact line integrals, udev_siddon.cu). */
+constexpr int kArithExact = 0, kArithFast = 1, kArithSiddon = 2;
+
+/* The siddon rays of one angle, in the float arithmetic of the ray walk
+ * (udev_siddon.cu), so that rays on a pixel boundary fall on the same side:
+ * the slab edge j of the walked rows is start + j slope columns from the
+ * image's edge, and a ray's lower end in slab j is edge j + down. Its length
+ * in the slab is len, and inv = 1 / |slope| turns a distance across into a
+ * share of it. */
+struct SiddonRay {
+    float r, sn, cs, slope, inv, len, down;
+};
+
+__device__ __forceinline__ SiddonRay siddon_ray(int dir, float sr, float cr)
+{
+    SiddonRay q;
+    q.r = sqrtf(sr * sr + cr * cr);
+    q.sn = sr / q.r;
+    q.cs = cr / q.r;
+    q.slope = dir ? q.sn / q.cs : q.cs / q.sn;
+    q.inv = fminf(1.0f / fabsf(q.slope), 3.0e38f);       /* slope 0: the whole slab in one column */
+    q.len = 1.0f / fabsf(dir ? q.cs : q.sn);
+    q.down = q.slope >= 0.0f ? 0.0f : 1.0f;
+    return q;
+}
+
+/* rows: X(Y) = (u0 + Y sin) / cos; columns: Y(X) = (X cos - u0) / sin */
+__device__ __forceinline__ float siddon_start(const SiddonRay &q, int dir, int k, int n, float axis)
+{
+    const float half = 0.5f * (float) n, u0 = (((float) k + 0.5f) - axis) / q.r;
+    return (dir ? u0 / q.cs : (-u0) / q.sn) + (-half) * q.slope + half;
+}
+
+template <int J, int A, bool WIN, int AR>
 __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int dpart, int slice,
                                         unsigned char *smem_raw)
 {
@@ -161,22 +195,36 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
      * one angle travel as a pair through packed FP32. Slots past the tile's
      * angles or the CTA's detectors repeat its last angle or detector (their
      * sums are not written), so every slot holds a ray of the image. */
+    constexpr bool FM = AR == kArithFast, SID = AR == kArithSiddon;
     const bool nonfinite = !FM && P.nonfinite && __ldg(P.nonfinite) != 0;
     constexpr int A2 = A / 2;
     const int lane = (int) (threadIdx.x & 31), warp = (int) (threadIdx.x >> 5);
     const int g = lane >> 4;
     const int d0 = dstart + warp * 32 * J + (lane & 15);
     float2 c[A2][J], inner[A2][J], sum[A2][J], stp[A2];
+    float inv[A2], down[A2];      /* siddon only */
 #pragma unroll
     for (int k = 0; k < A2; ++k) {
         const int angle = tile.x + min(g + 2 * k, tile.y - 1);
         float st, det_step;
-        joseph::ray_steps(dir, __ldg(P.sinv + angle), __ldg(P.cosv + angle), det_step, st);
+        SiddonRay ray;
+        if (SID) {
+            ray = siddon_ray(dir, __ldg(P.sinv + angle), __ldg(P.cosv + angle));
+            st = ray.slope;
+            inv[k] = ray.inv;
+            down[k] = ray.down;
+        } else {
+            joseph::ray_steps(dir, __ldg(P.sinv + angle), __ldg(P.cosv + angle), det_step, st);
+        }
         stp[k] = joseph::splat(st);
 #pragma unroll
         for (int m = 0; m < J; ++m) {
             const int s0 = min(d0 + 32 * m, dend - 1), s1 = min(d0 + 32 * m + 16, dend - 1);
-            c[k][m] = make_float2(joseph::ray_start(kc, s0, n, det_step, st), joseph::ray_start(kc, s1, n, det_step, st));
+            if (SID)
+                c[k][m] = make_float2(siddon_start(ray, dir, s0, n, P.axis), siddon_start(ray, dir, s1, n, P.axis));
+            else
+                c[k][m] = make_float2(joseph::ray_start(kc, s0, n, det_step, st),
+                                      joseph::ray_start(kc, s1, n, det_step, st));
             inner[k][m] = make_float2(0.0f, 0.0f);
             sum[k][m] = make_float2(0.0f, 0.0f);
         }
@@ -191,11 +239,22 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
      * slots after it, as taps outside the image read the zero border. */
     if (win && threadIdx.x < A) {
         const int a = (int) threadIdx.x;
-        float det_step = 0.0f, st = 0.0f;
-        if (a < tile.y)
-            joseph::ray_steps(dir, __ldg(P.sinv + tile.x + a), __ldg(P.cosv + tile.x + a), det_step, st);
-        ext[a] = a < tile.y ? joseph::ray_start(kc, dstart, n, det_step, st) : 0.0f;
-        ext[A + a] = a < tile.y ? joseph::ray_start(kc, dend - 1, n, det_step, st) : 0.0f;
+        float det_step = 0.0f, st = 0.0f, ca = 0.0f, cb = 0.0f;
+        if (a < tile.y) {
+            const float sn = __ldg(P.sinv + tile.x + a), cs = __ldg(P.cosv + tile.x + a);
+            if (SID) {
+                const SiddonRay ray = siddon_ray(dir, sn, cs);
+                st = ray.slope;
+                ca = siddon_start(ray, dir, dstart, n, P.axis) + fmaf(ray.down, st, 0.5f);
+                cb = siddon_start(ray, dir, dend - 1, n, P.axis) + fmaf(ray.down, st, 0.5f);
+            } else {
+                joseph::ray_steps(dir, sn, cs, det_step, st);
+                ca = joseph::ray_start(kc, dstart, n, det_step, st);
+                cb = joseph::ray_start(kc, dend - 1, n, det_step, st);
+            }
+        }
+        ext[a] = ca;
+        ext[A + a] = cb;
         ext[2 * A + a] = st;
     }
     /* window start (a multiple of 4 columns) of the chunk at row r0 */
@@ -275,16 +334,28 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
         /* in FP32 and fast division: the error (< 0.01 column) is part of P.drift */
         const float sn = __ldg(P.sinv + angle), cs = __ldg(P.cosv + angle);
         const float inv = __fdividef(1.0f, dir == 0 ? sn : cs), st = (dir == 0 ? cs : sn) * inv;
+        /* the siddon coordinate, a column boundary, is this one's less 0.5, or
+         * the slab's other end (st < 0) */
         const float cc = fmaf(0.5f + kc.ros + (float) s - 0.5f * (float) n, dir == 0 ? -inv : inv,
-                              fmaf(-kc.os, st, 0.5f * (float) n));
+                              fmaf(-kc.os, st, 0.5f * (float) n)) +
+                         (SID ? 0.5f + fminf(st, 0.0f) : 0.0f);
         ray_rows(cc, st, 0.5f + P.drift, (float) n + 1.5f - P.drift, n, true, rin0, rin1);
         ray_rows(cc, st, -0.5f - P.drift, (float) n + 0.5f + P.drift, n, false, rout0, rout1);
         rin0 = __reduce_max_sync(0xffffffffu, rin0);
         rin1 = __reduce_min_sync(0xffffffffu, rin1);
         rout0 = __reduce_min_sync(0xffffffffu, rout0);
         rout1 = __reduce_max_sync(0xffffffffu, rout1);
-        /* the inside form's filter (joseph::lerp2n) needs finite data */
-        if (rin0 >= rin1 || nonfinite)
+        /* the inside form's filter (joseph::lerp2n) needs finite data, and its
+         * siddon coordinate slopes of one sign */
+        bool mixed = false;
+        if (SID) {
+            const float first = __shfl_sync(0xffffffffu, down[0], 0);
+#pragma unroll
+            for (int k = 0; k < A2; ++k)
+                mixed = mixed || down[k] != first;
+            mixed = __any_sync(0xffffffffu, mixed);
+        }
+        if (rin0 >= rin1 || nonfinite || mixed)
             rin0 = rin1 = n + 64;
     }
 
@@ -317,14 +388,29 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
             const bool outside = r0 + rows <= rout0 || r0 >= rout1;
             if (inside) {
                 /* address = row + 4 (floor(c - 0.5) + kPadL - w0) = base + 4 bits(y) */
-                uint32_t base = row_s0 + 4u * (uint32_t) (kPadL - w0) - 4u * (uint32_t) joseph::kHalfFloorBits;
+                uint32_t base = row_s0 + 4u * (uint32_t) (kPadL - w0) -
+                                4u * (uint32_t) (SID ? joseph::kFloorMagicBits : joseph::kHalfFloorBits);
+                float2 jf = joseph::splat((float) r0 + (SID ? down[0] : 0.0f));
 /* more rows at once outgrow the instruction cache at small n */
-#pragma unroll (J == 1 ? 2 : 4)
+#pragma unroll (J == 1 ? 3 : 4)
                 for (int r = 0; r < rows; ++r, base += 4u * (uint32_t) wstride) {
 #pragma unroll
                     for (int k = 0; k < A2; ++k) {
 #pragma unroll
                         for (int m = 0; m < J; ++m) {
+                            if (SID) {
+                                float2 fr;
+                                const float2 y = joseph::floor2(joseph::fma2(jf, stp[k], c[k][m]), fr);
+                                const uint32_t a0 = base + 4u * (uint32_t) __float_as_int(y.x);
+                                const uint32_t a1 = base + 4u * (uint32_t) __float_as_int(y.y);
+                                const float2 t0 = make_float2(joseph::lds(a0), joseph::lds(a1));
+                                const float2 t1 = make_float2(joseph::lds(a0 + 4u), joseph::lds(a1 + 4u));
+                                /* the share of the slab left of the boundary */
+                                const float2 w = make_float2(joseph::fma_sat(-inv[k], fr.x, inv[k]),
+                                                             joseph::fma_sat(-inv[k], fr.y, inv[k]));
+                                inner[k][m] = joseph::lerp_acc_fast2(inner[k][m], w, t1, t0);
+                                continue;
+                            }
                             float2 t;
                             const float2 y = FM ? joseph::floor_half2(c[k][m], t) : joseph::floor_half2n(c[k][m], t);
                             const uint32_t a0 = base + 4u * (uint32_t) __float_as_int(y.x);
@@ -336,9 +422,11 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
                             c[k][m] = joseph::add2(c[k][m], stp[k]);
                         }
                     }
+                    if (SID)
+                        jf = joseph::add2(jf, joseph::splat(1.0f));
                 }
             } else if (outside) {
-                for (int r = 0; r < rows; ++r) {
+                for (int r = 0; r < rows && !SID; ++r) {
 #pragma unroll
                     for (int k = 0; k < A2; ++k)
 #pragma unroll
@@ -347,6 +435,10 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
                 }
             } else {
                 uint32_t row_s = row_s0;
+                float2 jf[A2];
+#pragma unroll
+                for (int k = 0; k < A2; ++k)
+                    jf[k] = joseph::splat((float) r0 + (SID ? down[k] : 0.0f));
 #pragma unroll 1
                 for (int r = 0; r < rows; ++r, row_s += 4u * (uint32_t) wstride) {
 #pragma unroll
@@ -354,16 +446,26 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
 #pragma unroll
                         for (int m = 0; m < J; ++m) {
                             float2 t;
-                            const float2 y = joseph::floor_any2(c[k][m], t);
+                            const float2 y = SID ? joseph::floor2(joseph::fma2(jf[k], stp[k], c[k][m]), t)
+                                                 : joseph::floor_any2(c[k][m], t);
                             const uint32_t p0 = min((uint32_t) (__float_as_int(y.x) - colbits), lim);
                             const uint32_t p1 = min((uint32_t) (__float_as_int(y.y) - colbits), lim);
                             const uint32_t a0 = row_s + 4u * p0, a1 = row_s + 4u * p1;
                             const float2 t0 = make_float2(joseph::lds(a0), joseph::lds(a1));
                             const float2 t1 = make_float2(joseph::lds(a0 + 4u), joseph::lds(a1 + 4u));
+                            if (SID) {
+                                const float wx = joseph::fma_sat(-inv[k], t.x, inv[k]);
+                                const float wy = joseph::fma_sat(-inv[k], t.y, inv[k]);
+                                inner[k][m].x += wx * t0.x + (1.0f - wx) * t1.x;
+                                inner[k][m].y += wy * t0.y + (1.0f - wy) * t1.y;
+                                continue;
+                            }
                             inner[k][m] = FM ? joseph::lerp_acc_fast2(inner[k][m], t, t0, t1)
                                              : joseph::add2(inner[k][m], joseph::lerp2(t, t0, t1, z2));
                             c[k][m] = joseph::add2(c[k][m], stp[k]);
                         }
+                        if (SID)
+                            jf[k] = joseph::add2(jf[k], joseph::splat(1.0f));
                     }
                 }
             }
@@ -409,6 +511,7 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
         if (a >= tile.y)
             continue;
         const int angle = tile.x + a;
+        const float len = SID ? siddon_ray(dir, __ldg(P.sinv + angle), __ldg(P.cosv + angle)).len : 0.0f;
 #pragma unroll
         for (int i = 0; i < 2 * J; ++i) {
             const int s = d0 + i * 16;
@@ -417,7 +520,9 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
             const size_t oidx = (size_t) slice * P.sino_stride + (size_t) angle * n + s;
             float result = P.src ? P.src[oidx] : 0.0f;
             const float ray = (i & 1) ? sum[k][i >> 1].y : sum[k][i >> 1].x;
-            if (!joseph::detector_inactive(kc, s))
+            if (SID)
+                result += P.scale * (ray * len);
+            else if (!joseph::detector_inactive(kc, s))
                 result = __fadd_rn(result, __fmul_rn(ray, P.scale));
             if (P.w)
                 result = __fmul_rn(result, P.w[(size_t) slice * P.w_stride + (size_t) angle * n + s]);
@@ -426,12 +531,12 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
     }
 }
 
-template <int J, int A, bool WIN, bool FM>
+template <int J, int A, bool WIN, int AR>
 __global__ void __launch_bounds__(WIN ? kMaxWinThreads : 768, (WIN && J == 1 && A <= 4) ? 2 : 1)
     fp_tiles_kernel(const __grid_constant__ FpTileArgs P)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    fp_tile<J, A, WIN, FM>(P, (int) (blockIdx.x / (unsigned) P.dsplit), (int) (blockIdx.x % (unsigned) P.dsplit),
+    fp_tile<J, A, WIN, AR>(P, (int) (blockIdx.x / (unsigned) P.dsplit), (int) (blockIdx.x % (unsigned) P.dsplit),
                        (int) blockIdx.y, smem_raw);
 }
 
@@ -441,7 +546,7 @@ __global__ void __launch_bounds__(WIN ? kMaxWinThreads : 768, (WIN && J == 1 && 
  * item_start[j + 1]; its record (the job's FpTileArgs) is staged in shared
  * memory. Jobs whose active flag is 0 are skipped.
  */
-template <int J, int A, bool WIN, bool FM>
+template <int J, int A, bool WIN, int AR>
 __global__ void __launch_bounds__(WIN ? kMaxWinThreads : 768, (WIN && J == 1 && A <= 4) ? 2 : 1)
     fp_tiles_batch_kernel(const FpTileArgs *__restrict__ recs, const int *__restrict__ item_start, int n_jobs,
                           const int *__restrict__ job_index, const int *__restrict__ active)
@@ -473,7 +578,7 @@ __global__ void __launch_bounds__(WIN ? kMaxWinThreads : 768, (WIN && J == 1 && 
     }
     __syncthreads();
     const int local = b - __ldg(item_start + j);
-    fp_tile<J, A, WIN, FM>(rec, local / rec.dsplit, local % rec.dsplit, 0, smem_raw);
+    fp_tile<J, A, WIN, AR>(rec, local / rec.dsplit, local % rec.dsplit, 0, smem_raw);
 }
 
 /* One 32 x 32 block (bx, by) of an image's padded copy and padded transpose,
@@ -543,7 +648,7 @@ TileCfg tile_cfg(int n, int smem_optin)
     return c;
 }
 
-template <int J, int A, bool WIN, bool FM>
+template <int J, int A, bool WIN, int AR>
 int launch_tiles(udev *d, const FpTileArgs &args, int n_tiles, int n_slices, int threads, size_t smem)
 {
     for (int done = 0; done < n_slices;) {
@@ -557,7 +662,7 @@ int launch_tiles(udev *d, const FpTileArgs &args, int n_tiles, int n_slices, int
         if (B.w)
             B.w += (size_t) done * args.w_stride;
         const dim3 grid((unsigned int) (n_tiles * args.dsplit), (unsigned int) chunk);
-        fp_tiles_kernel<J, A, WIN, FM><<<grid, threads, smem, d->stream>>>(B);
+        fp_tiles_kernel<J, A, WIN, AR><<<grid, threads, smem, d->stream>>>(B);
         int rc = udev_after_launch(d, "fp_tiles_kernel");
         if (rc)
             return rc;
@@ -614,41 +719,44 @@ extern "C" int udev_fp_tile_angles(udev *d, int n)
     return tiles_supported(cfg, d->smem_optin) ? cfg.A : 0;
 }
 
-template <bool FM>
+template <int AR>
 static int kernels_init_fm(udev *d)
 {
 #define UDEV_TILE_ATTR(K_, bytes)                                                                              \
     UDEV_CHECK(d, cudaFuncSetAttribute(K_, cudaFuncAttributeMaxDynamicSharedMemorySize, (bytes)))
-    UDEV_TILE_ATTR((fp_tiles_kernel<1, 8, false, FM>), d->smem_optin);
-    UDEV_TILE_ATTR((fp_tiles_kernel<2, 8, false, FM>), d->smem_optin);
-    UDEV_TILE_ATTR((fp_tiles_kernel<4, 4, false, FM>), d->smem_optin);
-    UDEV_TILE_ATTR((fp_tiles_kernel<8, 2, false, FM>), d->smem_optin);
-    UDEV_TILE_ATTR((fp_tiles_kernel<1, 8, true, FM>), d->smem_optin);
-    UDEV_TILE_ATTR((fp_tiles_kernel<2, 8, true, FM>), d->smem_optin);
-    UDEV_TILE_ATTR((fp_tiles_kernel<4, 4, true, FM>), d->smem_optin);
-    UDEV_TILE_ATTR((fp_tiles_kernel<8, 2, true, FM>), d->smem_optin);
-    UDEV_TILE_ATTR((fp_tiles_kernel<1, 4, true, FM>), d->smem_optin);
-    UDEV_TILE_ATTR((fp_tiles_kernel<1, 2, true, FM>), d->smem_optin);
+    UDEV_TILE_ATTR((fp_tiles_kernel<1, 8, false, AR>), d->smem_optin);
+    UDEV_TILE_ATTR((fp_tiles_kernel<2, 8, false, AR>), d->smem_optin);
+    UDEV_TILE_ATTR((fp_tiles_kernel<4, 4, false, AR>), d->smem_optin);
+    UDEV_TILE_ATTR((fp_tiles_kernel<8, 2, false, AR>), d->smem_optin);
+    UDEV_TILE_ATTR((fp_tiles_kernel<1, 8, true, AR>), d->smem_optin);
+    UDEV_TILE_ATTR((fp_tiles_kernel<2, 8, true, AR>), d->smem_optin);
+    UDEV_TILE_ATTR((fp_tiles_kernel<4, 4, true, AR>), d->smem_optin);
+    UDEV_TILE_ATTR((fp_tiles_kernel<8, 2, true, AR>), d->smem_optin);
+    UDEV_TILE_ATTR((fp_tiles_kernel<1, 4, true, AR>), d->smem_optin);
+    UDEV_TILE_ATTR((fp_tiles_kernel<1, 2, true, AR>), d->smem_optin);
+    if (AR == kArithSiddon)      /* no mixed batches */
+        return UFOIR_OK;
     /* the batch kernels also hold their record in static shared memory */
     const int batch_dyn = d->smem_optin - (int) kBatchStatic;
-    UDEV_TILE_ATTR((fp_tiles_batch_kernel<1, 8, false, FM>), batch_dyn);
-    UDEV_TILE_ATTR((fp_tiles_batch_kernel<2, 8, false, FM>), batch_dyn);
-    UDEV_TILE_ATTR((fp_tiles_batch_kernel<4, 4, false, FM>), batch_dyn);
-    UDEV_TILE_ATTR((fp_tiles_batch_kernel<8, 2, false, FM>), batch_dyn);
-    UDEV_TILE_ATTR((fp_tiles_batch_kernel<1, 8, true, FM>), batch_dyn);
-    UDEV_TILE_ATTR((fp_tiles_batch_kernel<2, 8, true, FM>), batch_dyn);
-    UDEV_TILE_ATTR((fp_tiles_batch_kernel<4, 4, true, FM>), batch_dyn);
-    UDEV_TILE_ATTR((fp_tiles_batch_kernel<8, 2, true, FM>), batch_dyn);
-    UDEV_TILE_ATTR((fp_tiles_batch_kernel<1, 4, true, FM>), batch_dyn);
-    UDEV_TILE_ATTR((fp_tiles_batch_kernel<1, 2, true, FM>), batch_dyn);
+    UDEV_TILE_ATTR((fp_tiles_batch_kernel<1, 8, false, (AR == kArithSiddon ? kArithExact : AR)>), batch_dyn);
+    UDEV_TILE_ATTR((fp_tiles_batch_kernel<2, 8, false, (AR == kArithSiddon ? kArithExact : AR)>), batch_dyn);
+    UDEV_TILE_ATTR((fp_tiles_batch_kernel<4, 4, false, (AR == kArithSiddon ? kArithExact : AR)>), batch_dyn);
+    UDEV_TILE_ATTR((fp_tiles_batch_kernel<8, 2, false, (AR == kArithSiddon ? kArithExact : AR)>), batch_dyn);
+    UDEV_TILE_ATTR((fp_tiles_batch_kernel<1, 8, true, (AR == kArithSiddon ? kArithExact : AR)>), batch_dyn);
+    UDEV_TILE_ATTR((fp_tiles_batch_kernel<2, 8, true, (AR == kArithSiddon ? kArithExact : AR)>), batch_dyn);
+    UDEV_TILE_ATTR((fp_tiles_batch_kernel<4, 4, true, (AR == kArithSiddon ? kArithExact : AR)>), batch_dyn);
+    UDEV_TILE_ATTR((fp_tiles_batch_kernel<8, 2, true, (AR == kArithSiddon ? kArithExact : AR)>), batch_dyn);
+    UDEV_TILE_ATTR((fp_tiles_batch_kernel<1, 4, true, (AR == kArithSiddon ? kArithExact : AR)>), batch_dyn);
+    UDEV_TILE_ATTR((fp_tiles_batch_kernel<1, 2, true, (AR == kArithSiddon ? kArithExact : AR)>), batch_dyn);
 #undef UDEV_TILE_ATTR
     return UFOIR_OK;
 }
 
 int udev_kernels_init(udev *d)
 {
-    int rc = kernels_init_fm<false>(d);
-    rc = rc ? rc : kernels_init_fm<true>(d);
+    int rc = kernels_init_fm<kArithExact>(d);
+    rc = rc ? rc : kernels_init_fm<kArithFast>(d);
+    rc = rc ? rc : kernels_init_fm<kArithSiddon>(d);
     return rc ? rc : udev_sart_init(d);
 }
 
@@ -815,7 +923,7 @@ extern "C" int udev_fp_default_cfg(udev *d, const udev_geom *g, int n_tiles, int
     return UFOIR_OK;
 }
 
-template <bool FM>
+template <int AR>
 static int dispatch_tiles(udev *d, const FpTileArgs &A, const udev_fp_cfg *c, int n_tiles, int n_slices);
 
 /* A bound, in columns, of the coordinate recurrence's error over n rows: each
@@ -863,28 +971,30 @@ extern "C" int udev_fp_tiles_cfg(udev *d, const udev_geom *g, const udev_fp_cfg 
     A.wcols = c->wcols;
     A.wstride = c->wstride;
     A.margin = c->margin;
-    return c->fm ? dispatch_tiles<true>(d, A, c, n_tiles, n_slices) : dispatch_tiles<false>(d, A, c, n_tiles, n_slices);
+    return c->fm == kArithSiddon ? dispatch_tiles<kArithSiddon>(d, A, c, n_tiles, n_slices)
+           : c->fm               ? dispatch_tiles<kArithFast>(d, A, c, n_tiles, n_slices)
+                                 : dispatch_tiles<kArithExact>(d, A, c, n_tiles, n_slices);
 }
 
-template <bool FM>
+template <int AR>
 static int dispatch_tiles(udev *d, const FpTileArgs &A, const udev_fp_cfg *c, int n_tiles, int n_slices)
 {
     if (c->win) {
         switch (c->J * 16 + c->A) {
-        case 1 * 16 + 4: return launch_tiles<1, 4, true, FM>(d, A, n_tiles, n_slices, c->threads, c->smem);
-        case 1 * 16 + 2: return launch_tiles<1, 2, true, FM>(d, A, n_tiles, n_slices, c->threads, c->smem);
-        case 1 * 16 + 8: return launch_tiles<1, 8, true, FM>(d, A, n_tiles, n_slices, c->threads, c->smem);
-        case 2 * 16 + 8: return launch_tiles<2, 8, true, FM>(d, A, n_tiles, n_slices, c->threads, c->smem);
-        case 4 * 16 + 4: return launch_tiles<4, 4, true, FM>(d, A, n_tiles, n_slices, c->threads, c->smem);
-        case 8 * 16 + 2: return launch_tiles<8, 2, true, FM>(d, A, n_tiles, n_slices, c->threads, c->smem);
+        case 1 * 16 + 4: return launch_tiles<1, 4, true, AR>(d, A, n_tiles, n_slices, c->threads, c->smem);
+        case 1 * 16 + 2: return launch_tiles<1, 2, true, AR>(d, A, n_tiles, n_slices, c->threads, c->smem);
+        case 1 * 16 + 8: return launch_tiles<1, 8, true, AR>(d, A, n_tiles, n_slices, c->threads, c->smem);
+        case 2 * 16 + 8: return launch_tiles<2, 8, true, AR>(d, A, n_tiles, n_slices, c->threads, c->smem);
+        case 4 * 16 + 4: return launch_tiles<4, 4, true, AR>(d, A, n_tiles, n_slices, c->threads, c->smem);
+        case 8 * 16 + 2: return launch_tiles<8, 2, true, AR>(d, A, n_tiles, n_slices, c->threads, c->smem);
         default: break;
         }
     } else {
         switch (c->J * 16 + c->A) {
-        case 1 * 16 + 8: return launch_tiles<1, 8, false, FM>(d, A, n_tiles, n_slices, c->threads, c->smem);
-        case 2 * 16 + 8: return launch_tiles<2, 8, false, FM>(d, A, n_tiles, n_slices, c->threads, c->smem);
-        case 4 * 16 + 4: return launch_tiles<4, 4, false, FM>(d, A, n_tiles, n_slices, c->threads, c->smem);
-        case 8 * 16 + 2: return launch_tiles<8, 2, false, FM>(d, A, n_tiles, n_slices, c->threads, c->smem);
+        case 1 * 16 + 8: return launch_tiles<1, 8, false, AR>(d, A, n_tiles, n_slices, c->threads, c->smem);
+        case 2 * 16 + 8: return launch_tiles<2, 8, false, AR>(d, A, n_tiles, n_slices, c->threads, c->smem);
+        case 4 * 16 + 4: return launch_tiles<4, 4, false, AR>(d, A, n_tiles, n_slices, c->threads, c->smem);
+        case 8 * 16 + 2: return launch_tiles<8, 2, false, AR>(d, A, n_tiles, n_slices, c->threads, c->smem);
         default: break;
         }
     }
@@ -944,35 +1054,35 @@ extern "C" int udev_fp_record(udev *d, const udev_geom *g, const udev_fp_cfg *c,
     return UFOIR_OK;
 }
 
-template <int J, int A, bool WIN, bool FM>
+template <int J, int A, bool WIN, int AR>
 static int launch_batch(udev *d, const udev_fp_cfg *c, const void *recs, const int *item_start, int n_jobs,
                         const int *job_index, const int *active, int n_items)
 {
-    fp_tiles_batch_kernel<J, A, WIN, FM><<<(unsigned int) n_items, c->threads, c->smem, d->stream>>>(
+    fp_tiles_batch_kernel<J, A, WIN, AR><<<(unsigned int) n_items, c->threads, c->smem, d->stream>>>(
         static_cast<const FpTileArgs *>(recs), item_start, n_jobs, job_index, active);
     return udev_after_launch(d, "fp_tiles_batch_kernel");
 }
 
-template <bool FM>
+template <int AR>
 static int dispatch_batch(udev *d, const udev_fp_cfg *c, const void *r, const int *st, int nj, const int *ji,
                           const int *ac, int ni)
 {
     if (c->win) {
         switch (c->J * 16 + c->A) {
-        case 1 * 16 + 4: return launch_batch<1, 4, true, FM>(d, c, r, st, nj, ji, ac, ni);
-        case 1 * 16 + 2: return launch_batch<1, 2, true, FM>(d, c, r, st, nj, ji, ac, ni);
-        case 1 * 16 + 8: return launch_batch<1, 8, true, FM>(d, c, r, st, nj, ji, ac, ni);
-        case 2 * 16 + 8: return launch_batch<2, 8, true, FM>(d, c, r, st, nj, ji, ac, ni);
-        case 4 * 16 + 4: return launch_batch<4, 4, true, FM>(d, c, r, st, nj, ji, ac, ni);
-        case 8 * 16 + 2: return launch_batch<8, 2, true, FM>(d, c, r, st, nj, ji, ac, ni);
+        case 1 * 16 + 4: return launch_batch<1, 4, true, AR>(d, c, r, st, nj, ji, ac, ni);
+        case 1 * 16 + 2: return launch_batch<1, 2, true, AR>(d, c, r, st, nj, ji, ac, ni);
+        case 1 * 16 + 8: return launch_batch<1, 8, true, AR>(d, c, r, st, nj, ji, ac, ni);
+        case 2 * 16 + 8: return launch_batch<2, 8, true, AR>(d, c, r, st, nj, ji, ac, ni);
+        case 4 * 16 + 4: return launch_batch<4, 4, true, AR>(d, c, r, st, nj, ji, ac, ni);
+        case 8 * 16 + 2: return launch_batch<8, 2, true, AR>(d, c, r, st, nj, ji, ac, ni);
         default: break;
         }
     } else {
         switch (c->J * 16 + c->A) {
-        case 1 * 16 + 8: return launch_batch<1, 8, false, FM>(d, c, r, st, nj, ji, ac, ni);
-        case 2 * 16 + 8: return launch_batch<2, 8, false, FM>(d, c, r, st, nj, ji, ac, ni);
-        case 4 * 16 + 4: return launch_batch<4, 4, false, FM>(d, c, r, st, nj, ji, ac, ni);
-        case 8 * 16 + 2: return launch_batch<8, 2, false, FM>(d, c, r, st, nj, ji, ac, ni);
+        case 1 * 16 + 8: return launch_batch<1, 8, false, AR>(d, c, r, st, nj, ji, ac, ni);
+        case 2 * 16 + 8: return launch_batch<2, 8, false, AR>(d, c, r, st, nj, ji, ac, ni);
+        case 4 * 16 + 4: return launch_batch<4, 4, false, AR>(d, c, r, st, nj, ji, ac, ni);
+        case 8 * 16 + 2: return launch_batch<8, 2, false, AR>(d, c, r, st, nj, ji, ac, ni);
         default: break;
         }
     }
@@ -990,8 +1100,8 @@ extern "C" int udev_fp_batch(udev *d, const udev_fp_cfg *c, const void *d_record
         return UFOIR_ERR_UNSUPPORTED;
     }
     UDEV_BIND(d);
-    return c->fm ? dispatch_batch<true>(d, c, d_records, d_item_start, n_jobs, d_job_index, d_active, n_items)
-                 : dispatch_batch<false>(d, c, d_records, d_item_start, n_jobs, d_job_index, d_active, n_items);
+    return c->fm ? dispatch_batch<kArithFast>(d, c, d_records, d_item_start, n_jobs, d_job_index, d_active, n_items)
+                 : dispatch_batch<kArithExact>(d, c, d_records, d_item_start, n_jobs, d_job_index, d_active, n_items);
 }
 
 /* Padded copies of the volumes of a mixed batch: one launch, 32 x 32 tiles. */

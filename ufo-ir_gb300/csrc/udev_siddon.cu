@@ -16,12 +16,15 @@
  *   L(d) = 1 / max(a, b)                 for |d| <= |a - b| / 2,
  *   L(d) = ((a + b) / 2 - |d|) / (a b)   up to |d| = (a + b) / 2, 0 beyond.
  *
- * Forward: one thread per ray walks the slabs (rows for |cos| >= |sin|,
- * columns otherwise) of the zero-padded image or its padded transpose, the
- * copies the Joseph forward projector reads; in a slab the ray covers at
- * most two pixels, and its length in the slab (1 / max(a, b)) splits where
- * it crosses the pixel boundary. Backward: one thread per pixel evaluates L for the (at most
- * two) bins whose lines cross the pixel, per angle. Both compute the same
+ * Forward: a ray walks the slabs (rows for |cos| >= |sin|, columns
+ * otherwise) of the zero-padded image or its padded transpose, the copies the
+ * Joseph forward projector reads; in a slab it covers at most two pixels, and
+ * its length in the slab (1 / max(a, b)) splits where it crosses the pixel
+ * boundary. Whole angle sets run in the Joseph projector's tiles
+ * (udev_fp_tiles.cu, 1.62 -> 1.03 ms for one slice of 1448^2 x 1200); the
+ * kernel here, one thread per ray, serves subsets and sizes beyond the tiles'.
+ * Backward: one register sum per pixel evaluates L for the (at most two) bins
+ * whose lines cross the pixel, per angle. Both compute the same
  * chord lengths, so the backprojector is the adjoint of the forward one up
  * to rounding. Arithmetic is FP32; the sums are per ray in slab order and
  * per pixel in angle order, with the reference's contract for accumulation
@@ -29,6 +32,8 @@
  */
 #include <cuda_runtime.h>
 
+#include "bp_shapes.cuh"
+#include "joseph.cuh"
 #include "udev_internal.cuh"
 
 namespace {
@@ -139,6 +144,7 @@ struct SiddonBpArgs {
     const float *cosv;
     int n;
     int n_subsets;
+    int total_angles;
     float axis;
     float relax;
     long long vol_stride;
@@ -147,130 +153,287 @@ struct SiddonBpArgs {
     unsigned int sub_n[kMaxSub];
 };
 
-/* Per angle, per block: the constants of L and the bin coordinate of the
- * block's centre, C = Xc cos - Yc sin + axis - 0.5, split as kb + frac
- * (kb an integer, frac a float). */
-struct SiddonAngle {
-    float4 geo;     /* cos, sin, frac, 1 / r */
-    float4 shape;   /* p, w / (a b), h = 1 / max(a, b), 1 / (a b) */
-    int kb;
+/*
+ * Backprojection on the tiles of the Joseph one (bp_shapes.cuh): the CTA
+ * stages, per angle, the detector window its pixels can reach, and a thread
+ * keeps one register sum per pixel. With t the bin coordinate of a pixel's
+ * centre (less 0.5), only bins floor(t) and floor(t) + 1 can cross it, at
+ * distances f = frac(t) and 1 - f, and the trapezoid is its slope clamped:
+ * L = h sat(q (w - f / r)) with q = 1 / min(a, b), as the slope reaches h at p.
+ * So a pixel pair takes the coordinate (1 packed operation, with COLS / 2 + PR
+ * products an angle), the floor (3), four saturating multiply-adds, two taps
+ * and three multiply-adds.
+ *
+ * A pixel's t is the tile centre's bin coordinate C = Xc cos - Yc sin + axis -
+ * 0.5, kept as an integer kb and a fraction, plus its offset (|dx| <= 63.5,
+ * |dy| <= 31.5) times cos and sin: ~4e-6 bins of rounding.
+ *
+ * Bound by the FMA pipe. Global gathers for two pixels a thread, with the
+ * trapezoid by comparison (64 instructions a pixel pair), took 2.39 ms for one
+ * slice of 1448^2 x 1200; this takes 1.21.
+ */
+using namespace bp;
+
+struct __align__(16) SiddonAngle {
+    float2 cs, sn;
+    float2 h;            /* chord where the line misses both corners' slopes */
+    float frac;
+    float a, b, c;       /* L / h = sat(a - b f) and sat(c + b f) */
+    uint32_t base;       /* shared address of bin kb, less the floor bits */
+    int w0;
 };
 
-constexpr int kBpW = 32, kBpH = 8, kBpThreads = kBpW * kBpH;
-constexpr int kBpPx = 2;                       /* pixels per thread, 32 columns apart */
-constexpr int kBpTileW = kBpW * kBpPx;         /* tile: 64 x 8 pixels */
+template <class T>
+struct __align__(16) SiddonSmem {
+    float win[2][kAC][T::Win];
+    SiddonAngle ang[2][kAC];
+    unsigned int aligned[2];     /* angles of a chunk that take siddon_aligned */
+};
 
-/* Grid (ceil(n / 64), ceil(n / 8), slices), block 32 x 8: a thread owns
- * pixels tx and tx + 32 of its tile row.
- * The block's threads stage up to 256 angles' constants in shared memory,
- * then each pixel visits the two bins whose lines can cross it: with
- * t = uc - 0.5 the bin coordinate of its centre, bins floor(t) and
- * floor(t) + 1 at distances frac(t) and 1 - frac(t) (every other bin is at
- * least one bin away, beyond the support (a + b) / 2 <= 0.7072). A pixel's
- * t is the tile centre's fraction plus its offset (|dx| <= 31.5, |dy| <= 3.5)
- * times cos and sin, two fmas: ~2e-6 bins of rounding. */
-__global__ void __launch_bounds__(kBpThreads) siddon_bp_kernel(SiddonBpArgs P)
+/* Bin coordinate of (Xc, Yc), Xc cos - Yc sin + axis - 0.5, as an integer
+ * and a fraction: the products' rounding errors (exact by FMA) and both sums'
+ * (TwoSum), with explicit rounding so that no contraction merges the steps;
+ * the sum less its integer part is exact. */
+__device__ __forceinline__ void siddon_centre(float Xc, float Yc, float cr, float sr, float axis, float &kbf,
+                                              float &frac)
 {
-    __shared__ SiddonAngle ang[kBpThreads];
-    const int tid = (int) (threadIdx.y * kBpW + threadIdx.x);
-    const int i0 = (int) (blockIdx.x * kBpTileW + threadIdx.x);
-    const int j = (int) (blockIdx.y * kBpH + threadIdx.y);
-    const int slice = (int) blockIdx.z;
+    const float pa = __fmul_rn(Xc, cr), pb = __fmul_rn(Yc, sr);
+    const float ea = fmaf(Xc, cr, -pa), eb = fmaf(Yc, sr, -pb);
+    const float s1 = __fsub_rn(pa, pb);
+    const float b1 = __fsub_rn(s1, pa);
+    const float e1 = __fadd_rn(__fsub_rn(pa, __fsub_rn(s1, b1)), __fsub_rn(-pb, b1));
+    const float ax = axis - 0.5f;
+    const float hi = __fadd_rn(s1, ax);
+    const float b2 = __fsub_rn(hi, s1);
+    const float e2 = __fadd_rn(__fsub_rn(s1, __fsub_rn(hi, b2)), __fsub_rn(ax, b2));
+    kbf = floorf(hi);
+    frac = __fadd_rn(__fsub_rn(hi, kbf), __fadd_rn(__fadd_rn(e1, __fsub_rn(ea, eb)), e2));
+}
+
+/*
+ * Angles closer to an axis than kAligned: L falls from h to 0 within min(a, b)
+ * bins, so where a scan's bins meet pixel boundaries (an axis half a bin off
+ * the centre) the side a pixel falls on hangs on the coordinate's last bit.
+ * These angles (0 and 90 degrees, as a rule) keep the coordinate of 64 x 8
+ * pixel blocks and L by comparison. Returns what pixel (x, y) adds to its sum.
+ */
+constexpr float kAligned = 1.0e-3f;
+
+__device__ __noinline__ float siddon_aligned(const float *win, int w0, int width, int x, int y, int n, float axis,
+                                             float cr, float sr)
+{
+    const float half = 0.5f * (float) n;
+    const float r = sqrtf(cr * cr + sr * sr), ir = 1.0f / r;
+    const float a = fabsf(cr) * ir, b = fabsf(sr) * ir, ab = a * b;
+    float kbf, frac;
+    siddon_centre((float) ((x & ~63) + 32) - half, (float) ((y & ~7) + 4) - half, cr, sr, axis, kbf, frac);
+    const float dx = ((float) (x & 63) + 0.5f) - 32.0f, dy = ((float) (y & 7) + 0.5f) - 4.0f;
+    const float iab = ab > 0.0f ? 1.0f / ab : 3.0e38f;
+    const float p = 0.5f * fabsf(a - b), w_ab = 0.5f * (a + b) * iab, h = 1.0f / fmaxf(a, b);
+    const float t = fmaf(dx, cr, fmaf(-dy, sr, frac));
+    const float v = __fadd_rd(t, kFloorMagic);
+    const float f = t - (v - kFloorMagic);
+    const int k = (int) kbf + (__float_as_int(v) - kFloorMagicBits) - w0;
+    const float da = f * ir, db = ir - da;
+    const float la = da <= p ? h : fmaxf(0.0f, fmaf(-da, iab, w_ab));
+    const float lb = db <= p ? h : fmaxf(0.0f, fmaf(-db, iab, w_ab));
+    const float va = (unsigned int) k < (unsigned int) width ? win[k] : 0.0f;
+    const float vb = (unsigned int) (k + 1) < (unsigned int) width ? win[k + 1] : 0.0f;
+    return fmaf(lb, vb, la * va);
+}
+
+__device__ __forceinline__ int siddon_angle_of(const SiddonBpArgs &P, int vi)
+{
+    for (int k = 0; k < P.n_subsets; ++k) {
+        if (vi < (int) P.sub_n[k])
+            return (int) P.sub_offset[k] + vi;
+        vi -= (int) P.sub_n[k];
+    }
+    return 0;
+}
+
+template <class T>
+__device__ void siddon_load_chunk(const SiddonBpArgs &P, SiddonSmem<T> &S, int buf, int first, int count,
+                                  const float *sino, float Xc, float Yc)
+{
+    const int lane = (int) threadIdx.x, warp = (int) threadIdx.y;
+    bool aligned = false;
+    if (warp == 0 && lane < count) {
+        const int angle = siddon_angle_of(P, first + lane);
+        const float cr = __ldg(P.cosv + angle), sr = __ldg(P.sinv + angle);
+        const float r = sqrtf(cr * cr + sr * sr), ir = 1.0f / r;
+        const float a = fabsf(cr) * ir, b = fabsf(sr) * ir, lo_ab = fminf(a, b);
+        float kbf, frac;
+        siddon_centre(Xc, Yc, cr, sr, P.axis, kbf, frac);
+        SiddonAngle A;
+        int kb;
+        if (fabsf(kbf) < 1.0e6f) {
+            kb = (int) kbf;
+            A.cs = joseph::splat(cr);
+            A.sn = joseph::splat(sr);
+            A.frac = frac;
+            aligned = lo_ab < kAligned;
+        } else {
+            /* no bin near (an axis far outside, or no geometry): a window of zeros */
+            kb = -1000000;
+            A.cs = A.sn = joseph::splat(0.0f);
+            A.frac = 0.0f;
+        }
+        /* axis-aligned: L = h up to half a bin and 0 beyond; the slope's q
+         * stays finite and the half itself counts */
+        const float q = lo_ab > 0.0f ? 1.0f / lo_ab : 3.0e38f, edge = lo_ab > 0.0f ? 0.0f : 1.0e-6f;
+        const float w = 0.5f * (a + b) + edge;
+        A.h = joseph::splat(1.0f / fmaxf(a, b));
+        A.a = w * q;
+        A.b = ir * q;
+        A.c = (w - ir) * q;
+        const float half_x = 0.5f * (float) (T::TileX - 1), half_y = 0.5f * (float) (T::TileY - 1);
+        const float lo = A.frac - half_x * fabsf(A.cs.x) - half_y * fabsf(A.sn.x);
+        A.w0 = align_window(kb + (int) floorf(lo) - 1, sino + (size_t) angle * P.n);
+        A.base = (uint32_t) __cvta_generic_to_shared(&S.win[buf][lane][0]) + 4u * (uint32_t) (kb - A.w0) -
+                 4u * (uint32_t) joseph::kFloorMagicBits;
+        S.ang[buf][lane] = A;
+    }
+    if (warp == 0) {
+        const unsigned int m = __ballot_sync(0xffffffffu, aligned);
+        if (lane == 0)
+            S.aligned[buf] = m;
+    }
+    __syncthreads();
+    for (int slot = warp; slot < count; slot += T::TY) {
+        const int w0 = S.ang[buf][slot].w0;
+        copy_window<T>(S.win[buf][slot], sino + (ptrdiff_t) siddon_angle_of(P, first + slot) * P.n + w0, w0, P.n);
+    }
+}
+
+template <class T>
+__global__ void __launch_bounds__(T::Threads, T::CTAS) siddon_bp_kernel(const __grid_constant__ SiddonBpArgs P)
+{
+    __shared__ SiddonSmem<T> S;
     const int n = P.n;
+    const int tiles_x = (n + T::TileX - 1) / T::TileX;
+    const int x0 = ((int) blockIdx.x % tiles_x) * T::TileX, y0 = ((int) blockIdx.x / tiles_x) * T::TileY;
+    const int slice = (int) blockIdx.y;
+    const float *sino = P.sino + (size_t) slice * P.sino_stride;
     const float half = 0.5f * (float) n;
     /* tile centre and the pixels' offsets from it (all exact: half-integers) */
-    const float Xc = (float) (blockIdx.x * kBpTileW + kBpTileW / 2) - half;
-    const float Yc = (float) (blockIdx.y * kBpH + kBpH / 2) - half;
-    float dx[kBpPx];
-    bool inside[kBpPx];
-    size_t pix[kBpPx];
-    float v[kBpPx];
-    bool any = false;
+    const float Xc = (float) (x0 + T::TileX / 2) - half, Yc = (float) (y0 + T::TileY / 2) - half;
+    const int x = x0 + (int) threadIdx.x;
+    float2 dx[T::H], ndy[T::PR], sum[T::PR][T::H], v[T::PR][T::H];
 #pragma unroll
-    for (int u = 0; u < kBpPx; ++u) {
-        dx[u] = ((float) (threadIdx.x + kBpW * u) + 0.5f) - (float) (kBpTileW / 2);
-        inside[u] = i0 + kBpW * u < n && j < n;
-        any = any || inside[u];
-        pix[u] = (size_t) slice * P.vol_stride + (size_t) j * n + (size_t) (i0 + kBpW * u);
-        v[u] = (inside[u] && P.base) ? P.base[pix[u]] : 0.0f;
+    for (int h = 0; h < T::H; ++h) {
+        const float d = ((float) ((int) threadIdx.x + 2 * kTX * h) + 0.5f) - (float) (T::TileX / 2);
+        dx[h] = make_float2(d, d + (float) kTX);
     }
-    const float dy = ((float) threadIdx.y + 0.5f) - (float) (kBpH / 2);
-    const float *sino = P.sino + (size_t) slice * P.sino_stride;
-    for (int s = 0; s < P.n_subsets; ++s) {
-        const int count = (int) P.sub_n[s];
-        float sum[kBpPx];
 #pragma unroll
-        for (int u = 0; u < kBpPx; ++u)
-            sum[u] = 0.0f;
-        for (int q0 = 0; q0 < count; q0 += kBpThreads) {
-            const int nq = min(kBpThreads, count - q0);
-            if (tid < nq) {
-                const int angle = (int) P.sub_offset[s] + q0 + tid;
-                const float cr = __ldg(P.cosv + angle), sr = __ldg(P.sinv + angle);
-                const float r = sqrtf(cr * cr + sr * sr), ir = 1.0f / r;
-                const float a = fabsf(cr) * ir, b = fabsf(sr) * ir;
-                const float ab = a * b;
-                /* Xc cos - Yc sin + (axis - 0.5) as hi + lo: the products'
-                 * rounding errors (exact by FMA) and both sums' (TwoSum), with
-                 * explicit rounding so that no contraction merges the steps */
-                const float pa = __fmul_rn(Xc, cr), pb = __fmul_rn(Yc, sr);
-                const float ea = fmaf(Xc, cr, -pa), eb = fmaf(Yc, sr, -pb);
-                const float s1 = __fsub_rn(pa, pb);
-                const float b1 = __fsub_rn(s1, pa);
-                const float e1 = __fadd_rn(__fsub_rn(pa, __fsub_rn(s1, b1)), __fsub_rn(-pb, b1));
-                const float ax = P.axis - 0.5f;
-                const float hi = __fadd_rn(s1, ax);
-                const float b2 = __fsub_rn(hi, s1);
-                const float e2 = __fadd_rn(__fsub_rn(s1, __fsub_rn(hi, b2)), __fsub_rn(ax, b2));
-                const float kbf = floorf(hi);
-                SiddonAngle A;
-                /* hi - kb is exact (the fraction bits of hi) */
-                const float frac = __fadd_rn(__fsub_rn(hi, kbf), __fadd_rn(__fadd_rn(e1, __fsub_rn(ea, eb)), e2));
-                A.geo = make_float4(cr, sr, frac, ir);
-                /* 1 / (a b) stays finite (3e38) for axis-aligned angles, where
-                 * every offset beyond p = w gets L = 0 */
-                const float iab = ab > 0.0f ? 1.0f / ab : 3.0e38f;
-                A.shape = make_float4(0.5f * fabsf(a - b), 0.5f * (a + b) * iab, 1.0f / fmaxf(a, b), iab);
-                A.kb = (int) kbf;
-                ang[tid] = A;
+    for (int p = 0; p < T::PR; ++p) {
+        const int y = y0 + (int) threadIdx.y + T::TY * p;
+        ndy[p] = joseph::splat((float) (T::TileY / 2) - ((float) ((int) threadIdx.y + T::TY * p) + 0.5f));
+        const size_t row = (size_t) slice * P.vol_stride + (size_t) y * n;
+#pragma unroll
+        for (int h = 0; h < T::H; ++h) {
+            const int xa = x + 2 * kTX * h, xb = xa + kTX;
+            v[p][h] = make_float2((P.base && xa < n && y < n) ? P.base[row + xa] : 0.0f,
+                                  (P.base && xb < n && y < n) ? P.base[row + xb] : 0.0f);
+            sum[p][h] = make_float2(0.0f, 0.0f);
+        }
+    }
+    const int total = P.total_angles, nchunks = (total + kAC - 1) / kAC;
+    const float2 relax = joseph::splat(P.relax);
+    int sub = 0, sub_end = P.n_subsets > 0 ? (int) P.sub_n[0] : 0;
+    if (nchunks > 0) {
+        siddon_load_chunk<T>(P, S, 0, 0, min(kAC, total), sino, Xc, Yc);
+        cp_async_commit();
+    }
+    for (int ch = 0; ch < nchunks; ++ch) {
+        const int buf = ch & 1, first = ch * kAC, count = min(kAC, total - first);
+        if (ch + 1 < nchunks) {
+            siddon_load_chunk<T>(P, S, buf ^ 1, first + kAC, min(kAC, total - first - kAC), sino, Xc, Yc);
+            cp_async_commit();
+            cp_async_wait<1>();
+        } else {
+            cp_async_wait<0>();
+        }
+        __syncthreads();
+        for (int i = 0; i < count;) {
+            if (first + i == sub_end) {
+                /* end of a subset: v = v + relax * sum */
+#pragma unroll
+                for (int p = 0; p < T::PR; ++p)
+#pragma unroll
+                    for (int h = 0; h < T::H; ++h) {
+                        v[p][h] = joseph::fma2(relax, sum[p][h], v[p][h]);
+                        sum[p][h] = make_float2(0.0f, 0.0f);
+                    }
+                ++sub;
+                sub_end += (int) P.sub_n[sub];
+                continue;
             }
-            __syncthreads();
-            if (any) {
-                const float *row = sino + (size_t) (P.sub_offset[s] + q0) * n;
-#pragma unroll 2
-                for (int q = 0; q < nq; ++q, row += n) {
-                    const float4 g = ang[q].geo;
-                    const float4 h = ang[q].shape;
-                    const int kb = ang[q].kb;
-                    const float ty = fmaf(-dy, g.y, g.z);
+            /* up to the next subset, or axis-aligned angle */
+            const unsigned int al = S.aligned[buf] >> i;
+            if (al & 1u) {
+                const SiddonAngle A = S.ang[buf][i];
 #pragma unroll
-                    for (int u = 0; u < kBpPx; ++u) {
-                        const float t = fmaf(dx[u], g.x, ty);
-                        /* floor(t) by a round-down add of 1.5 * 2^23 (|t| < 2^22) */
-                        const float y = __fadd_rd(t, kFloorMagic);
-                        const float f = t - (y - kFloorMagic);     /* exact */
-                        const int ka = kb + (__float_as_int(y) - kFloorMagicBits);
-                        const float da = f * g.w, db = g.w - da;
-                        /* L(d) = h up to p, then (w - d) / (a b) down to 0 */
-                        const float la = da <= h.x ? h.z : fmaxf(0.0f, fmaf(-da, h.w, h.y));
-                        const float lb = db <= h.x ? h.z : fmaxf(0.0f, fmaf(-db, h.w, h.y));
-                        const float va = (unsigned int) ka < (unsigned int) n ? __ldg(row + ka) : 0.0f;
-                        const float vb = (unsigned int) (ka + 1) < (unsigned int) n ? __ldg(row + ka + 1) : 0.0f;
-                        sum[u] = fmaf(la, va, sum[u]);
-                        sum[u] = fmaf(lb, vb, sum[u]);
+                for (int p = 0; p < T::PR; ++p)
+#pragma unroll
+                    for (int h = 0; h < T::H; ++h) {
+                        const int y = y0 + (int) threadIdx.y + T::TY * p, xa = x + 2 * kTX * h;
+                        sum[p][h].x += siddon_aligned(S.win[buf][i], A.w0, T::Win, xa, y, n, P.axis, A.cs.x, A.sn.x);
+                        sum[p][h].y += siddon_aligned(S.win[buf][i], A.w0, T::Win, xa + kTX, y, n, P.axis, A.cs.x,
+                                                      A.sn.x);
+                    }
+                ++i;
+                continue;
+            }
+            const int end = min(min(count, sub_end - first), al ? i + __ffs((int) al) - 1 : count);
+#pragma unroll T::Unroll
+            for (; i < end; ++i) {
+                const SiddonAngle A = S.ang[buf][i];
+                float2 px[T::H];
+#pragma unroll
+                for (int h = 0; h < T::H; ++h)
+                    px[h] = joseph::mul2(dx[h], A.cs);
+#pragma unroll
+                for (int p = 0; p < T::PR; ++p) {
+                    const float2 py = joseph::fma2(ndy[p], A.sn, joseph::splat(A.frac));
+#pragma unroll
+                    for (int h = 0; h < T::H; ++h) {
+                        float2 f;
+                        const float2 y = joseph::floor2(joseph::add2(px[h], py), f);
+                        const uint32_t a0 = A.base + 4u * (uint32_t) __float_as_int(y.x);
+                        const uint32_t a1 = A.base + 4u * (uint32_t) __float_as_int(y.y);
+                        const float2 va = make_float2(joseph::lds(a0), joseph::lds(a1));
+                        const float2 vb = make_float2(joseph::lds(a0 + 4u), joseph::lds(a1 + 4u));
+                        const float2 la = make_float2(joseph::fma_sat(-A.b, f.x, A.a), joseph::fma_sat(-A.b, f.y, A.a));
+                        const float2 lb = make_float2(joseph::fma_sat(A.b, f.x, A.c), joseph::fma_sat(A.b, f.y, A.c));
+                        const float2 s = joseph::fma2(lb, vb, joseph::mul2(la, va));
+                        sum[p][h] = joseph::fma2(A.h, s, sum[p][h]);
                     }
                 }
             }
-            __syncthreads();
         }
-#pragma unroll
-        for (int u = 0; u < kBpPx; ++u)
-            v[u] += P.relax * sum[u];
+        __syncthreads();
     }
 #pragma unroll
-    for (int u = 0; u < kBpPx; ++u)
-        if (inside[u])
-            P.dst[pix[u]] = v[u];
+    for (int p = 0; p < T::PR; ++p) {
+        const int y = y0 + (int) threadIdx.y + T::TY * p;
+#pragma unroll
+        for (int c = 0; c < T::COLS; ++c) {
+            const int xc = x + kTX * c;
+            if (xc >= n || y >= n)
+                continue;
+            const float2 vv = joseph::fma2(relax, sum[p][c >> 1], v[p][c >> 1]);
+            P.dst[(size_t) slice * P.vol_stride + (size_t) y * n + xc] = (c & 1) ? vv.y : vv.x;
+        }
+    }
+}
+
+template <class T>
+int launch_siddon_bp(udev *d, const SiddonBpArgs &A, int n_slices)
+{
+    const dim3 grid(udev_div_up(A.n, T::TileX) * udev_div_up(A.n, T::TileY), (unsigned int) n_slices);
+    siddon_bp_kernel<T><<<grid, dim3(kTX, T::TY), 0, d->stream>>>(A);
+    return udev_after_launch(d, "siddon_bp_kernel");
 }
 
 }  // namespace
@@ -320,6 +483,7 @@ extern "C" int udev_siddon_bp(udev *d, const udev_geom *g, const ufoir_subset *s
         return UFOIR_ERR_INVALID;
     }
     SiddonBpArgs A;
+    A.total_angles = 0;
     for (int s = 0; s < n_subsets; ++s) {
         if (subsets[s].offset + subsets[s].n > (unsigned int) g->n_angles) {
             udev_set_error(d, "siddon_bp: subset %d [%u, %u) beyond %d angles", s, subsets[s].offset,
@@ -328,6 +492,7 @@ extern "C" int udev_siddon_bp(udev *d, const udev_geom *g, const ufoir_subset *s
         }
         A.sub_offset[s] = subsets[s].offset;
         A.sub_n[s] = subsets[s].n;
+        A.total_angles += (int) subsets[s].n;
     }
     UDEV_BIND(d);
     A.sino = sino;
@@ -341,7 +506,10 @@ extern "C" int udev_siddon_bp(udev *d, const udev_geom *g, const ufoir_subset *s
     A.relax = relax;
     A.vol_stride = (long long) n * n;
     A.sino_stride = (long long) g->n_angles * n;
-    dim3 grid(udev_div_up(n, kBpTileW), udev_div_up(n, kBpH), (unsigned int) n_slices);
-    siddon_bp_kernel<<<grid, dim3(kBpW, kBpH), 0, d->stream>>>(A);
-    return udev_after_launch(d, "siddon_bp_kernel");
+    switch (bp_shape(d, n, n_slices)) {
+    case 0: return launch_siddon_bp<ShapeL>(d, A, n_slices);
+    case 1: return launch_siddon_bp<ShapeM>(d, A, n_slices);
+    case 2: return launch_siddon_bp<ShapeS>(d, A, n_slices);
+    default: return launch_siddon_bp<ShapeT>(d, A, n_slices);
+    }
 }
