@@ -461,6 +461,19 @@ int ufoir_sirt_batch_profile(ufoir_sirt_batch *b, float ms[3])
 /* ------------------------------------------------------------------------ */
 /* SART                                                                     */
 /* ------------------------------------------------------------------------ */
+/* 1 if no ray of p is steeper than the split form of the sweep kernel takes
+ * (a direction given by the caller may be). */
+static int sart_split(const ufoir_projector *p)
+{
+    for (unsigned int a = 0; a < p->n_angles; a++) {
+        const double sn = p->h_sin[a], cs = p->h_cos[a];
+        const double slope = p->h_dir[a] == UFOIR_HORIZONTAL ? cs / sn : sn / cs;
+        if (!(fabs(slope) <= UDEV_SART_SPLIT_SLOPE))
+            return 0;
+    }
+    return 1;
+}
+
 int ufoir__sart_body(void *arg)
 {
     ufoir__sart_iter *s = (ufoir__sart_iter *) arg;
@@ -471,10 +484,24 @@ int ufoir__sart_body(void *arg)
      * x = x + lambda A_theta^T r_theta. The volume lives in the layout of the
      * current direction run, transposed while the angles are horizontal, so
      * that every ray walks rows.
-     * The padded kernels where they serve the geometry, else the general
-     * ones; UFOIR_SART_KERNELS=general selects the general kernels always. */
+     * The sweep kernel where it is the faster one, else the padded kernels
+     * where they serve the geometry, else the general ones; UFOIR_SART_KERNELS=general selects the general kernels always. */
     const char *only = getenv("UFOIR_SART_KERNELS");
     const int general_only = only && strcmp(only, "general") == 0;
+    const int split = sart_split(s->p);
+    if (!general_only && udev_sart_sweep_serves(d, &s->g, split, S)) {
+        /* one kernel per run of angles of one direction */
+        unsigned int a = 0;
+        while (a < s->p->n_angles && rc == UFOIR_OK) {
+            unsigned int end = a + 1;
+            while (end < s->p->n_angles && s->p->h_dir[end] == s->p->h_dir[a])
+                end++;
+            rc = udev_sart_sweep(d, &s->g, (int) a, (int) end, s->p->h_dir[a], split, s->table, s->b, s->R, 1, s->x,
+                                 -1.0f, s->lambda, s->relax_dev, S);
+            a = end;
+        }
+        return rc;
+    }
     if (!general_only && udev_sart_padded(d, &s->g, S)) {
         /* padded copies V (vertical run) and H (horizontal run) in s->work */
         int place = -1;

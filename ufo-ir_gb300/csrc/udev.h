@@ -121,6 +121,16 @@ int udev_sart_fp(udev *d, const udev_geom *g, int angle, int dir, const float *t
                  const float *src, const float *w, int w_shared, float *out, float scale, int n_slices);
 int udev_sart_bp(udev *d, const udev_geom *g, int angle, float sn, float cs, const float *sino, float *work,
                  int place, float relax, const float *relax_dev, int n_slices);
+/* Angles [first, end), all of direction dir, in one kernel with the slice in
+ * a cluster's shared memory (udev_sart_sweep.cu): x in the user's layout,
+ * updated in place. split: every ray's slope is at most
+ * UDEV_SART_SPLIT_SLOPE (a block's columns may then be split over CTAs). */
+#define UDEV_SART_SPLIT_SLOPE 1.02
+/* 1 if that kernel serves this geometry and is the faster one for n_slices. */
+int udev_sart_sweep_serves(udev *d, const udev_geom *g, int split, int n_slices);
+int udev_sart_sweep(udev *d, const udev_geom *g, int first, int end, int dir, int split, const float *table,
+                    const float *src, const float *w, int w_shared, float *x, float scale, float relax,
+                    const float *relax_dev, int n_slices);
 
 /* ---- Tiled forward projector (all angles, shared-memory row streaming) ---- */
 /* Row pitch (floats, multiple of 4) of the padded images: 2 zero columns,

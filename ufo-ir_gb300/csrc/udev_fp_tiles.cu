@@ -757,7 +757,9 @@ int udev_kernels_init(udev *d)
     int rc = kernels_init_fm<kArithExact>(d);
     rc = rc ? rc : kernels_init_fm<kArithFast>(d);
     rc = rc ? rc : kernels_init_fm<kArithSiddon>(d);
-    return rc ? rc : udev_sart_init(d);
+    if (!rc)
+        rc = udev_sart_init(d);
+    return rc ? rc : udev_sart_sweep_init(d);
 }
 
 extern "C" int udev_pad_transpose(udev *d, const float *vol, float *volP, float *volTP, int *nonfinite, int n,

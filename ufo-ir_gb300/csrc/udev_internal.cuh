@@ -41,6 +41,9 @@ int udev_kernels_init(udev *d);
 
 /* The same for the SART per-angle kernels (non-portable cluster sizes). */
 int udev_sart_init(udev *d);
+int udev_sart_sweep_init(udev *d);
+/* Origin shift, os - ros and clamp edges of the backprojection (udev_sart.cu). */
+void udev_sart_bp_consts(const udev_geom *g, float *os, float *shift, float *e0, float *e1);
 
 #define UDEV_BIND(d)                                                                   \
     do {                                                                               \

@@ -17,7 +17,8 @@
  * rays its transpose. SART keeps the volume in the layout of the current
  * direction run (the angles of [0, pi) form three runs) and transposes it at
  * the two run boundaries; the per-angle backprojection updates either layout
- * in place. Two sets of kernels:
+ * in place. Small images, and stacks of them, run whole direction runs in the
+ * kernel of udev_sart_sweep.cu instead. Two sets of kernels here:
  *  - the padded path (sart_fp_kernel, sart_bp_kernel, sart_copy_kernel):
  *    zero-padded copies of the volume, a cluster of CTAs per group of 64
  *    rays whose block sums meet in distributed shared memory, and a tiled
@@ -927,7 +928,7 @@ extern "C" size_t udev_sart_work_floats(int n, int n_slices)
 
 /* The clamp edges of the backprojection (…joseph.cl:174-187), computed as
  * the host side of udev_bp_angle does. */
-static void sart_bp_consts(const udev_geom *g, float *os, float *shift, float *e0, float *e1)
+void udev_sart_bp_consts(const udev_geom *g, float *os, float *shift, float *e0, float *e1)
 {
     const float w = (float) g->n_dets, axis = g->axis;
     const float required_width = axis * 2.0f;
@@ -946,7 +947,7 @@ static bool sart_geometry_ok(const udev_geom *g)
     float os, shift, e0, e1;
     if (g->n_dets < 1 || g->n_dets > kMaxBlocks * kBlock)
         return false;
-    sart_bp_consts(g, &os, &shift, &e0, &e1);
+    udev_sart_bp_consts(g, &os, &shift, &e0, &e1);
     return e0 <= e1;
 }
 
@@ -1154,7 +1155,7 @@ extern "C" int udev_sart_bp(udev *d, const udev_geom *g, int angle, float sn, fl
     const int pitch = sart_pitch(n);
     const size_t plane = (size_t) sart_rows(n) * pitch;
     SartBpArgs A;
-    sart_bp_consts(g, &A.os, &A.shift, &A.e0, &A.e1);
+    udev_sart_bp_consts(g, &A.os, &A.shift, &A.e0, &A.e1);
     A.sino = sino;
     A.vol = work + (size_t) place * n_slices * plane;
     A.n = n;
