@@ -159,7 +159,8 @@ __device__ __forceinline__ float siddon_start(const SiddonRay &q, int dir, int k
     return (dir ? u0 / q.cs : (-u0) / q.sn) + (-half) * q.slope + half;
 }
 
-template <int J, int A, bool WIN, int AR>
+/* BATCH: P lies in shared memory, and its src is never NULL. */
+template <int J, int A, bool WIN, int AR, bool BATCH = false>
 __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int dpart, int slice,
                                         unsigned char *smem_raw)
 {
@@ -392,7 +393,7 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
                                 4u * (uint32_t) (SID ? joseph::kFloorMagicBits : joseph::kHalfFloorBits);
                 float2 jf = joseph::splat((float) r0 + (SID ? down[0] : 0.0f));
 /* more rows at once outgrow the instruction cache at small n */
-#pragma unroll (J == 1 ? 3 : 4)
+#pragma unroll (J == 1 || BATCH ? 3 : 4)
                 for (int r = 0; r < rows; ++r, base += 4u * (uint32_t) wstride) {
 #pragma unroll
                     for (int k = 0; k < A2; ++k) {
@@ -518,7 +519,7 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
             if (s >= dend)
                 continue;
             const size_t oidx = (size_t) slice * P.sino_stride + (size_t) angle * n + s;
-            float result = P.src ? P.src[oidx] : 0.0f;
+            float result = BATCH || P.src ? P.src[oidx] : 0.0f;
             const float ray = (i & 1) ? sum[k][i >> 1].y : sum[k][i >> 1].x;
             if (SID)
                 result += P.scale * (ray * len);
@@ -578,7 +579,7 @@ __global__ void __launch_bounds__(WIN ? kMaxWinThreads : 768, (WIN && J == 1 && 
     }
     __syncthreads();
     const int local = b - __ldg(item_start + j);
-    fp_tile<J, A, WIN, AR>(rec, local / rec.dsplit, local % rec.dsplit, 0, smem_raw);
+    fp_tile<J, A, WIN, AR, true>(rec, local / rec.dsplit, local % rec.dsplit, 0, smem_raw);
 }
 
 /* One 32 x 32 block (bx, by) of an image's padded copy and padded transpose,

@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(T::Threads, T::CTAS) siddon_bp_kernel(const __
                 continue;
             }
             const int end = min(min(count, sub_end - first), al ? i + __ffs((int) al) - 1 : count);
-#pragma unroll T::Unroll
+#pragma unroll 2
             for (; i < end; ++i) {
                 const SiddonAngle A = S.ang[buf][i];
                 float2 px[T::H];
