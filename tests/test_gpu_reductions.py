@@ -54,3 +54,28 @@ def test_dot_products(ufoir_lib, gpu_ctx, oracle, h, w):
     terms = float(np.abs(a.astype(np.float64)).max() * np.abs(b.astype(np.float64)).max()) * h * w
     # one rounding of the result to float, and FP64 rounding of every sum
     assert abs(gpu_ctx.dot_product(a, b) - want) <= 2.0 ** -24 * abs(want) + 2.0 ** -50 * terms
+
+
+# The TV gradient computes its FP64 norm beside it: image edges on and beside
+# the edges of its 32 x 32 tiles, fewer tiles than CTAs and more, several slices.
+@pytest.mark.parametrize("n,slices", [(1, 1), (31, 2), (32, 1), (33, 3), (65, 1), (300, 2), (1500, 1)])
+def test_tv_step_takes_the_norm_of_its_gradient(ufoir_lib, gpu_ctx, n, slices):
+    rng = np.random.default_rng(n + slices)
+    na = 4
+    sinos = (rng.random((slices, na, n), dtype=np.float32) + 0.5) * n
+    p = ufoir_lib.ParallelProjector(gpu_ctx, step=float(np.float32(np.pi / na)), is_forward=False)
+    kw = dict(num_iterations=1, norm_mode=ufoir_lib.NORM_FP64,
+              df_minimizer=dict(num_iterations=1, relaxation_factor=0.25))
+    vol, x_tv, sc = ufoir_lib.asdpocs_state(p, sinos, **kw)
+    p.close()
+    for s in range(slices):
+        # 20 sub-steps x -= (alpha dp / |g|_1) g from the volume before them, each
+        # operation rounded to float; the norm's 64-bit sums differ in their order
+        # only (a relative 2^-40 at most), so they round to the same float
+        x = vol[s].astype(np.float32)
+        dtgv = np.float32(0.2) * np.float32(sc[s]["dp"])
+        for _ in range(20):
+            g = ufoir_lib.tv_gradient(gpu_ctx, x[None])[0]
+            factor = dtgv / np.float32(np.abs(g.astype(np.float64)).sum())
+            x = x - factor * g
+        assert np.array_equal(x_tv[s], x), np.abs(x_tv[s] - x).max()

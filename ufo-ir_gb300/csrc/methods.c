@@ -730,8 +730,7 @@ static int asd_post_body(void *arg)
         return rc;
     /* ufo_math_tvstd_method_process_real (:550-580): 20 sub-steps */
     for (int step = 0; step < 20; step++) {
-        if ((rc = udev_l1_grad(d, s->x, s->grad, (int) n, (int) n, S)) ||
-            (rc = udev_l1_norm_to(d, s->grad, n, n, S, prm->norm_mode, s->partials, c->l1)) ||
+        if ((rc = udev_l1_grad_norm(d, s->x, s->grad, (int) n, (int) n, S, prm->norm_mode, s->partials, c->l1)) ||
             (rc = udev_asd_tv_step(d, s->x, s->grad, c, nv, S)))
             return rc;
     }

@@ -254,6 +254,9 @@ int udev_unary(udev *d, int op, const float *a, float m, float m2, float *out, s
 
 /* TV subgradient (l1_grad) of n_slices w x h images. */
 int udev_l1_grad(udev *d, const float *in, float *out, int w, int h, int n_slices);
+/* The same, and its L1 norm as udev_l1_norm_to gives it (FP64: another order of the sum). */
+int udev_l1_grad_norm(udev *d, const float *in, float *out, int w, int h, int n_slices, int mode, double *partials,
+                      float *d_out);
 /* Periodic differences. */
 enum { UDEV_DX = 0, UDEV_DXT = 1, UDEV_DY = 2, UDEV_DYT = 3 };
 int udev_diff(udev *d, int which, const float *in, float *out, int w, int h, int n_slices);

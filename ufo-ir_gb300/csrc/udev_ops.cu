@@ -86,49 +86,6 @@ __device__ __forceinline__ float tex0(const float *img, int x, int y, int w, int
     return (x >= 0 && y >= 0 && x < w && y < h) ? img[(size_t) y * w + x] : 0.0f;
 }
 
-/* l1_grad: 7-point isotropic-TV subgradient with EPS 0.001 and zero border.
- * A block computes a 32 x 32 tile, 4 rows per thread, from the tile and its
- * one-pixel halo staged in shared memory (zeros outside the image). */
-constexpr int kGradTile = 32;
-
-__global__ void __launch_bounds__(256) l1_grad_kernel(const float *in, float *out, int w, int h, long long stride)
-{
-    __shared__ float t[kGradTile + 2][kGradTile + 3];
-    const int x0 = (int) blockIdx.x * kGradTile, y0 = (int) blockIdx.y * kGradTile;
-    const float *img = in + (size_t) blockIdx.z * stride;
-    const int tid = (int) (threadIdx.y * 32 + threadIdx.x);
-    for (int e = tid; e < (kGradTile + 2) * (kGradTile + 2); e += 256) {
-        const int ty = e / (kGradTile + 2), tx = e % (kGradTile + 2);
-        t[ty][tx] = tex0(img, x0 - 1 + tx, y0 - 1 + ty, w, h);
-    }
-    __syncthreads();
-    const int lx = (int) threadIdx.x + 1, x = x0 + (int) threadIdx.x;
-    if (x >= w)
-        return;
-    const float eps = 0.001f;
-#pragma unroll
-    for (int m = 0; m < kGradTile / 8; ++m) {
-        const int ly = (int) threadIdx.y + 8 * m + 1, y = y0 + ly - 1;
-        if (y >= h)
-            break;
-        const float f3 = t[ly][lx];
-        const float f1 = t[ly - 1][lx];
-        const float f0 = t[ly - 1][lx - 1];
-        const float f2 = t[ly][lx - 1];
-        const float f4 = t[ly][lx + 1];
-        const float f6 = t[ly + 1][lx + 1];
-        const float f5 = t[ly + 1][lx];
-        const float d32 = __fsub_rn(f3, f2), d35 = __fsub_rn(f3, f5);
-        const float d43 = __fsub_rn(f4, f3), d46 = __fsub_rn(f4, f6);
-        const float d13 = __fsub_rn(f1, f3), d10 = __fsub_rn(f1, f0);
-        const float t1 = __fdiv_rn(__fsub_rn(__fsub_rn(__fmul_rn(2.0f, f3), f2), f5),
-                                   __fsqrt_rn(__fadd_rn(__fadd_rn(eps, __fmul_rn(d32, d32)), __fmul_rn(d35, d35))));
-        const float t2 = __fdiv_rn(d43, __fsqrt_rn(__fadd_rn(__fadd_rn(eps, __fmul_rn(d43, d43)), __fmul_rn(d46, d46))));
-        const float t3 = __fdiv_rn(d13, __fsqrt_rn(__fadd_rn(__fadd_rn(eps, __fmul_rn(d13, d13)), __fmul_rn(d10, d10))));
-        out[(size_t) blockIdx.z * stride + (size_t) y * w + x] = __fsub_rn(__fsub_rn(t1, t2), t3);
-    }
-}
-
 template <int WHICH>
 __global__ void diff_kernel(const float *in, float *out, int w, int h, long long stride)
 {
@@ -161,7 +118,7 @@ __device__ __forceinline__ double block_sum_double(double v)
     __shared__ double warp_sums[kRedThreads / 32];
     for (int o = 16; o > 0; o >>= 1)
         v += __shfl_down_sync(0xffffffffu, v, o);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int tid = (int) (threadIdx.y * blockDim.x + threadIdx.x), lane = tid & 31, wid = tid >> 5;
     if (lane == 0)
         warp_sums[wid] = v;
     __syncthreads();
@@ -172,6 +129,83 @@ __device__ __forceinline__ double block_sum_double(double v)
             r += __shfl_down_sync(0xffffffffu, r, o);
     }
     return r;   /* valid in thread 0 */
+}
+
+/* l1_grad: 7-point isotropic-TV subgradient with EPS 0.001 and zero border.
+ * With NORM also the FP64 sum of its magnitudes, one partial per CTA.
+ *
+ * A CTA takes 32 x 32 tiles in turn, 4 rows per thread, from the tile and its
+ * one-pixel halo staged in shared memory (zeros outside the image). Bound by
+ * issue: three divisions and square roots per pixel. The root under the
+ * second term is the first term's of the pixel to the right, taken from the
+ * next lane; lanes 0 .. 3 compute those right of the tile, one row each. The
+ * FP64 additions and conversions (2 per clock and SM) run beside it, so the
+ * norm costs little: the gradient and its norm took 38 + 40 us at 2900^2 (11 +
+ * 12 at 1448^2, 11 + 16 for four slices of 724^2) as two kernels, and take 55
+ * (17, 21) here. */
+constexpr int kGradTile = 32;
+constexpr int kGradRows = kGradTile / 8;
+constexpr int kGradCtas = 8;          /* per SM */
+constexpr int kGradBlocks = 2048;     /* per slice: as many as the reduction scratch holds */
+
+template <bool NORM>
+__global__ void __launch_bounds__(256) l1_grad_kernel(const float *in, float *out, int w, int h, long long stride,
+                                                      double *partials)
+{
+    __shared__ float t[kGradTile + 2][kGradTile + 3];
+    const int tiles_x = (w + kGradTile - 1) / kGradTile, tiles = tiles_x * ((h + kGradTile - 1) / kGradTile);
+    const float *img = in + (size_t) blockIdx.y * stride;
+    float *dst = out + (size_t) blockIdx.y * stride;
+    const int lane = (int) threadIdx.x, lx = lane + 1;
+    const float eps = 0.001f;
+    double acc = 0.0;
+    for (int tile = (int) blockIdx.x; tile < tiles; tile += (int) gridDim.x) {
+        const int x0 = tile % tiles_x * kGradTile, y0 = tile / tiles_x * kGradTile;
+        /* a warp stages whole rows: its 32 columns, then lanes 0 and 1 the two at the end */
+        for (int ty = (int) threadIdx.y; ty < kGradTile + 2; ty += 8) {
+            t[ty][lane] = tex0(img, x0 - 1 + lane, y0 - 1 + ty, w, h);
+            if (lane < 2)
+                t[ty][kGradTile + lane] = tex0(img, x0 - 1 + kGradTile + lane, y0 - 1 + ty, w, h);
+        }
+        __syncthreads();
+        /* sqrt(eps + (f(x, y) - f(x - 1, y))^2 + (f(x, y) - f(x, y + 1))^2) at the pixel right of the tile */
+        const int er = (int) threadIdx.y + 8 * (lane & (kGradRows - 1)) + 1;
+        const float ef = t[er][kGradTile + 1];
+        const float eh = __fsub_rn(ef, t[er][kGradTile]), ev = __fsub_rn(ef, t[er + 1][kGradTile + 1]);
+        const float edge = __fsqrt_rn(__fadd_rn(__fadd_rn(eps, __fmul_rn(eh, eh)), __fmul_rn(ev, ev)));
+#pragma unroll 4
+        for (int m = 0; m < kGradRows; ++m) {
+            const int ly = (int) threadIdx.y + 8 * m + 1, y = y0 + ly - 1, x = x0 + lane;
+            const float f3 = t[ly][lx];
+            const float f1 = t[ly - 1][lx];
+            const float f0 = t[ly - 1][lx - 1];
+            const float f2 = t[ly][lx - 1];
+            const float f4 = t[ly][lx + 1];
+            const float f5 = t[ly + 1][lx];
+            const float d32 = __fsub_rn(f3, f2), d35 = __fsub_rn(f3, f5);
+            const float d43 = __fsub_rn(f4, f3);
+            const float d13 = __fsub_rn(f1, f3), d10 = __fsub_rn(f1, f0);
+            const float n1 = __fsqrt_rn(__fadd_rn(__fadd_rn(eps, __fmul_rn(d32, d32)), __fmul_rn(d35, d35)));
+            const float n3 = __fsqrt_rn(__fadd_rn(__fadd_rn(eps, __fmul_rn(d13, d13)), __fmul_rn(d10, d10)));
+            const float right = __shfl_down_sync(0xffffffffu, n1, 1), last = __shfl_sync(0xffffffffu, edge, m);
+            const float n2 = lane == 31 ? last : right;
+            const float t1 = __fdiv_rn(__fsub_rn(__fsub_rn(__fmul_rn(2.0f, f3), f2), f5), n1);
+            const float t2 = __fdiv_rn(d43, n2);
+            const float t3 = __fdiv_rn(d13, n3);
+            const float g = __fsub_rn(__fsub_rn(t1, t2), t3);
+            if (x < w && y < h) {
+                dst[(size_t) y * w + x] = g;
+                if (NORM)
+                    acc += (double) fabsf(g);
+            }
+        }
+        __syncthreads();
+    }
+    if (NORM) {
+        acc = block_sum_double(acc);
+        if (threadIdx.x == 0 && threadIdx.y == 0)
+            partials[(size_t) blockIdx.y * gridDim.x + blockIdx.x] = acc;
+    }
 }
 
 /* FP64 l1, pass 1: block b of slice s sums a fixed contiguous chunk. */
@@ -397,14 +431,44 @@ extern "C" int udev_unary(udev *d, int op, const float *a, float m, float m2, fl
     return udev_after_launch(d, "unary_kernel");
 }
 
+/* CTAs per slice for the gradient: all that run at once, as far as there are tiles. */
+static unsigned int grad_blocks(udev *d, int w, int h, int n_slices)
+{
+    const long long tiles = (long long) udev_div_up(w, kGradTile) * udev_div_up(h, kGradTile);
+    long long blocks = ((long long) d->sm_count * kGradCtas + n_slices - 1) / n_slices;
+    if (blocks > kGradBlocks)
+        blocks = kGradBlocks;
+    return (unsigned int) (tiles < blocks ? tiles : blocks);
+}
+
 extern "C" int udev_l1_grad(udev *d, const float *in, float *out, int w, int h, int n_slices)
 {
     if (n_slices <= 0)
         return UFOIR_OK;
     UDEV_BIND(d);
-    dim3 grid(udev_div_up(w, kGradTile), udev_div_up(h, kGradTile), (unsigned int) n_slices);
-    l1_grad_kernel<<<grid, dim3(32, 8), 0, d->stream>>>(in, out, w, h, (long long) w * h);
+    const dim3 grid(grad_blocks(d, w, h, n_slices), (unsigned int) n_slices);
+    l1_grad_kernel<false><<<grid, dim3(32, 8), 0, d->stream>>>(in, out, w, h, (long long) w * h, nullptr);
     return udev_after_launch(d, "l1_grad_kernel");
+}
+
+extern "C" int udev_l1_grad_norm(udev *d, const float *in, float *out, int w, int h, int n_slices, int mode,
+                                 double *partials, float *d_out)
+{
+    int rc;
+    if (n_slices <= 0)
+        return UFOIR_OK;
+    if (mode == UFOIR_NORM_COMPAT) {
+        if ((rc = udev_l1_grad(d, in, out, w, h, n_slices)))
+            return rc;
+        return udev_l1_norm_to(d, out, (size_t) w, (size_t) h, n_slices, mode, partials, d_out);
+    }
+    UDEV_BIND(d);
+    const dim3 grid(grad_blocks(d, w, h, n_slices), (unsigned int) n_slices);
+    l1_grad_kernel<true><<<grid, dim3(32, 8), 0, d->stream>>>(in, out, w, h, (long long) w * h, partials);
+    if ((rc = udev_after_launch(d, "l1_grad_kernel")))
+        return rc;
+    sum_partials_kernel<<<n_slices, kRedThreads, 0, d->stream>>>(partials, (int) grid.x, d_out);
+    return udev_after_launch(d, "sum_partials_kernel");
 }
 
 extern "C" int udev_diff(udev *d, int which, const float *in, float *out, int w, int h, int n_slices)
