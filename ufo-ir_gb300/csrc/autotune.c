@@ -3,8 +3,8 @@
  *
  * For a geometry (n_dets, n_angles, step, axis) and a slice count, every
  * launch shape the kernels support is timed on scratch data of that
- * geometry (zeros: the kernel has no data-dependent branches, its chunk
- * forms depend on the geometry only) with CUDA events: one warm-up run,
+ * geometry (zeros: the kernel's forms depend on the geometry, and on the
+ * data only where they are not finite) with CUDA events: one warm-up run,
  * then the best of two. The fixed rules' shape is always a candidate and is
  * kept unless another is at least 2 % faster. The result is cached per
  * context and recorded on the projector, whose later forward projections
@@ -14,9 +14,9 @@
  *
  * Search space (pruned to what can pay): angles per tile A in {8, 4, 2}
  * with the detector pairs per thread J of an existing kernel variant, rows
- * per chunk K in {32, 16, 8} (shared memory permitting), and, only when the
- * tiles alone cannot fill the GPU twice over, 2, 4 or 8 CTAs per tile with
- * and without column windows.
+ * per chunk K in {32, 16, 8} (shared memory permitting), 1 to 4 CTAs per
+ * tile with whole rows, and, only when the tiles alone cannot fill the GPU
+ * twice over, 8 CTAs per tile and column windows.
  */
 #include <math.h>
 #include <stdlib.h>
