@@ -172,3 +172,23 @@ def test_siddon_tiles_and_ray_walk_agree_on_pixel_boundaries(ufoir_lib, gpu_ctx,
         p.subset_fp(vol, part, off, cnt, direction)
     p.close()
     np.testing.assert_allclose(whole, part, rtol=0, atol=2 * n * 2.0 ** -24 * float(np.abs(part).max()))
+
+
+# Launches of few tiles spread a tile's detectors over parts of whole rows or of
+# column windows, by size and by how many tiles there are; launches of many tiles
+# take other parts. The sums of a ray do not depend on it.
+@pytest.mark.parametrize("n,na,axis,arithmetic", [
+    (127, 16, -1.0, 0), (128, 16, 63.1, 0), (129, 24, -1.0, 0), (255, 60, 130.3, 0), (256, 200, -1.0, 0),
+    (257, 24, -1.0, 1), (513, 24, 250.2, 0), (640, 280, -1.0, 0), (769, 90, -1.0, 0), (1024, 40, 517.7, 0),
+    (1025, 200, -1.0, 1), (1449, 90, -1.0, 0), (1536, 30, 760.4, 0), (1537, 30, -1.0, 0)])
+def test_few_tiles_give_what_many_give(ufoir_lib, gpu_ctx, n, na, axis, arithmetic):
+    slices = 40 if n < 600 else 12
+    rng = np.random.default_rng(n + na)
+    vols = rng.standard_normal((slices, n, n), dtype=f32)
+    p = ufoir_lib.ParallelProjector(gpu_ctx, step=float(f32(np.pi / na)), axis_position=axis, is_forward=True,
+                                    angles_num=na, arithmetic=arithmetic)
+    many = p.process(vols)
+    for s in (0, slices - 1):
+        one = p.process(vols[s])
+        assert np.array_equal(one, many[s]), np.abs(one - many[s]).max()
+    p.close()

@@ -15,8 +15,8 @@
  * once per tile instead of once per ray.
  *
  * When there are too few tiles to fill the GPU (one slice, few angles), a
- * tile's detectors are split over several CTAs. Each then stages only a
- * window of each chunk's rows: the columns its rays can reach, bounded by
+ * tile's detectors are split over up to 8 CTAs, with whole rows while a part
+ * keeps at most 8 warps. Else each stages only a window of each chunk's rows: the columns its rays can reach, bounded by
  * the extreme rays of its angles (the coordinate is monotone in detector and
  * row), one 1-D copy per row, with two zero slots after the window for taps
  * outside it (they lie outside the image). 2900^2 x 90 angles: 925 -> 818 us.
@@ -878,9 +878,33 @@ extern "C" int udev_fp_default_cfg(udev *d, const udev_geom *g, int n_tiles, int
         }
         return UFOIR_OK;
     }
-    /* Fewer tiles than a quarter of the SMs (one slice, few angles): up to 8
-     * CTAs per tile, with chunks small enough for two CTAs per SM, and each
-     * CTA stages only the window of columns its rays can reach (the detector
+    /* Fewer tiles than a quarter of the SMs (one slice, few angles). A CTA's
+     * time is its rows', and a row's grows with the CTA's warps: about 100 ns
+     * with 3 or 4 warps of one detector pair per slot, 135 with 5 to 8, 175
+     * with 12. So up to 8 parts of at least 64 detectors with whole rows, one
+     * pair per slot, where that leaves at most 8 warps: a windowed part (below)
+     * takes 160 ns a row, most of it waiting for its row copies. At most two
+     * thirds of the SMs get a CTA: with nearly all of them, 600 to 1448 columns
+     * went 20 to 50 % slower. us, windows -> whole rows: 256^2 x 60 43 -> 31,
+     * 367^2 x 90 57 -> 40, 530^2 x 24 90 -> 54, 724^2 x 90 104 -> 70, 900^2 x
+     * 90 143 -> 86, 1448^2 x 90 247 -> 192. */
+    if (cfg.A == 8) {
+        int parts = (int) (2LL * sms / (3 * ctas));
+        parts = parts > 8 ? 8 : parts;
+        parts = parts > n / 64 ? n / 64 : parts;
+        if (parts > 1 && fp_threads(n, parts, 1) <= 256) {
+            udev_fp_cfg w = *c;
+            w.J = 1;
+            w.dsplit = parts;
+            for (w.K = 32; w.K >= 8; w.K /= 2)
+                if (udev_fp_cfg_finish(d, g, tile_spread, &w) == UFOIR_OK) {
+                    *c = w;
+                    return UFOIR_OK;
+                }
+        }
+    }
+    /* Else up to 8 CTAs per tile, with chunks small enough for two CTAs per
+     * SM, and each CTA stages only the window of columns its rays can reach (the detector
      * range times max |det_step| = sqrt 2, the chunk's rows times max |step|
      * = 1, the spread of the tile's angles, and a margin), unless that is the
      * whole row. One slice of 2900^2 x 90: 0.639 ms, against 1.30 in two whole-row
