@@ -16,10 +16,11 @@
  *
  * When there are too few tiles to fill the GPU (one slice, few angles), a
  * tile's detectors are split over up to 8 CTAs, with whole rows while a part
- * keeps at most 8 warps. Else each stages only a window of each chunk's rows: the columns its rays can reach, bounded by
- * the extreme rays of its angles (the coordinate is monotone in detector and
- * row), one 1-D copy per row, with two zero slots after the window for taps
- * outside it (they lie outside the image). 2900^2 x 90 angles: 925 -> 818 us.
+ * keeps at most 8 warps. Else each stages only a window of each chunk's rows:
+ * the columns its rays can reach, bounded by the extreme rays of its angles
+ * (the coordinate is monotone in detector and row), one 1-D copy per row, with
+ * two zero slots after the window for taps outside it (they lie outside the
+ * image). 2900^2 x 90 angles: 925 -> 818 us when that came.
  *
  * Bound by the FMA pipe and, at one CTA per SM, by the barrier at each chunk.
  * 16 slices of 1448^2 x 1200: 13.03 -> 11.72 ms, two of 2900^2 x 360 3.53 ->
