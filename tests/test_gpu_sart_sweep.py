@@ -52,3 +52,20 @@ def test_sweep_passes_non_finite_values_on(ufoir_lib, gpu_ctx, monkeypatch, n, n
     want, _ = _sart(ufoir_lib, gpu_ctx, sinos, -1.0, 1)
     assert not np.isfinite(want).all()
     assert np.array_equal(got, want, equal_nan=True)
+
+
+# Geometries where a column part has no rays at some angles (the last block's
+# centre lies past the image, or the axis beside the image's centre): such a CTA
+# sends no sums, and must keep up with the others all the same.
+@pytest.mark.parametrize("n,na,axis,slices", [
+    (129, 24, -1.0, 20), (200, 31, 97.4, 12), (257, 90, -1.0, 1), (262, 90, -1.0, 3), (277, 90, -1.0, 1),
+    (256, 60, 168.0, 1), (256, 60, 208.0, 2), (367, 60, 263.5, 1)])
+def test_sweep_with_parts_that_have_no_rays(ufoir_lib, gpu_ctx, monkeypatch, n, na, axis, slices):
+    rng = np.random.default_rng(3 * n + na)
+    sinos = rng.random((slices, na, n), dtype=np.float32) * n
+    monkeypatch.delenv("UFOIR_SART_KERNELS", raising=False)
+    got, few = _sart(ufoir_lib, gpu_ctx, sinos, axis, 25)
+    monkeypatch.setenv("UFOIR_SART_KERNELS", "general")
+    want, many = _sart(ufoir_lib, gpu_ctx, sinos, axis, 25)
+    assert few < many / 4, (few, many)        # the sweep served
+    assert np.array_equal(got, want), np.abs(got - want).max()
