@@ -111,6 +111,11 @@ UFOIR_API int ufoir_ctx_timer_begin(ufoir_ctx *ctx);
  * copies (all of which land), writes nothing and records the timeout, and the
  * call returns UFOIR_ERR_TIMEOUT; the context stays usable. One-shot. */
 UFOIR_API int ufoir_ctx_inject_copy_timeout(ufoir_ctx *ctx, int chunk);
+/* The same for the SART sweep kernel's exchange of block sums: in the next
+ * sweep that holds angle `angle` (-1 cancels), the barrier of one CTA expects
+ * 16 bytes more than the sums bring; its waits and then those of the CTAs that
+ * wait for it run out. One-shot: the next launch, or the one captured next. */
+UFOIR_API int ufoir_ctx_inject_exchange_timeout(ufoir_ctx *ctx, int angle);
 UFOIR_API int ufoir_ctx_timer_end(ufoir_ctx *ctx, float *ms);
 
 /* ------------------------------------------------------------------------ */

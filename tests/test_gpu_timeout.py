@@ -52,3 +52,36 @@ def test_inject_copy_timeout_argument_checks(ufoir_lib, gpu_ctx):
     assert L.ufoir_ctx_inject_copy_timeout(gpu_ctx.handle, -2) == ufoir_lib.ERR_INVALID
     assert L.ufoir_ctx_inject_copy_timeout(gpu_ctx.handle, 5) == ufoir_lib.OK
     assert L.ufoir_ctx_inject_copy_timeout(gpu_ctx.handle, -1) == ufoir_lib.OK    # cancelled
+
+
+# The SART sweep's exchange of block sums between the CTAs of a cluster: one
+# CTA's barrier never completes, so its wait runs out and then those of the CTAs
+# that wait for its next arrival. One CTA (n = 60) and several; the first angle,
+# one within a run and the last of one.
+@pytest.mark.parametrize("n,angle", [(60, 0), (60, 7), (200, 0), (200, 3), (200, 7), (257, 30)])
+def test_sart_exchange_timeout_is_reported_and_context_recovers(ufoir_lib, gpu_ctx, oracle, n, angle):
+    na = 31
+    step = np.float32(np.pi / na)
+    sino = np.random.default_rng(n + angle).random((na, n), dtype=np.float32) * n
+    p = ufoir_lib.ParallelProjector(gpu_ctx, step=float(step), is_forward=0)
+    want = oracle.sart(oracle.projector(n, na, step), sino, 1, 0.5)
+    assert np.array_equal(ufoir_lib.sart(p, sino, num_iterations=1, relaxation_factor=0.5), want)
+
+    assert ufoir_lib.lib().ufoir_ctx_inject_exchange_timeout(gpu_ctx.handle, angle) == ufoir_lib.OK
+    t0 = time.perf_counter()
+    with pytest.raises(ufoir_lib.UfoirError) as e:
+        ufoir_lib.sart(p, sino, num_iterations=1, relaxation_factor=0.5)
+    elapsed = time.perf_counter() - t0
+    assert e.value.status == ufoir_lib.ERR_TIMEOUT, str(e.value)
+    assert 0.2 < elapsed < 10.0, elapsed
+
+    assert np.array_equal(ufoir_lib.sart(p, sino, num_iterations=1, relaxation_factor=0.5), want)
+    p.close()
+
+
+def test_inject_exchange_timeout_argument_checks(ufoir_lib, gpu_ctx):
+    L = ufoir_lib.lib()
+    assert L.ufoir_ctx_inject_exchange_timeout(None, 0) == ufoir_lib.ERR_INVALID
+    assert L.ufoir_ctx_inject_exchange_timeout(gpu_ctx.handle, -2) == ufoir_lib.ERR_INVALID
+    assert L.ufoir_ctx_inject_exchange_timeout(gpu_ctx.handle, 5) == ufoir_lib.OK
+    assert L.ufoir_ctx_inject_exchange_timeout(gpu_ctx.handle, -1) == ufoir_lib.OK    # cancelled

@@ -110,6 +110,14 @@ int ufoir_ctx_inject_copy_timeout(ufoir_ctx *ctx, int chunk)
     return UFOIR_OK;
 }
 
+int ufoir_ctx_inject_exchange_timeout(ufoir_ctx *ctx, int angle)
+{
+    if (!ctx || angle < -1)
+        return UFOIR_ERR_INVALID;
+    udev_inject_exchange_skip(ctx->dev, angle);
+    return UFOIR_OK;
+}
+
 int ufoir_ctx_timer_begin(ufoir_ctx *ctx)
 {
     if (!ctx)

@@ -208,6 +208,9 @@ int udev_take_kernel_error(udev *d);
 /* Testing: in the next tiled forward projection launch, the barrier of row
  * chunk `chunk` never completes in any CTA (-1 = none). */
 void udev_inject_copy_skip(udev *d, int chunk);
+/* Testing: in the next SART sweep that holds `angle`, one CTA's barrier of that
+ * angle never completes (-1 = none). */
+void udev_inject_exchange_skip(udev *d, int angle);
 
 /* The "siddon" model (udev_siddon.cu): exact line integrals of the pixel
  * image, bin k of angle theta being the line X cos - Y sin + axis = k + 0.5.

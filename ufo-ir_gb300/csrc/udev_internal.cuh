@@ -29,6 +29,7 @@ struct udev {
     int *h_err = nullptr;           /* kernel error word (bounded-wait timeouts), mapped host memory */
     int *d_err = nullptr;           /* the same as kernels address it */
     int inject_skip_chunk = -1;     /* testing: see udev_inject_copy_skip */
+    int inject_skip_angle = -1;     /* testing: see udev_inject_exchange_skip */
     int sart_wide_clusters = 0;     /* 16-CTA clusters of the segment-form SART FP that fit at once */
     cudaStream_t side = nullptr;    /* side copies (udev_copy_after), created on first use */
     cudaEvent_t side_go = nullptr;  /* current stream -> side stream ordering */

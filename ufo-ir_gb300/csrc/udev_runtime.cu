@@ -402,6 +402,11 @@ void udev_inject_copy_skip(udev *d, int chunk)
     d->inject_skip_chunk = chunk < 0 ? -1 : chunk;
 }
 
+void udev_inject_exchange_skip(udev *d, int angle)
+{
+    d->inject_skip_angle = angle < 0 ? -1 : angle;
+}
+
 int udev_timer_begin(udev *d)
 {
     UDEV_BIND(d);

@@ -59,6 +59,7 @@ struct SweepArgs {
     float relax;
     float neg_zero;
     const float *relax_dev;
+    int skip_angle;            /* testing: angle whose exchange never completes (-1 = none) */
     int *err;
     long long vol_stride;
     long long sino_stride;
@@ -109,6 +110,12 @@ __device__ __forceinline__ bool wait_cluster(uint64_t *bar, uint32_t parity, int
         }
     }
     return true;
+}
+
+/* Bytes that rank 0's barrier of angle `a` expects beyond the sums (testing). */
+__device__ __forceinline__ uint32_t skip_bytes(const SweepArgs &P, int rank, int a)
+{
+    return rank == 0 && a == P.skip_angle ? 16u : 0u;
 }
 
 /* The rays that part `part` projects: those whose coordinate m0 + s * det_step
@@ -346,7 +353,7 @@ __global__ void __launch_bounds__(kThreads, 1) sart_sweep_kernel(SweepArgs P)
     if (tid == 0) {
         for (int k = 0; k < 2; ++k) {
             tma::mbar_init(&bars[k], 1);
-            tma::mbar_arrive_expect_tx(&bars[k], sum_bytes);
+            tma::mbar_arrive_expect_tx(&bars[k], sum_bytes + skip_bytes(P, rank, P.first + k));
         }
         tma::fence_mbar_init();
     }
@@ -448,10 +455,11 @@ __global__ void __launch_bounds__(kThreads, 1) sart_sweep_kernel(SweepArgs P)
                     pair_sync(pair);
             }
         }
-        if (ok)
-            ok = wait_cluster(&bars[par], (uint32_t) ((a - P.first) >> 1) & 1, P.err);
-        if (tid == 0 && a + 2 < P.end)      /* before any CTA can send that angle's sums */
-            tma::mbar_arrive_expect_tx(&bars[par], sum_bytes);
+        ok = wait_cluster(&bars[par], (uint32_t) ((a - P.first) >> 1) & 1, P.err);
+        /* before any CTA can send that angle's sums; never after a wait that ran
+         * out, whose phase has no arrival left to take */
+        if (ok && tid == 0 && a + 2 < P.end)
+            tma::mbar_arrive_expect_tx(&bars[par], sum_bytes + skip_bytes(P, rank, a + 2));
 #pragma unroll
         for (int k = 0; k < kPerThread; ++k) {
             const int s = tid + k * kThreads;
@@ -475,7 +483,10 @@ __global__ void __launch_bounds__(kThreads, 1) sart_sweep_kernel(SweepArgs P)
                 rs[kResidPad + s] = result;
             }
         }
-        __syncthreads();
+        /* a wait ran out: this CTA leaves the angles, the others at their next wait */
+        ok = __syncthreads_and(ok) != 0;
+        if (!ok)
+            break;
         /* tile += relax * (0 + sample): rows warp + 16 m, pairs (m, m + 1) */
         {
             const float sn = rays_s[par].sn, cs = rays_s[par].cs;
@@ -490,10 +501,14 @@ __global__ void __launch_bounds__(kThreads, 1) sart_sweep_kernel(SweepArgs P)
         }
     }
     bp::cp_async_wait<0>();
-    /* every CTA has read its halo (before the first cluster barrier); no CTA
-     * leaves while another's wait may have run out with stores to it in flight */
+    /* every CTA has read its halo (before the first cluster barrier). No CTA
+     * leaves before all are here: the stores to a CTA whose wait ran out were
+     * sent before their senders' last waits, so that limit has passed since,
+     * or this one's has. */
     __syncwarp();
     cluster_sync_all();
+    if (!ok)
+        return;     /* this CTA's part of the image stays as it was */
     if (T) {
         for (int i = c_lo + (tid >> 6); i < c_hi; i += kThreads / 64)
             if ((tid & 63) < rows)
@@ -651,6 +666,11 @@ extern "C" int udev_sart_sweep(udev *d, const udev_geom *g, int first, int end, 
     A.relax = relax;
     A.neg_zero = -0.0f;
     A.relax_dev = relax_dev;
+    A.skip_angle = -1;
+    if (d->inject_skip_angle >= first && d->inject_skip_angle < end) {     /* one-shot test injection */
+        A.skip_angle = d->inject_skip_angle;
+        d->inject_skip_angle = -1;
+    }
     A.err = d->d_err;
     A.vol_stride = (long long) n * n;
     A.sino_stride = (long long) g->n_angles * n;

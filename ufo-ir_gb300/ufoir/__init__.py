@@ -161,6 +161,7 @@ EXPORTED = (
     "ufoir_graph_job_desc", "ufoir_graph_run", "ufoir_io_last_error", "ufoir_io_tiff_info", "ufoir_io_read_tiff",
     "ufoir_io_write_tiff", "ufoir_io_read_raw", "ufoir_io_write_raw", "ufoir_sample_ceiling", "ufoir_sample_ceiling_bp",
     "ufoir_asdpocs_process_ex", "ufoir_tv_gradient", "ufoir_ctx_inject_copy_timeout",
+    "ufoir_ctx_inject_exchange_timeout",
     "ufoir_ctx_set_autotune", "ufoir_projector_autotune", "ufoir_batch_create", "ufoir_batch_run",
     "ufoir_batch_set_active", "ufoir_batch_launches", "ufoir_batch_destroy", "ufoir_ctx_sm_count",
 )
@@ -260,6 +261,7 @@ def _declare(L):
                                            C.POINTER(AsdpocsScalars)]
     L.ufoir_tv_gradient.argtypes = [vp, vp, C.c_size_t, C.c_size_t, C.c_size_t, vp]
     L.ufoir_ctx_inject_copy_timeout.argtypes = [vp, C.c_int]
+    L.ufoir_ctx_inject_exchange_timeout.argtypes = [vp, C.c_int]
     L.ufoir_ctx_set_autotune.argtypes = [vp, C.c_int]
     L.ufoir_ctx_sm_count.argtypes = [vp]
     L.ufoir_projector_autotune.argtypes = [vp, C.c_size_t, C.POINTER(FpTuning)]
