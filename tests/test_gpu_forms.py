@@ -192,3 +192,37 @@ def test_few_tiles_give_what_many_give(ufoir_lib, gpu_ctx, n, na, axis, arithmet
         one = p.process(vols[s])
         assert np.array_equal(one, many[s]), np.abs(one - many[s]).max()
     p.close()
+
+
+# A warp's detectors may span the whole image: at a row one end ray lies left of
+# it, the other right of it, and the rays between cross it. With the axis beside
+# the centre that happens in whole chunks of rows. The siddon model's tiles are
+# compared with its ray walk: two orders of n float roundings (an axis at half a
+# bin puts rays on pixel boundaries, which the two put on the same side).
+@pytest.mark.parametrize("n,na,axis", [(33, 720, 6.6), (34, 720, 25.5), (34, 720, 5.1), (35, 360, 26.25), (36, 720, 27.0)])
+def test_rows_between_rays_on_either_side_of_the_image(ufoir_lib, gpu_ctx, n, na, axis):
+    step = f32(np.pi / na)
+    vol = np.random.default_rng(n).random((n, n), dtype=f32)
+    kw = dict(step=float(step), is_forward=1, axis_position=axis, angles_num=na)
+    p = ufoir_lib.ParallelProjector(gpu_ctx, **kw)
+    np.testing.assert_array_equal(p.process(vol), _forward(vol, na, step, axis))
+    p.close()
+    p = ufoir_lib.ParallelProjector(gpu_ctx, model="siddon", **kw)
+    whole, part = p.process(vol), np.zeros((na, n), f32)
+    for off, cnt, direction in p.subsets():
+        p.subset_fp(vol, part, off, cnt, direction)
+    np.testing.assert_allclose(whole, part, rtol=0, atol=2 * n * 2.0 ** -24 * float(np.abs(part).max()))
+    p.close()
+
+
+# The tuner also tries shapes with more detectors per warp, which span larger images.
+@pytest.mark.parametrize("n,na,axis", [(96, 60, 70.0), (256, 24, 184.3), (300, 40, 90.2)])
+def test_tuned_shapes_off_centre(ufoir_lib, n, na, axis):
+    step = f32(np.pi / na)
+    vol = np.random.default_rng(n).random((n, n), dtype=f32)
+    with ufoir_lib.Context(0) as ctx:
+        p = ufoir_lib.ParallelProjector(ctx, step=float(step), is_forward=1, axis_position=axis, angles_num=na)
+        p.get_requisition((n, n))
+        p.autotune(1)
+        np.testing.assert_array_equal(p.process(vol), _forward(vol, na, step, axis))
+        p.close()

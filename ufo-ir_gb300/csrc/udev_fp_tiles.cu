@@ -89,14 +89,18 @@ constexpr size_t kBatchStatic = (sizeof(FpTileArgs) + 16 + 127) / 128 * 128;
 
 constexpr int kMaxWinThreads = 448;   /* detector-split CTAs hold at most half the slots */
 
-/* Rows of a ray with coordinate c + r st (r in [0, n)) inside [lo, hi): an
- * inner bound [a, b) where `inner`, else an outer one. An empty set gives
- * a = n, b = 0. */
-__device__ __forceinline__ void ray_rows(float c, float st, float lo, float hi, int n, bool inner, int &a, int &b)
+/* Rows r in [0, n) with cl + r st >= lo and ch + r st < hi: an inner bound
+ * [a, b) where `inner`, else an outer one. An empty set gives a = n, b = 0.
+ * With cl = ch = c the rows of a ray inside [lo, hi); with cl >= ch the ends of
+ * a span of rays, the rows that any ray between them may have inside (where all
+ * of them lie beyond one edge, and not one end beyond either). */
+__device__ __forceinline__ void ray_rows(float cl, float ch, float st, float lo, float hi, int n, bool inner, int &a,
+                                         int &b)
 {
     a = n;
     b = 0;
-    if (!(fabsf(c) < 1e9f) || !(fabsf(st) < 1e9f)) {   /* no geometry: never inside, never outside */
+    /* no geometry: never inside, never outside */
+    if (!(fabsf(cl) < 1e9f) || !(fabsf(ch) < 1e9f) || !(fabsf(st) < 1e9f)) {
         if (!inner) {
             a = 0;
             b = n;
@@ -104,14 +108,14 @@ __device__ __forceinline__ void ray_rows(float c, float st, float lo, float hi, 
         return;
     }
     if (fabsf(st) < 1e-6f) {       /* moves less than 0.01 column over the image */
-        if (c >= lo && c < hi) {
+        if (cl >= lo && ch < hi) {
             a = 0;
             b = n;
         }
         return;
     }
     const float inv = __fdividef(1.0f, st), fn = (float) n;
-    const float x = (lo - c) * inv, y = (hi - c) * inv;
+    const float x = (lo - cl) * inv, y = (hi - ch) * inv;
     const float x0 = fminf(fmaxf(fminf(x, y), -4.0f), fn + 4.0f), x1 = fminf(fmaxf(fmaxf(x, y), -4.0f), fn + 4.0f);
     if (x1 < -2.0f || x0 > fn + 2.0f)
         return;
@@ -324,8 +328,8 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
      *  - [rin0, rin1): every ray's coordinate lies in [0.5, n + 1.5), so
      *    floor(c - 0.5) takes the three-operation form (floor_half2) and the
      *    tap address is one multiply-add on its bits, with no clamp;
-     *  - before rout0 and from rout1 on: every coordinate is below -0.5 or at
-     *    least n + 0.5, where both taps are border zeros. Only the recurrence
+     *  - before rout0 and from rout1 on: an angle's coordinates are all below
+     *    -0.5 or all at least n + 0.5, where both taps are border zeros. Only the recurrence
      *    advances: adding +-0 leaves a block sum unchanged (it starts at +0
      *    and a sum of finite floats in round-to-nearest is never -0);
      *  - the rows between take the general form. */
@@ -341,8 +345,11 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
         const float cc = fmaf(0.5f + kc.ros + (float) s - 0.5f * (float) n, dir == 0 ? -inv : inv,
                               fmaf(-kc.os, st, 0.5f * (float) n)) +
                          (SID ? 0.5f + fminf(st, 0.0f) : 0.0f);
-        ray_rows(cc, st, 0.5f + P.drift, (float) n + 1.5f - P.drift, n, true, rin0, rin1);
-        ray_rows(cc, st, -0.5f - P.drift, (float) n + 0.5f + P.drift, n, false, rout0, rout1);
+        ray_rows(cc, cc, st, 0.5f + P.drift, (float) n + 1.5f - P.drift, n, true, rin0, rin1);
+        /* the other end's: rays between an end left of the image and one right
+         * of it cross the image (a warp's 32 J detectors can span all of it) */
+        const float cd = __shfl_xor_sync(0xffffffffu, cc, A);
+        ray_rows(fmaxf(cc, cd), fminf(cc, cd), st, -0.5f - P.drift, (float) n + 0.5f + P.drift, n, false, rout0, rout1);
         rin0 = __reduce_max_sync(0xffffffffu, rin0);
         rin1 = __reduce_min_sync(0xffffffffu, rin1);
         rout0 = __reduce_min_sync(0xffffffffu, rout0);
