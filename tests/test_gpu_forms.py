@@ -226,3 +226,66 @@ def test_tuned_shapes_off_centre(ufoir_lib, n, na, axis):
         p.autotune(1)
         np.testing.assert_array_equal(p.process(vol), _forward(vol, na, step, axis))
         p.close()
+
+
+def _fma(a, b, c):
+    """float32 a * b + c with one rounding: the product is exact in 64 bits, the
+    sum is rounded to odd there, which the second rounding cannot tell from exact."""
+    p, c = a.astype(np.float64) * b.astype(np.float64), c.astype(np.float64)
+    s = p + c
+    bb = s - p
+    err = (p - (s - bb)) + (c - bb)
+    bits = s.view(np.int64)
+    odd = np.where((err != 0) & (bits & 1 == 0), np.where((err > 0) == (s > 0), 1, -1), 0)
+    return (bits + odd).view(np.float64).astype(f32)
+
+
+def _backward_fast(sino, step, axis):
+    """_backward in the fast arithmetic: coordinates fX cos + ((-fY) sin + shift), samples (sum + T0) + t (T1 - T0)."""
+    na, n = sino.shape
+    sn, cs = _lut(na, step)
+    w, ax = f32(n), f32(axis)
+    diff = w - ax * f32(2)
+    half = w - ax if diff < 0 else ax
+    e0, e1 = ax - half + f32(0.5), ax + half - f32(0.5)
+    shift = w / f32(2) - diff / f32(2)
+    f = np.arange(n, dtype=f32) + f32(0.5) - w / f32(2)
+    v, total = np.zeros((n, n), f32), np.zeros((n, n), f32)
+    vertical = np.abs(sn.astype(np.float64)) <= np.abs(cs.astype(np.float64))
+    for a in range(na):
+        if a and vertical[a] != vertical[a - 1]:
+            v, total = v + total, np.zeros((n, n), f32)
+        c = np.minimum(np.maximum(f[None, :] * cs[a] + ((-f[:, None]) * sn[a] + shift), e0), e1) - f32(0.5)
+        k = np.floor(c)
+        row = np.append(sino[a], f32(0))
+        t0, t1 = row[k.astype(np.int64)], row[k.astype(np.int64) + 1]
+        total = _fma(c - k, t1 - t0, total + t0)
+    return v + total
+
+
+# At a quarter turn the last row of a centred image has its coordinates on the
+# detector edge, or an ulp beside it, as the sum is ordered. Values in the first
+# and last detector show which. All four launch shapes (slices).
+@pytest.mark.parametrize("n,na,slices,axis", [(200, 20, 1, 100.0), (200, 20, 12, 100.0), (256, 60, 1, 128.0), (256, 60, 90, 128.0),
+                                              (512, 16, 1, 256.0), (512, 16, 80, 256.0), (129, 37, 12, 60.3)])
+def test_fast_backprojector_at_the_detector_edges(ufoir_lib, gpu_ctx, n, na, slices, axis):
+    step = f32(np.pi / na)
+    sino = np.random.default_rng(n).standard_normal((slices, na, n)).astype(f32)
+    sino[:, :, [0, n - 1]] += f32(4)
+    p = ufoir_lib.ParallelProjector(gpu_ctx, step=float(step), is_forward=0, axis_position=axis, angles_num=na,
+                                    arithmetic=ufoir_lib.ARITH_FAST)
+    got = p.process(sino)
+    p.close()
+    for s in sorted({0, slices - 1}):
+        np.testing.assert_array_equal(got[s], _backward_fast(sino[s], step, axis))
+
+
+@pytest.mark.parametrize("n,na", [(256, 60), (512, 400), (1024, 360)])
+def test_fast_and_exact_backprojections_of_ones_agree(ufoir_lib, gpu_ctx, n, na):
+    step = f32(np.pi / na)
+    out = []
+    for arithmetic in (ufoir_lib.ARITH_FAST, ufoir_lib.ARITH_EXACT):
+        p = ufoir_lib.ParallelProjector(gpu_ctx, step=float(step), is_forward=0, angles_num=na, arithmetic=arithmetic)
+        out.append(p.process(np.ones((na, n), f32)).astype(np.float64))
+        p.close()
+    assert np.linalg.norm(out[0] - out[1]) <= 1e-5 * np.linalg.norm(out[1])      # the path's bar

@@ -105,9 +105,13 @@ __device__ __forceinline__ int angle_of(const BpTileArgs &P, int vi)
     return 0;
 }
 
-/* Detector coordinate of pixel (x, y) for one angle, exactly as the reference. */
+/* Detector coordinate of pixel (x, y) for one angle, exactly as the reference,
+ * or with FM as the fast arithmetic sums it (sample_angles). */
+template <bool FM>
 __device__ __forceinline__ float det_coord(float fX, float fY, float cs, float sn, float shift)
 {
+    if (FM)
+        return __fadd_rn(__fmul_rn(fX, cs), __fadd_rn(__fmul_rn(-fY, sn), shift));
     return __fadd_rn(__fsub_rn(__fmul_rn(fX, cs), __fmul_rn(fY, sn)), shift);
 }
 
@@ -118,10 +122,12 @@ __device__ __forceinline__ float det_coord(float fX, float fY, float cs, float s
  * that cross the ends of the detector row go element by element, with zeros
  * outside [0, n). A warp copies whole windows (lane = group of 4).
  *
- * The coordinate is monotone in each pixel index (every rounding step is), so
- * over the tile it lies between its values at the corners.
+ * The coordinate is monotone in each pixel index (every rounding step is, in
+ * either order of the sum), so over the tile it lies between its values at the
+ * corners, summed in the order of the samples: a tile decided inside by another
+ * order can hold coordinates an ulp below the edge.
  */
-template <class T>
+template <class T, bool FM>
 __device__ void load_chunk(const BpTileArgs &P, BpSmem<T> &S, int buf, int chunk, const float *sino, int x0, int y0,
                            const joseph::AxisConsts &k, float e0, float e1, float shift)
 {
@@ -137,8 +143,8 @@ __device__ void load_chunk(const BpTileArgs &P, BpSmem<T> &S, int buf, int chunk
             const float fx1 = __fsub_rn(__fadd_rn((float) (x0 + T::TileX - 1), 0.5f), k.os);
             const float fy0 = __fsub_rn(__fadd_rn((float) y0, 0.5f), k.os);
             const float fy1 = __fsub_rn(__fadd_rn((float) (y0 + T::TileY - 1), 0.5f), k.os);
-            const float c00 = det_coord(fx0, fy0, cs, sn, shift), c10 = det_coord(fx1, fy0, cs, sn, shift);
-            const float c01 = det_coord(fx0, fy1, cs, sn, shift), c11 = det_coord(fx1, fy1, cs, sn, shift);
+            const float c00 = det_coord<FM>(fx0, fy0, cs, sn, shift), c10 = det_coord<FM>(fx1, fy0, cs, sn, shift);
+            const float c01 = det_coord<FM>(fx0, fy1, cs, sn, shift), c11 = det_coord<FM>(fx1, fy1, cs, sn, shift);
             const float lo = fminf(fminf(c00, c10), fminf(c01, c11));
             const float hi = fmaxf(fmaxf(c00, c10), fmaxf(c01, c11));
             in = lo >= e0 && hi <= e1;
@@ -315,13 +321,13 @@ __device__ __forceinline__ void bp_tile(const BpTileArgs &P, BpSmem<T> &S, int t
     int sub = 0;
     int sub_end = P.n_subsets > 0 ? (int) P.sub_n[0] : 0;
     if (nchunks > 0) {
-        load_chunk<T>(P, S, 0, 0, sino, x0, y0, k, e0, e1, shift);
+        load_chunk<T, FM>(P, S, 0, 0, sino, x0, y0, k, e0, e1, shift);
         cp_async_commit();
     }
     for (int ch = 0; ch < nchunks; ++ch) {
         const int buf = ch & 1;
         if (ch + 1 < nchunks) {
-            load_chunk<T>(P, S, buf ^ 1, ch + 1, sino, x0, y0, k, e0, e1, shift);
+            load_chunk<T, FM>(P, S, buf ^ 1, ch + 1, sino, x0, y0, k, e0, e1, shift);
             cp_async_commit();
             cp_async_wait<1>();
         } else {
