@@ -79,3 +79,18 @@ def test_tv_step_takes_the_norm_of_its_gradient(ufoir_lib, gpu_ctx, n, slices):
             factor = dtgv / np.float32(np.abs(g.astype(np.float64)).sum())
             x = x - factor * g
         assert np.array_equal(x_tv[s], x), np.abs(x_tv[s] - x).max()
+
+
+@pytest.mark.parametrize("n,slices", [(65, 9), (367, 5), (530, 7), (1200, 2)])
+def test_a_slice_of_a_stack_has_its_own_norms(ufoir_lib, gpu_ctx, n, slices):
+    """ASD-POCS (FP64 norms): a slice's steps do not depend on the stack it is in."""
+    na = 12
+    sinos = np.random.default_rng(n).random((slices, na, n), dtype=np.float32) * n
+    p = ufoir_lib.ParallelProjector(gpu_ctx, step=float(np.float32(np.pi / na)), is_forward=False)
+    kw = dict(num_iterations=2, df_minimizer=dict(num_iterations=1, relaxation_factor=0.5))
+    vol, x_tv, scalars = ufoir_lib.asdpocs_state(p, sinos, **kw)
+    for s in (0, slices - 1):
+        one = ufoir_lib.asdpocs_state(p, sinos[s], **kw)
+        assert np.array_equal(one[0], vol[s]) and np.array_equal(one[1], x_tv[s])
+        assert one[2][0] == scalars[s]
+    p.close()

@@ -145,8 +145,12 @@ __device__ __forceinline__ double block_sum_double(double v)
  * (17, 21) here. */
 constexpr int kGradTile = 32;
 constexpr int kGradRows = kGradTile / 8;
-constexpr int kGradCtas = 8;          /* per SM */
-constexpr int kGradBlocks = 2048;     /* per slice: as many as the reduction scratch holds */
+/* CTAs and partial sums per slice at most: what 152 SMs run at once (the
+ * reduction scratch holds 2048). Not by the number of slices or of SMs, as the
+ * sum's grouping follows it and a slice is to have one norm in any stack.
+ * (Gradient calls of 4 x 724^2 35 -> 31 us and 3 x 2900^2 212 -> 150 against
+ * 1216 CTAs shared among the slices.) */
+constexpr int kGradBlocks = 1216;
 
 template <bool NORM>
 __global__ void __launch_bounds__(256) l1_grad_kernel(const float *in, float *out, int w, int h, long long stride,
@@ -431,14 +435,11 @@ extern "C" int udev_unary(udev *d, int op, const float *a, float m, float m2, fl
     return udev_after_launch(d, "unary_kernel");
 }
 
-/* CTAs per slice for the gradient: all that run at once, as far as there are tiles. */
-static unsigned int grad_blocks(udev *d, int w, int h, int n_slices)
+/* CTAs per slice for the gradient. */
+static unsigned int grad_blocks(int w, int h)
 {
     const long long tiles = (long long) udev_div_up(w, kGradTile) * udev_div_up(h, kGradTile);
-    long long blocks = ((long long) d->sm_count * kGradCtas + n_slices - 1) / n_slices;
-    if (blocks > kGradBlocks)
-        blocks = kGradBlocks;
-    return (unsigned int) (tiles < blocks ? tiles : blocks);
+    return (unsigned int) (tiles < kGradBlocks ? tiles : kGradBlocks);
 }
 
 extern "C" int udev_l1_grad(udev *d, const float *in, float *out, int w, int h, int n_slices)
@@ -446,7 +447,7 @@ extern "C" int udev_l1_grad(udev *d, const float *in, float *out, int w, int h, 
     if (n_slices <= 0)
         return UFOIR_OK;
     UDEV_BIND(d);
-    const dim3 grid(grad_blocks(d, w, h, n_slices), (unsigned int) n_slices);
+    const dim3 grid(grad_blocks(w, h), (unsigned int) n_slices);
     l1_grad_kernel<false><<<grid, dim3(32, 8), 0, d->stream>>>(in, out, w, h, (long long) w * h, nullptr);
     return udev_after_launch(d, "l1_grad_kernel");
 }
@@ -463,7 +464,7 @@ extern "C" int udev_l1_grad_norm(udev *d, const float *in, float *out, int w, in
         return udev_l1_norm_to(d, out, (size_t) w, (size_t) h, n_slices, mode, partials, d_out);
     }
     UDEV_BIND(d);
-    const dim3 grid(grad_blocks(d, w, h, n_slices), (unsigned int) n_slices);
+    const dim3 grid(grad_blocks(w, h), (unsigned int) n_slices);
     l1_grad_kernel<true><<<grid, dim3(32, 8), 0, d->stream>>>(in, out, w, h, (long long) w * h, partials);
     if ((rc = udev_after_launch(d, "l1_grad_kernel")))
         return rc;
