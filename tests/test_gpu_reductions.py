@@ -94,3 +94,22 @@ def test_a_slice_of_a_stack_has_its_own_norms(ufoir_lib, gpu_ctx, n, slices):
         assert np.array_equal(one[0], vol[s]) and np.array_equal(one[1], x_tv[s])
         assert one[2][0] == scalars[s]
     p.close()
+
+
+# Short slices are added by one thread, longer ones in chunks of 512 elements or
+# more, 512 of them at most: counts on and beside those lines.
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("count", [15, 17, 1023, 1024, 1025, 2048, 8191, 8192, 8193, 8703, 8704, 8705, 262143, 262144, 262657])
+def test_compat_l1_norm_of_short_and_chunked_slices(ufoir_lib, gpu_ctx, count, kind):
+    x = _values(kind, count).reshape(1, count)
+    with np.errstate(over="ignore", invalid="ignore"):
+        want = np.cumsum(np.abs(x).reshape(-1), dtype=np.float32)[-1]
+    np.testing.assert_array_equal(np.float32(gpu_ctx.l1_norm(x, ufoir_lib.NORM_COMPAT)), want)
+
+
+@pytest.mark.parametrize("count,kernels", [(1, 1), (8192, 1), (8193, 3)])
+def test_compat_l1_norm_of_a_short_slice_is_one_kernel(ufoir_lib, gpu_ctx, count, kernels):
+    x = np.ones((1, count), np.float32)
+    before = gpu_ctx.kernel_launches()
+    assert gpu_ctx.l1_norm(x, ufoir_lib.NORM_COMPAT) == count
+    assert gpu_ctx.kernel_launches() - before == kernels

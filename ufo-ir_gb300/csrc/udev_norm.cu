@@ -12,8 +12,8 @@
  * binade. What is left of the chain is the places where the sum reaches the
  * next binade, a few dozen at most: m would pass 2^24 there.
  *
- *  1. l1_sums_kernel: float sums of 512 chunks (a prediction of where each
- *     chunk starts, and whether it holds a NaN);
+ *  1. l1_sums_kernel: float sums of up to 512 chunks of 512 elements or more (a
+ *     prediction of where each chunk starts, and whether it holds a NaN);
  *  2. l1_steps_kernel: each chunk's (d0, d1) in the three binades around its
  *     predicted start;
  *  3. l1_walk_kernel, one CTA per slice: a warp scans 32 chunks at a time and
@@ -21,9 +21,18 @@
  *     folded again by the whole CTA, segment by segment of one thread, and
  *     the one segment that crosses is added element by element.
  *
- * One thread adding in order waited for its loads: 3.78 ms for 530^2 elements
- * (13 ns each), against 0.040 ms for the three kernels here (most of it the walk: a
- * few microseconds at each of the binades left after the first 1024 elements).
+ * One thread adding in order waited for its loads, 13 ns an element: 3.36 ms for
+ * 530^2 of them, 0.04 ms with the three kernels here (most of it the walk: a few
+ * microseconds at each of the binades left after the first 1024 elements).
+ * Those cost 30 us whatever the size, so up to 8192 elements one thread adds
+ * from shared memory (l1_short_kernel, 2 ns an element). A call with 256 / 1024 /
+ * 4096 / 8192 / 8200 / 65536 elements takes 16 / 18 / 27 / 39 / 42 / 42 us of
+ * which 15 are the call; 18 / 26 / 65 / 115 / 114 / 800 element by element from
+ * global memory, 47 / 54 / 54 / 54 / 54 / 46 with the three kernels and 512
+ * chunks always. Chunks of at least 512 elements keep stacks of small slices from
+ * launching mostly idle CTAs: ASD-POCS of 1000 slices of 64^2, two iterations,
+ * 6.3 ms element by element, 86 with 512 chunks each, 3.3 now; 200 of 120^2
+ * 12.1, 19.9 and 4.8.
  */
 #include <cuda_runtime.h>
 
@@ -33,9 +42,11 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr int kChunks = 512;                 /* chunks per slice */
+constexpr int kChunks = 512;                 /* chunks per slice at most */
+constexpr int kMinChunk = 512;               /* elements of a chunk at least */
 constexpr int kCand = 3;                     /* binades tried per chunk */
 constexpr int kHead = 1024;                  /* elements added one by one at the start */
+constexpr size_t kShort = 8192;              /* elements of a slice that one thread adds */
 constexpr unsigned int kTop = 1u << 24;      /* units at the end of a binade */
 constexpr unsigned int kMany = 1u << 25;     /* any increment past the binade */
 
@@ -116,20 +127,20 @@ __device__ __forceinline__ unsigned int join(int e, unsigned int m)
     return m >= 0x800000u ? ((unsigned int) (e + 127) << 23) | (m & 0x7fffffu) : m;
 }
 
-__device__ __forceinline__ void chunk_range(size_t count, int c, size_t &lo, size_t &hi)
+/* Elements of chunk c of len. */
+__device__ __forceinline__ void chunk_range(size_t count, size_t len, int c, size_t &lo, size_t &hi)
 {
-    const size_t len = (count + kChunks - 1) / kChunks;
     lo = min((size_t) c * len, count);
     hi = min(lo + len, count);
 }
 
-__global__ void __launch_bounds__(kThreads) l1_sums_kernel(const float *__restrict__ v, size_t count,
+__global__ void __launch_bounds__(kThreads) l1_sums_kernel(const float *__restrict__ v, size_t count, size_t len,
                                                            ChunkRec *__restrict__ recs)
 {
     __shared__ float part[kWarps];
     const float *p = v + (size_t) blockIdx.y * count;
     size_t lo, hi;
-    chunk_range(count, (int) blockIdx.x, lo, hi);
+    chunk_range(count, len, (int) blockIdx.x, lo, hi);
     float s = 0.0f;
     for (size_t i = lo + threadIdx.x; i < hi; i += kThreads)
         s += fabsf(p[i]);
@@ -145,7 +156,7 @@ __global__ void __launch_bounds__(kThreads) l1_sums_kernel(const float *__restri
     }
 }
 
-__global__ void __launch_bounds__(kThreads) l1_steps_kernel(const float *__restrict__ v, size_t count,
+__global__ void __launch_bounds__(kThreads) l1_steps_kernel(const float *__restrict__ v, size_t count, size_t len,
                                                             ChunkRec *__restrict__ recs)
 {
     __shared__ float part[kWarps];
@@ -170,7 +181,7 @@ __global__ void __launch_bounds__(kThreads) l1_steps_kernel(const float *__restr
     const int ex = (int) ((__float_as_uint(s) & 0x7fffffffu) >> 23);
     const int e0 = max(max(ex, 1) - 127 - 1, -126);
     size_t lo, hi;
-    chunk_range(count, c, lo, hi);
+    chunk_range(count, len, c, lo, hi);
     /* a warp folds a run of whole 32-element rows, each lane 4 adjacent
      * elements of a 128-element step */
     const size_t per = (hi - lo + 128 * kWarps - 1) / (128 * kWarps) * 128;
@@ -272,9 +283,13 @@ __device__ unsigned int walk_chunk(const float *__restrict__ p, size_t lo, size_
     return bits;
 }
 
-__global__ void __launch_bounds__(kThreads) l1_walk_kernel(const float *__restrict__ v, size_t count,
-                                                           const ChunkRec *__restrict__ recs, float *out)
+/* FULL: kChunks of them, known to the code generator (3 % of the walk). */
+template <bool FULL>
+__global__ void __launch_bounds__(kThreads) l1_walk_kernel(const float *__restrict__ v, size_t count, size_t any_len,
+                                                           int any_chunks, const ChunkRec *__restrict__ recs, float *out)
 {
+    const int chunks = FULL ? kChunks : any_chunks;
+    const size_t len = FULL ? (count + kChunks - 1) / kChunks : any_len;
     __shared__ ChunkRec rs[kChunks];
     __shared__ float head[kHead];
     __shared__ Step tot[kWarps];
@@ -283,7 +298,7 @@ __global__ void __launch_bounds__(kThreads) l1_walk_kernel(const float *__restri
     const float *p = v + (size_t) blockIdx.x * count;
     const int lane = (int) (threadIdx.x & 31), warp = (int) (threadIdx.x >> 5);
     bool nan = false;
-    for (int c = (int) threadIdx.x; c < kChunks; c += kThreads) {
+    for (int c = (int) threadIdx.x; c < chunks; c += kThreads) {
         rs[c] = recs[(size_t) blockIdx.x * kChunks + c];
         nan = nan || rs[c].sum != rs[c].sum;
     }
@@ -297,7 +312,7 @@ __global__ void __launch_bounds__(kThreads) l1_walk_kernel(const float *__restri
     int c = 0;
     {
         size_t lo, hi;
-        chunk_range(count, 0, lo, hi);
+        chunk_range(count, len, 0, lo, hi);
         const int n_head = (int) min(hi, (size_t) kHead);
         for (int i = (int) threadIdx.x; i < kHead; i += kThreads)
             head[i] = i < n_head ? fabsf(p[i]) : 0.0f;
@@ -318,7 +333,7 @@ __global__ void __launch_bounds__(kThreads) l1_walk_kernel(const float *__restri
             bits = walk_chunk(p, (size_t) n_head, hi, bits, tot, share);
         c = 1;
     }
-    while (c < kChunks && bits < 0x7f800000u) {
+    while (c < chunks && bits < 0x7f800000u) {
         if (warp == 0) {
             for (;;) {
                 int e;
@@ -326,7 +341,7 @@ __global__ void __launch_bounds__(kThreads) l1_walk_kernel(const float *__restri
                 split(bits, e, m);
                 Step s;
                 s.d0 = s.d1 = 0u;
-                if (c + lane < kChunks) {
+                if (c + lane < chunks) {
                     const int k = e - rs[c + lane].e0;
                     if (k >= 0 && k < kCand)
                         s = rs[c + lane].s[k];
@@ -340,27 +355,64 @@ __global__ void __launch_bounds__(kThreads) l1_walk_kernel(const float *__restri
                 if (good > 0)
                     bits = join(e, __shfl_sync(0xffffffffu, end, max(good, 1) - 1));
                 c += good;
-                if (good < 32 || c >= kChunks || bits >= 0x7f800000u)
+                if (good < 32 || c >= chunks || bits >= 0x7f800000u)
                     break;
             }
             if (lane == 0) {
                 share[1] = bits;
-                next = min(c, kChunks);
+                next = min(c, chunks);
             }
         }
         __syncthreads();
         bits = share[1];
         c = next;
         __syncthreads();
-        if (c >= kChunks || bits >= 0x7f800000u)
+        if (c >= chunks || bits >= 0x7f800000u)
             break;
         size_t lo, hi;
-        chunk_range(count, c, lo, hi);
+        chunk_range(count, len, c, lo, hi);
         bits = walk_chunk(p, lo, hi, bits, tot, share);
         ++c;
     }
     if (threadIdx.x == 0)
         out[blockIdx.x] = __uint_as_float(bits);
+}
+
+/* The plain sum of a short slice: one thread adds from shared memory (4 cycles
+ * an element) while the next elements are on their way. */
+__global__ void __launch_bounds__(kThreads) l1_short_kernel(const float *__restrict__ v, int count, float *out)
+{
+    __shared__ __align__(16) float part[kHead];
+    const float *p = v + (size_t) blockIdx.x * count;
+    constexpr int kEach = kHead / kThreads;
+    float next[kEach];
+    auto load = [&](int i0) {
+#pragma unroll
+        for (int q = 0; q < kEach; ++q) {
+            const int i = i0 + q * kThreads + (int) threadIdx.x;
+            next[q] = i < count ? fabsf(p[i]) : 0.0f;
+        }
+    };
+    float sum = 0.0f;
+    load(0);
+    for (int i0 = 0; i0 < count; i0 += kHead) {
+#pragma unroll
+        for (int q = 0; q < kEach; ++q)
+            part[q * kThreads + threadIdx.x] = next[q];
+        __syncthreads();
+        load(i0 + kHead);
+        if (threadIdx.x == 0) {
+            const int n = min(kHead, count - i0);
+            for (int i = 0; i < n; i += 16) {      /* zeros after the end */
+#pragma unroll
+                for (int q = 0; q < 16; ++q)
+                    sum = __fadd_rn(sum, part[i + q]);
+            }
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0)
+        out[blockIdx.x] = sum;
 }
 
 }  // namespace
@@ -373,14 +425,24 @@ extern "C" size_t udev_l1_partials(int n_slices)
 int udev_l1_compat(udev *d, const float *v, size_t count, int n_slices, double *scratch, float *d_out)
 {
     ChunkRec *recs = reinterpret_cast<ChunkRec *>(scratch);
-    const dim3 grid((unsigned int) kChunks, (unsigned int) n_slices);
     int rc;
-    l1_sums_kernel<<<grid, kThreads, 0, d->stream>>>(v, count, recs);
+    if (count <= kShort) {
+        l1_short_kernel<<<(unsigned int) n_slices, kThreads, 0, d->stream>>>(v, (int) count, d_out);
+        return udev_after_launch(d, "l1_short_kernel");
+    }
+    const size_t fit = count / kMinChunk;
+    const int chunks = fit < (size_t) kChunks ? (int) fit : kChunks;
+    const size_t len = (count + chunks - 1) / chunks;
+    const dim3 grid((unsigned int) chunks, (unsigned int) n_slices);
+    l1_sums_kernel<<<grid, kThreads, 0, d->stream>>>(v, count, len, recs);
     if ((rc = udev_after_launch(d, "l1_sums_kernel")))
         return rc;
-    l1_steps_kernel<<<grid, kThreads, 0, d->stream>>>(v, count, recs);
+    l1_steps_kernel<<<grid, kThreads, 0, d->stream>>>(v, count, len, recs);
     if ((rc = udev_after_launch(d, "l1_steps_kernel")))
         return rc;
-    l1_walk_kernel<<<(unsigned int) n_slices, kThreads, 0, d->stream>>>(v, count, recs, d_out);
+    if (chunks == kChunks)
+        l1_walk_kernel<true><<<(unsigned int) n_slices, kThreads, 0, d->stream>>>(v, count, len, chunks, recs, d_out);
+    else
+        l1_walk_kernel<false><<<(unsigned int) n_slices, kThreads, 0, d->stream>>>(v, count, len, chunks, recs, d_out);
     return udev_after_launch(d, "l1_walk_kernel");
 }
