@@ -289,3 +289,41 @@ def test_fast_and_exact_backprojections_of_ones_agree(ufoir_lib, gpu_ctx, n, na)
         out.append(p.process(np.ones((na, n), f32)).astype(np.float64))
         p.close()
     assert np.linalg.norm(out[0] - out[1]) <= 1e-5 * np.linalg.norm(out[1])      # the path's bar
+
+
+# Coordinates beyond 2^31, where the index of a tap saturates: an axis far
+# outside, and a quarter turn walked as vertical rays (cos = -4e-8) by the kernel
+# of one thread per ray, which serves subsets beyond 8192 detectors.
+@pytest.mark.parametrize("na", [5, 20])
+@pytest.mark.parametrize("axis", [3.0e9, 1.0e10, 1.0e30])
+def test_an_axis_far_outside_gives_zeros(ufoir_lib, gpu_ctx, axis, na):
+    n = 33
+    rng = np.random.default_rng(na)
+    p = ufoir_lib.ParallelProjector(gpu_ctx, step=float(f32(np.pi / na)), axis_position=axis, angles_num=na)
+    assert not p.forward(rng.random((n, n), dtype=f32), np.zeros((na, n), f32)).any()
+    assert not p.backward(np.zeros((n, n), f32), rng.random((na, n), dtype=f32)).any()
+    p.close()
+    p = ufoir_lib.ParallelProjector(gpu_ctx, step=float(f32(np.pi / na)), axis_position=axis, is_forward=0)
+    assert not ufoir_lib.sart(p, rng.random((na, n), dtype=f32), num_iterations=1).any()
+    p.close()
+
+
+def test_a_quarter_turn_walked_as_vertical_rays(ufoir_lib, gpu_ctx):
+    n, na = 8200, 2
+    vol = np.random.default_rng(0).random((n, n), dtype=f32)
+    p = ufoir_lib.ParallelProjector(gpu_ctx, step=float(f32(np.pi / na)), angles_num=na)
+    p.get_requisition((n, n))
+    got = p.subset_fp(vol, np.zeros((na, n), f32), 1, 1, 1)
+    p.close()
+    sn, cs = _lut(na, f32(np.pi / na))
+    det, st, half = f32(1) / cs[1], sn[1] / cs[1], f32(0.5) * f32(n)
+    c = ((0.5 + np.arange(n) - float(half)) * float(det) + float(-half * st) + float(half)).astype(f32)
+    assert np.abs(c).max() > 2.0 ** 31
+    total, block = np.zeros(n, f32), np.zeros(n, f32)
+    for r in range(n):
+        block = block + _lerp(vol[r], c)
+        c = c + st
+        if r % 64 == 63:
+            total, block = total + block, np.zeros(n, f32)
+    np.testing.assert_array_equal(got[1], total + block)
+    assert not got[0].any()

@@ -83,13 +83,21 @@ __device__ __forceinline__ int n_blocks(int width)
     return (int) ceilf(__fdiv_rn((float) width, 64.0f));
 }
 
-/* Linear-filter weights at coordinate c: index i0 and fraction t. */
+/* Linear-filter weights at coordinate c: index i0 and fraction t. Beyond 2^31
+ * (an angle walked across its own direction, an axis far outside) the index
+ * saturates; the second tap's is next_tap(i0), not i0 + 1, which could then
+ * overflow: a bounds check on a signed overflow guards nothing. */
 __device__ __forceinline__ void lerp_coord(float c, int &i0, float &t)
 {
     const float cm = __fsub_rn(c, 0.5f);
     const float f = floorf(cm);
     i0 = (int) f;
     t = __fsub_rn(cm, f);
+}
+
+__device__ __forceinline__ int next_tap(int i0)
+{
+    return (int) ((unsigned int) i0 + 1u);
 }
 
 __device__ __forceinline__ float lerp(float t, float t0, float t1)

@@ -89,8 +89,9 @@ __global__ void __launch_bounds__(128) fp_rows_kernel(FpArgs A)
                 int i0;
                 float t;
                 joseph::lerp_coord(c, i0, t);
+                const int i1 = joseph::next_tap(i0);
                 const float t0 = (i0 >= 0 && i0 < n) ? __ldg(r + (size_t) i0 * col_step) : 0.0f;
-                const float t1 = (i0 + 1 >= 0 && i0 + 1 < n) ? __ldg(r + (size_t) (i0 + 1) * col_step) : 0.0f;
+                const float t1 = (i1 >= 0 && i1 < n) ? __ldg(r + (size_t) i1 * col_step) : 0.0f;
                 inner = __fadd_rn(inner, joseph::lerp(t, t0, t1));
                 c = __fadd_rn(c, slice_step);
             }
@@ -157,9 +158,9 @@ __global__ void __launch_bounds__(32 * kSplitWarps) fp_blocks_kernel(FpArgs A)
                 const bool in = row + q < n;
                 const float *r = img + (size_t) min(row + q, n - 1) * row_step;
                 ina[q] = in && (unsigned int) i0 < (unsigned int) n;
-                inb[q] = in && (unsigned int) i0 + 1u < (unsigned int) n;
+                inb[q] = in && (unsigned int) joseph::next_tap(i0) < (unsigned int) n;
                 va[q] = ina[q] ? __ldg(r + (size_t) i0 * col_step) : 0.0f;
-                vb[q] = inb[q] ? __ldg(r + (size_t) ((unsigned int) i0 + 1u) * col_step) : 0.0f;
+                vb[q] = inb[q] ? __ldg(r + (size_t) joseph::next_tap(i0) * col_step) : 0.0f;
             }
 #pragma unroll
             for (int q = 0; q < kBatch; ++q)
@@ -240,7 +241,7 @@ __global__ void __launch_bounds__(256) bp_gather_kernel(BpArgs A)
             float t;
             joseph::lerp_coord(sc, i0, t);
             const float *r = sino + (size_t) a * n;
-            sum = __fadd_rn(sum, joseph::lerp(t, joseph::texel(r, i0, n), joseph::texel(r, i0 + 1, n)));
+            sum = __fadd_rn(sum, joseph::lerp(t, joseph::texel(r, i0, n), joseph::texel(r, joseph::next_tap(i0), n)));
         }
         v = __fadd_rn(v, __fmul_rn(A.relax, sum));
     }

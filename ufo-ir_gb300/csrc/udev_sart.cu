@@ -124,14 +124,14 @@ __global__ void __launch_bounds__(kMaxThreads) fp_angle_kernel(FpAngleArgs P)
         for (int k = 0; k < 16; ++k) {
             const float *rr = img + (size_t) min(row0 + k, n - 1) * n;
             va[k] = __ldg(rr + min(max(i0[k], 0), n - 1));
-            vb[k] = __ldg(rr + min(max(i0[k] + 1, 0), n - 1));
+            vb[k] = __ldg(rr + min(max(joseph::next_tap(i0[k]), 0), n - 1));
         }
         float v[16];
 #pragma unroll
         for (int k = 0; k < 16; ++k) {
             const bool in_row = row0 + k < n;
             const float t0 = in_row && (unsigned) i0[k] < (unsigned) n ? va[k] : 0.0f;
-            const float t1 = in_row && (unsigned) (i0[k] + 1) < (unsigned) n ? vb[k] : 0.0f;
+            const float t1 = in_row && (unsigned) joseph::next_tap(i0[k]) < (unsigned) n ? vb[k] : 0.0f;
             v[k] = joseph::lerp(t[k], t0, t1);
         }
         /* inner = (((0 + v_0) + v_1) + ... + v_63), quarter by quarter */
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(256) bp_angle_kernel(BpAngleArgs P)
         float t;
         joseph::lerp_coord(sc, i0, t);
         const float sum =
-            __fadd_rn(0.0f, joseph::lerp(t, joseph::texel(r, i0, n), joseph::texel(r, i0 + 1, n)));
+            __fadd_rn(0.0f, joseph::lerp(t, joseph::texel(r, i0, n), joseph::texel(r, joseph::next_tap(i0), n)));
         v[h] = __fadd_rn(v[h], __fmul_rn(relax, sum));
     }
     if (VEC) {
