@@ -327,3 +327,9 @@ def test_a_quarter_turn_walked_as_vertical_rays(ufoir_lib, gpu_ctx):
             total, block = total + block, np.zeros(n, f32)
     np.testing.assert_array_equal(got[1], total + block)
     assert not got[0].any()
+
+
+@pytest.mark.parametrize("n,na,axis", [(130, 1600, 60.2), (200, 1250, 104.0)])
+def test_subset_projections_of_many_angles(ufoir_lib, gpu_ctx, oracle, n, na, axis):
+    """Subsets of more ray groups than the GPU has room for spread ones: one thread per ray."""
+    test_subset_projections(ufoir_lib, gpu_ctx, oracle, n, na, axis)

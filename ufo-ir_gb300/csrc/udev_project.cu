@@ -9,9 +9,10 @@
  * neighbouring detectors touch a few consecutive cache lines per step.
  * Samples are summed per ray in blocks of 64 in the reference's order, with
  * the float coordinate recurrence, so the sum is the reference's to the last
- * bit. The blocks of a ray are spread over the warps of a CTA
- * (fp_blocks_kernel); beyond 8192 detectors one thread walks a whole ray
- * (fp_rows_kernel).
+ * bit. Where the rays are few the blocks of a ray are spread over the warps of
+ * a CTA (fp_blocks_kernel), else, and beyond 8192 detectors, one thread walks a
+ * whole ray (fp_rows_kernel). Whole angle sets beyond the tiled projector's sizes
+ * come here as well.
  *
  * Backprojection (replaces BP, projector-parallel-joseph.cl:158-218): one
  * thread per pixel gathers every angle of every subset in order; no atomics,
@@ -107,6 +108,7 @@ __global__ void __launch_bounds__(128) fp_rows_kernel(FpArgs A)
 constexpr int kSplitBlocks = 128;   /* 64-sample blocks per ray at most (n <= 8192) */
 constexpr int kSplitWarps = 16;
 constexpr int kBatch = 16;          /* samples whose loads are in flight together */
+constexpr int kBigSlice = 5700;     /* detectors from which a slice is larger than L2 */
 
 /*
  * The same for 32 adjacent rays per CTA, lane = ray, with the rays' 64-sample
@@ -315,9 +317,19 @@ extern "C" int udev_fp(udev *d, const udev_geom *g, int a0, int na, int dir_over
         B.out += (size_t) done * A.sino_stride;
         int rc;
         const int nb = (g->n_dets + 63) / 64;
-        if (nb <= kSplitBlocks) {
+        /* Spread over warps while the groups of 32 rays leave the GPU short of
+         * them: 14 CTAs fit an SM (16 KB of sums each), so more groups than that
+         * wait for a second wave where one thread per ray has them all in
+         * flight. us, spread / one thread per ray, by groups:
+         *    724^2: 1472 71 / 89,  2208 102 / 93,  4416 187 / 160,  6900 268 / 207
+         *   1448^2: 1472 128 / 166, 2208 188 / 171, 4416 348 / 303, 13800 946 / 722
+         *   4096^2: 1536 372 / 469, 2048 426 / 471, 3072 702 / 583,  8192 1620 / 1336
+         * A slice larger than L2 waits for memory and gains up to 20 an SM:
+         *   6000^2: 2256 789 / 1249, 3008 1091 / 1237, 4512 1575 / 1205 */
+        const long long groups = (long long) udev_div_up(g->n_dets, 32) * na * chunk;
+        const int most = g->n_dets >= kBigSlice ? 20 : 14;
+        if (nb <= kSplitBlocks && groups <= (long long) most * d->sm_count) {
             /* as many warps per ray group as fill the GPU with 16 per SM */
-            const long long groups = (long long) udev_div_up(g->n_dets, 32) * na * chunk;
             long long W = (16LL * d->sm_count + groups - 1) / groups;
             W = W > kSplitWarps ? kSplitWarps : W;
             W = W > nb ? nb : W;
