@@ -710,13 +710,21 @@ static int fp_threads(int n, int dsplit, int J)
  *   2 x 2900^2 x 360  3.025 / 2.540*   (more parts do not fit two to an SM)
  *   1 x 1001^2 x 451  0.403 / 0.282* / 0.340 / 0.309
  *   1 x 512^2 x 400   0.129 / 0.088* / 0.100 / 0.092
+ *   3 x 960^2 x 800   0.755 / 0.733* / 0.852 / 0.843   (fast arithmetic)
+ * and with the angles in golden steps, which leaves tiles of one or two angles:
+ *   3 x 960^2 x 147   0.837 / 0.850* / 0.941 / 0.863
+ * Where a launch has few rounds of CTAs the parts cost less by themselves and
+ * the rounds more: over 480 launches of 64 to 3500 columns the choice is 1.0 %
+ * above the best part count on average; with the penalties of many rounds there
+ * as well it was 2.2 %, and up to 15 % above one part.
  */
 static double fp_split_cost(long long ctas, int sms, int threads, int ds)
 {
-    static const double pen[5] = {0.0, 1.046, 1.0, 1.02, 1.08};
+    static const double pen_many[5] = {0.0, 1.046, 1.0, 1.02, 1.08}, pen_few[5] = {0.0, 1.0, 1.0, 1.08, 1.15};
     const double mean = (double) (ctas * ds) / sms;
     const double most = mean >= 8.0 ? mean : (double) ((ctas * ds + sms - 1) / sms);
-    return pen[ds] * (threads / 32) * (0.7 * most + 0.3 * mean);
+    const double *pen = ctas >= 8LL * sms ? pen_many : pen_few;
+    return pen[ds] * (threads / 32) * (0.85 * most + 0.15 * mean);
 }
 
 static bool tiles_supported(const TileCfg &cfg, int smem_optin)
@@ -862,7 +870,16 @@ extern "C" int udev_fp_default_cfg(udev *d, const udev_geom *g, int n_tiles, int
      * rows for its range (fp_split_cost says when that pays). */
     const long long ctas = (long long) n_tiles * n_slices;
     const int sms = d->sm_count;
-    if (4 * ctas >= sms) {
+    /* Below a quarter of the SMs tiles are few (further down). Beyond 768
+     * columns whole-row parts keep two detector pairs a thread and start badly,
+     * so there windows serve up to 0.3 of the SMs (39 / 44 tiles of 776 columns
+     * 207 / 206 -> 174 us; 960 columns 251 / 251 -> 240 / 272, hence the line at
+     * 900), and in the fast arithmetic, whose samples wait longer for each other,
+     * up to 3/8 (39 / 56 tiles of 776 columns 242 / 241 -> 164 / 233 us, 960
+     * 293 / 300 -> 232 / 280, 1448 438 / 496 -> 451 / 502, 2900 924 / 1038 -> 748 /
+     * 1016; at 63 tiles 1448 goes 496 -> 712). */
+    const int few = n <= 768 ? sms / 4 : g->fast_arith ? 3 * sms / 8 : n < 900 ? 3 * sms / 10 : sms / 4;
+    if (ctas >= few) {
         double best = fp_split_cost(ctas, sms, cfg.threads, 1);
         for (int ds = 2; ds <= 4; ++ds) {
             udev_fp_cfg w = *c;
@@ -888,7 +905,7 @@ extern "C" int udev_fp_default_cfg(udev *d, const udev_geom *g, int n_tiles, int
         }
         return UFOIR_OK;
     }
-    /* Fewer tiles than a quarter of the SMs (one slice, few angles). A CTA's
+    /* Few tiles (one slice, few angles). A CTA's
      * time is its rows', and a row's grows with the CTA's warps: about 100 ns
      * with 3 or 4 warps of one detector pair per slot, 135 with 5 to 8, 175
      * with 12. So up to 8 parts of at least 64 detectors with whole rows, one
