@@ -333,3 +333,18 @@ def test_a_quarter_turn_walked_as_vertical_rays(ufoir_lib, gpu_ctx):
 def test_subset_projections_of_many_angles(ufoir_lib, gpu_ctx, oracle, n, na, axis):
     """Subsets of more ray groups than the GPU has room for spread ones: one thread per ray."""
     test_subset_projections(ufoir_lib, gpu_ctx, oracle, n, na, axis)
+
+
+# Whole sets of the siddon model go through tiles or the ray walk, whichever the
+# launch's tiles make faster: few tiles of many columns, golden steps (tiles of
+# one or two angles) and many full tiles, against the double oracle.
+@pytest.mark.parametrize("n,na,slices,golden", [(776, 12, 1, False), (300, 60, 6, True), (200, 90, 1, True), (120, 400, 4, False)])
+def test_siddon_tiles_and_walk_by_the_launch(ufoir_lib, gpu_ctx, oracle, n, na, slices, golden):
+    step = f32(np.pi * (np.sqrt(5) - 1) / 2 if golden else np.pi / na)
+    vols = np.random.default_rng(n).random((slices, n, n), dtype=f32)
+    p = ufoir_lib.ParallelProjector(gpu_ctx, step=float(step), is_forward=1, axis_position=n / 2 + 0.3, angles_num=na, model="siddon")
+    got = p.process(vols)
+    p.close()
+    for s in sorted({0, slices - 1}):
+        want = oracle.siddon_forward(n, na, step, vols[s], n / 2 + 0.3)
+        assert np.linalg.norm(got[s] - want) <= 1e-5 * np.linalg.norm(want)      # the model's tolerance

@@ -254,6 +254,7 @@ void ufoir__projector_geom(const ufoir_projector *p, udev_geom *g)
     g->d_cos = p->d_cos;
     g->d_dir = p->d_dir;
     g->fast_arith = p->prm.arithmetic == UFOIR_ARITH_FAST;
+    g->siddon = strcmp(p->prm.model, "siddon") == 0;
 }
 
 int ufoir_projector_get_requisition(ufoir_projector *proj, const size_t in_dims[2], size_t out_dims[2])
@@ -477,8 +478,31 @@ static int siddon_fp(ufoir_projector *p, ufoir_fp_scratch *s, int a0, int na, co
     return rc;
 }
 
-/* All angles through the tiled kernel, or the ray walk where it cannot serve
- * the size. */
+/*
+ * 1 if all angles are as fast through the tiles as by the ray walk: estimated us
+ * of both, from what they take on 152 SMs. The walk needs 0.16 us a row while
+ * its rays run at once (12 CTAs of 128 an SM), which is its loads' latency, and
+ * 1.7e6 samples a us beyond that. A tile's rows take r0 us at least, and an SM sp
+ * samples a us, those of angles that a tile lacks included. Tiles lose where
+ * they are few (3 x 776^2 x 129 walk / tiles 223 / 392 us, 1448^2 x 300 511 /
+ * 708) or hold few angles (golden steps: 8 x 1448^2 x 300 3.3 / 12.3 ms) and win
+ * else (1448^2 x 1200 1.62 / 1.03 ms, 512^2 x 800 181 / 122 us). Over 299
+ * geometries of 64 to 3500 columns the choice is 1 % above the better one.
+ */
+static int siddon_tiles_pay(ufoir_projector *p, const udev_fp_cfg *c, int n_tiles, int n_slices)
+{
+    const double n = p->n_dets, sm = udev_sm_count(p->ctx->dev), ctas = (double) n_tiles * n_slices;
+    const double rays = n * p->n_angles * n_slices;
+    const double walk = 20.0 + n * (rays <= 12 * 128 * sm ? 0.16 : 0.108 + rays / 1.7e6);
+    const int few = 4.0 * ctas < sm, small = p->n_dets <= 768, mid = p->n_dets <= 1536;
+    const double r0 = few ? (small ? 0.12 : mid ? 0.16 : 0.22) : small ? 0.16 : 0.44;
+    const double sp = few ? (mid ? 9500.0 : 12800.0) : small ? 18000.0 : 16000.0;
+    const double row = 0.5 * r0 + ctas * c->A * n / (sm * sp);
+    return 20.0 + n * (row > r0 ? row : r0) <= walk;
+}
+
+/* All angles through the tiled kernel, or the ray walk where that is faster or
+ * the tiles cannot serve the size. */
 static int siddon_fp_all(ufoir_projector *p, ufoir_fp_scratch *s, const float *dvol, const float *src, float *dsino,
                          int n_slices)
 {
@@ -488,7 +512,8 @@ static int siddon_fp_all(ufoir_projector *p, ufoir_fp_scratch *s, const float *d
     const void *tiles = NULL;
     int n_tiles = 0;
     int rc = ufoir__fp_shape(p, n_slices, &c, &tiles, &n_tiles);
-    if (rc == UFOIR_ERR_UNSUPPORTED)
+    if (rc == UFOIR_ERR_UNSUPPORTED ||
+        (!rc && !siddon_tiles_pay(p, &c, n_tiles, n_slices)))
         return siddon_fp(p, s, 0, (int) p->n_angles, dvol, src, dsino, n_slices);
     if (!rc)
         rc = udev_pad_transpose(p->ctx->dev, dvol, s->P, s->TP, s->nonfinite, (int) p->n_dets, n_slices);

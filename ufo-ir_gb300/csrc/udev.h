@@ -66,6 +66,7 @@ typedef struct {
     const float *d_cos;
     const unsigned char *d_dir;    /* [n_angles] direction of each angle (full subsets) */
     int fast_arith;                /* 1: the tiled projectors' fast interpolation (not the reference's rounding) */
+    int siddon;                    /* 1: the siddon model (its launches of the tiled forward projector) */
 } udev_geom;
 
 /* Forward projection of angles [a0, a0 + na) for n_slices slices:

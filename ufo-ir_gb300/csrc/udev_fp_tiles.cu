@@ -716,15 +716,17 @@ static int fp_threads(int n, int dsplit, int J)
  * Where a launch has few rounds of CTAs the parts cost less by themselves and
  * the rounds more: over 480 launches of 64 to 3500 columns the choice is 1.0 %
  * above the best part count on average; with the penalties of many rounds there
- * as well it was 2.2 %, and up to 15 % above one part.
+ * as well it was 2.2 %, and up to 15 % above one part. (The siddon model's samples
+ * are longer, so it keeps those: 1448^2 x 1200 1.06 ms in two parts, 1.15 in one.)
  */
-static double fp_split_cost(long long ctas, int sms, int threads, int ds)
+static double fp_split_cost(long long ctas, int sms, int threads, int ds, bool siddon)
 {
     static const double pen_many[5] = {0.0, 1.046, 1.0, 1.02, 1.08}, pen_few[5] = {0.0, 1.0, 1.0, 1.08, 1.15};
     const double mean = (double) (ctas * ds) / sms;
     const double most = mean >= 8.0 ? mean : (double) ((ctas * ds + sms - 1) / sms);
-    const double *pen = ctas >= 8LL * sms ? pen_many : pen_few;
-    return pen[ds] * (threads / 32) * (0.85 * most + 0.15 * mean);
+    const bool many = siddon || ctas >= 8LL * sms;
+    const double round = many ? 0.7 : 0.85;
+    return (many ? pen_many : pen_few)[ds] * (threads / 32) * (round * most + (1.0 - round) * mean);
 }
 
 static bool tiles_supported(const TileCfg &cfg, int smem_optin)
@@ -880,7 +882,7 @@ extern "C" int udev_fp_default_cfg(udev *d, const udev_geom *g, int n_tiles, int
      * 1016; at 63 tiles 1448 goes 496 -> 712). */
     const int few = n <= 768 ? sms / 4 : g->fast_arith ? 3 * sms / 8 : n < 900 ? 3 * sms / 10 : sms / 4;
     if (ctas >= few) {
-        double best = fp_split_cost(ctas, sms, cfg.threads, 1);
+        double best = fp_split_cost(ctas, sms, cfg.threads, 1, g->siddon != 0);
         for (int ds = 2; ds <= 4; ++ds) {
             udev_fp_cfg w = *c;
             w.dsplit = ds;
@@ -897,7 +899,7 @@ extern "C" int udev_fp_default_cfg(udev *d, const udev_geom *g, int n_tiles, int
                     break;
             if (w.K < 4)
                 continue;
-            const double cost = fp_split_cost(ctas, sms, w.threads, ds);
+            const double cost = fp_split_cost(ctas, sms, w.threads, ds, g->siddon != 0);
             if (cost < best) {
                 best = cost;
                 *c = w;

@@ -21,8 +21,9 @@
  * Joseph forward projector reads; in a slab it covers at most two pixels, and
  * its length in the slab (1 / max(a, b)) splits where it crosses the pixel
  * boundary. Whole angle sets run in the Joseph projector's tiles
- * (udev_fp_tiles.cu, 1.62 -> 1.03 ms for one slice of 1448^2 x 1200); the
- * kernel here, one thread per ray, serves subsets and sizes beyond the tiles'.
+ * (udev_fp_tiles.cu, 1.62 -> 1.03 ms for one slice of 1448^2 x 1200) where those
+ * are many and full enough (siddon_tiles_pay); the kernel here, one thread per
+ * ray, serves the other sets, subsets and sizes beyond the tiles'.
  * Backward: one register sum per pixel evaluates L for the (at most two) bins
  * whose lines cross the pixel, per angle. Both compute the same
  * chord lengths, so the backprojector is the adjoint of the forward one up
