@@ -656,7 +656,7 @@ int ufoir_projector_subset_fp(ufoir_projector *proj, const float *vol, float *si
     } else {
         /* horizontal rays walk the rows of the transpose, or the columns
          * where there is no memory for it */
-        if (!s->direction && s->n > 0 && ufoir__alloc(ctx, &volT, nv) == UFOIR_OK)
+        if (!s->direction && s->n > 0 && udev_try_malloc(ctx->dev, (void **) &volT, nv * sizeof(float)) == UFOIR_OK)
             UFOIR_TRY(udev_transpose(ctx->dev, bv.dev, volT, (int) n, 1));
         UFOIR_TRY(udev_fp(ctx->dev, &g, (int) s->offset, (int) s->n, s->direction ? 1 : 0, bv.dev, volT, bs.dev,
                           NULL, 0, bs.dev, proj->prm.correction_scale, 1));

@@ -33,6 +33,8 @@ int udev_mem_info(udev *d, size_t *free_bytes, size_t *total_bytes);
 int udev_sm_count(const udev *d);
 
 int udev_malloc(udev *d, void **p, size_t bytes);           /* stream-ordered */
+/* The same for memory that the caller can do without: no error text. */
+int udev_try_malloc(udev *d, void **p, size_t bytes);
 int udev_free(udev *d, void *p);
 int udev_host_malloc(udev *d, void **p, size_t bytes);      /* page-locked */
 int udev_host_free(udev *d, void *p);

@@ -222,20 +222,32 @@ int udev_mem_info(udev *d, size_t *free_bytes, size_t *total_bytes)
     return UFOIR_OK;
 }
 
-int udev_malloc(udev *d, void **p, size_t bytes)
+static cudaError_t alloc_async(udev *d, void **p, size_t bytes)
 {
-    UDEV_BIND(d);
     *p = nullptr;
-    if (bytes == 0)
-        bytes = 16;
-    cudaError_t e = cudaMallocAsync(p, bytes, d->stream);
+    const cudaError_t e = cudaMallocAsync(p, bytes ? bytes : 16, d->stream);
     if (e != cudaSuccess) {
         cudaGetLastError();
         *p = nullptr;
+    }
+    return e;
+}
+
+int udev_malloc(udev *d, void **p, size_t bytes)
+{
+    UDEV_BIND(d);
+    const cudaError_t e = alloc_async(d, p, bytes);
+    if (e != cudaSuccess) {
         udev_set_error(d, "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
         return e == cudaErrorMemoryAllocation ? UFOIR_ERR_NOMEM : UFOIR_ERR_CUDA;
     }
     return UFOIR_OK;
+}
+
+int udev_try_malloc(udev *d, void **p, size_t bytes)
+{
+    UDEV_BIND(d);
+    return alloc_async(d, p, bytes) == cudaSuccess ? UFOIR_OK : UFOIR_ERR_NOMEM;
 }
 
 int udev_free(udev *d, void *p)
