@@ -348,3 +348,17 @@ def test_siddon_tiles_and_walk_by_the_launch(ufoir_lib, gpu_ctx, oracle, n, na, 
     for s in sorted({0, slices - 1}):
         want = oracle.siddon_forward(n, na, step, vols[s], n / 2 + 0.3)
         assert np.linalg.norm(got[s] - want) <= 1e-5 * np.linalg.norm(want)      # the model's tolerance
+
+
+# The siddon model's limits hold whichever kernel would serve the call. Many
+# slices or angles of a small image are what the tiles would take.
+@pytest.mark.parametrize("n,na,slices", [(24, 1, 65536), (24, 65536, 1)])
+def test_siddon_refuses_what_is_beyond_its_limits(ufoir_lib, gpu_ctx, n, na, slices):
+    v, s = ufoir_lib.DeviceArray(gpu_ctx, (slices, n, n), zero=True), ufoir_lib.DeviceArray(gpu_ctx, (slices, na, n))
+    p = ufoir_lib.ParallelProjector(gpu_ctx, step=1e-4, is_forward=1, angles_num=na, model="siddon")
+    with pytest.raises(ufoir_lib.UfoirError) as e:
+        p.process(v, s)
+    assert e.value.status == ufoir_lib.ERR_INVALID
+    p.close()
+    v.close()
+    s.close()

@@ -512,8 +512,9 @@ static int siddon_fp_all(ufoir_projector *p, ufoir_fp_scratch *s, const float *d
     const void *tiles = NULL;
     int n_tiles = 0;
     int rc = ufoir__fp_shape(p, n_slices, &c, &tiles, &n_tiles);
-    if (rc == UFOIR_ERR_UNSUPPORTED ||
-        (!rc && !siddon_tiles_pay(p, &c, n_tiles, n_slices)))
+    /* the walk refuses what is beyond the model's limits */
+    const int refused = n_slices > UDEV_SIDDON_MOST || p->n_angles > UDEV_SIDDON_MOST;
+    if (rc == UFOIR_ERR_UNSUPPORTED || (!rc && (refused || !siddon_tiles_pay(p, &c, n_tiles, n_slices))))
         return siddon_fp(p, s, 0, (int) p->n_angles, dvol, src, dsino, n_slices);
     if (!rc)
         rc = udev_pad_transpose(p->ctx->dev, dvol, s->P, s->TP, s->nonfinite, (int) p->n_dets, n_slices);

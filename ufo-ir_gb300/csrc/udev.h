@@ -215,6 +215,8 @@ void udev_inject_copy_skip(udev *d, int chunk);
  * angle never completes (-1 = none). */
 void udev_inject_exchange_skip(udev *d, int angle);
 
+/* Slices or angles of one siddon call at most. */
+#define UDEV_SIDDON_MOST 65535
 /* The "siddon" model (udev_siddon.cu): exact line integrals of the pixel
  * image, bin k of angle theta being the line X cos - Y sin + axis = k + 0.5.
  * Forward over angles [a0, a0 + na): out = (src + scale * S) [* w] (src may

@@ -471,7 +471,7 @@ extern "C" int udev_siddon_fp(udev *d, const udev_geom *g, int a0, int na, const
     if (n_slices <= 0 || na <= 0)
         return UFOIR_OK;
     const int n = g->n_dets;
-    if (a0 < 0 || a0 + na > g->n_angles || n < 1 || n > 32768 || n_slices > 65535 || na > 65535) {
+    if (a0 < 0 || a0 + na > g->n_angles || n < 1 || n > 32768 || n_slices > UDEV_SIDDON_MOST || na > UDEV_SIDDON_MOST) {
         udev_set_error(d, "siddon_fp: angles [%d, %d) of %d, n = %d, %d slices out of range", a0, a0 + na,
                        g->n_angles, n, n_slices);
         return UFOIR_ERR_INVALID;
@@ -505,7 +505,7 @@ extern "C" int udev_siddon_bp(udev *d, const udev_geom *g, const ufoir_subset *s
     if (n_slices <= 0)
         return UFOIR_OK;
     const int n = g->n_dets;
-    if (n_subsets < 0 || n_subsets > kMaxSub || n < 1 || n_slices > 65535) {
+    if (n_subsets < 0 || n_subsets > kMaxSub || n < 1 || n_slices > UDEV_SIDDON_MOST) {
         udev_set_error(d, "siddon_bp: %d subsets (at most %d), %d slices", n_subsets, kMaxSub, n_slices);
         return UFOIR_ERR_INVALID;
     }
