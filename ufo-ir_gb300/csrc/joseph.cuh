@@ -189,10 +189,11 @@ __device__ __forceinline__ float2 lerp2(float2 t, float2 t0, float2 t1, float2 z
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c);
 
 /*
- * The same value from nt = -t in three packed operations instead of four:
- * t is a multiple of 2^-24 in [0, 1] (the fraction of a float coordinate), so
- * 1 - t is exact and (1 - t) * T0 is T0 - t * T0 rounded once, one fused
- * multiply-add. It needs finite taps: with T0 = inf the fused form gives
+ * The same value from nt = -t in three packed operations instead of four, for
+ * coordinates c >= 0.5 (the domain of floor_half2n): there t is a multiple of
+ * 2^-24 in [0, 1), so 1 - t is exact and (1 - t) * T0 is T0 - t * T0 rounded
+ * once, one fused multiply-add. (Just below 0 t has more bits than that and 1 - t
+ * rounds.) It also needs finite taps: with T0 = inf the fused form gives
  * inf - inf = NaN where the four-operation form gives inf, so callers use
  * lerp2 where the data hold a non-finite value. (A zero result may differ in
  * sign, which no sum that starts at +0 can show.)

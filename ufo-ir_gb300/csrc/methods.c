@@ -485,7 +485,8 @@ int ufoir__sart_body(void *arg)
      * current direction run, transposed while the angles are horizontal, so
      * that every ray walks rows.
      * The sweep kernel where it is the faster one, else the padded kernels
-     * where they serve the geometry, else the general ones; UFOIR_SART_KERNELS=general selects the general kernels always. */
+     * where they serve the geometry, else the general ones;
+     * UFOIR_SART_KERNELS=general selects the general kernels always. */
     const char *only = getenv("UFOIR_SART_KERNELS");
     const int general_only = only && strcmp(only, "general") == 0;
     const int split = sart_split(s->p);
@@ -590,7 +591,8 @@ static int sart_run(ufoir_projector *proj, unsigned int iters, float lambda, con
     it.work = work;
     it.table = table;
     it.relax_dev = NULL;
-    /* one angle sweep per graph: a sweep is already 2 * n_angles kernels */
+    /* one iteration per graph: 2 * n_angles kernels, or one per direction run
+     * where the sweep kernel serves */
     int rc2 = UFOIR_OK;
     void *exec = NULL;
     uint64_t kernels = 0;

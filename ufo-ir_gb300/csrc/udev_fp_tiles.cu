@@ -6,17 +6,16 @@
  * rays) are first written as padded copies, each row [2 zeros | n values |
  * zeros] of `pitch` floats (pitch % 4 == 0), so that every ray of either
  * direction walks the rows of a row-major image and a zero border needs no
- * bounds checks. One CTA owns a tile of up to A consecutive angles of one
- * direction and all n detectors (J per thread, lanes on adjacent
- * detectors). All of its A*n rays advance row by row in lockstep; chunks of
- * K rows (K | 64) are brought into shared memory by a single 1-D TMA bulk
- * copy each (cp.async.bulk + mbarrier, double buffered), and every row in
- * shared memory is sampled by all A*n rays, so the image is read from L2
- * once per tile instead of once per ray.
+ * bounds checks. A tile is up to A consecutive angles of one direction; one CTA
+ * owns its n detectors or one of 2 to 4 parts of them (2J per thread and angle
+ * slot, lanes on adjacent detectors; fp_split_cost says how many parts). All
+ * rays of a CTA advance row by row in lockstep; chunks of K rows (K | 64) are
+ * brought into shared memory by a single 1-D TMA bulk copy each (cp.async.bulk +
+ * mbarrier, double buffered), and every row in shared memory is sampled by all of
+ * them, so the image is read from L2 once per part instead of once per ray.
  *
- * When there are too few tiles to fill the GPU (one slice, few angles), a
- * tile's detectors are split over up to 8 CTAs, with whole rows while a part
- * keeps at most 8 warps. Else each stages only a window of each chunk's rows:
+ * When tiles are few (one slice, few angles), a tile's detectors are split over
+ * up to 8 CTAs, with whole rows while a part keeps at most 8 warps. Else each stages only a window of each chunk's rows:
  * the columns its rays can reach, bounded by the extreme rays of its angles
  * (the coordinate is monotone in detector and row), one 1-D copy per row, with
  * two zero slots after the window for taps outside it (they lie outside the
@@ -125,11 +124,6 @@ __device__ __forceinline__ void ray_rows(float cl, float ch, float st, float lo,
     b = min(max(ib, 0), n);
 }
 
-/* Windowed CTAs of the J = 1 variants made for large n (A <= 4) hold few
- * rays per thread: two of them per SM. (The A = 8 variant, the default at
- * n <= 768, measured 4 % slower held to that register budget.) */
-/* One CTA's work: angle tile `tile_idx` of P.tiles, detector part `dpart`
- * of P.dsplit, slice `slice`; smem_raw is the dynamic shared memory. */
 /* The tiled kernels' arithmetic: the reference's, the fast interpolation, or
  * the siddon model (exact line integrals, udev_siddon.cu). */
 constexpr int kArithExact = 0, kArithFast = 1, kArithSiddon = 2;
@@ -164,7 +158,9 @@ __device__ __forceinline__ float siddon_start(const SiddonRay &q, int dir, int k
     return (dir ? u0 / q.cs : (-u0) / q.sn) + (-half) * q.slope + half;
 }
 
-/* BATCH: P lies in shared memory, and its src is never NULL. */
+/* One CTA's work: angle tile `tile_idx` of P.tiles, detector part `dpart` of
+ * P.dsplit, slice `slice`; smem_raw is the dynamic shared memory. BATCH: P lies
+ * in shared memory, and its src is never NULL. */
 template <int J, int A, bool WIN, int AR, bool BATCH = false>
 __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int dpart, int slice,
                                         unsigned char *smem_raw)
@@ -540,6 +536,9 @@ __device__ __forceinline__ void fp_tile(const FpTileArgs &P, int tile_idx, int d
     }
 }
 
+/* Windowed CTAs of the J = 1 variants made for large n (A <= 4) hold few rays
+ * per thread: two of them per SM. (The A = 8 variant, the default at n <= 768,
+ * measured 4 % slower held to that register budget.) */
 template <int J, int A, bool WIN, int AR>
 __global__ void __launch_bounds__(WIN ? kMaxWinThreads : 768, (WIN && J == 1 && A <= 4) ? 2 : 1)
     fp_tiles_kernel(const __grid_constant__ FpTileArgs P)
