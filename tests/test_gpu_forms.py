@@ -362,3 +362,9 @@ def test_siddon_refuses_what_is_beyond_its_limits(ufoir_lib, gpu_ctx, n, na, sli
     p.close()
     v.close()
     s.close()
+
+
+@pytest.mark.parametrize("n,na,axis,arithmetic", [(776, 300, -1.0, 0), (776, 400, 380.4, 1), (1100, 420, -1.0, 1), (1900, 200, -1.0, 1)])
+def test_windows_serve_more_tiles_beyond_768_columns(ufoir_lib, gpu_ctx, n, na, axis, arithmetic):
+    """39 to 57 tiles: column windows in one slice, whole rows in twelve."""
+    test_few_tiles_give_what_many_give(ufoir_lib, gpu_ctx, n, na, axis, arithmetic)
